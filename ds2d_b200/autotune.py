@@ -21,7 +21,7 @@ import numpy as np
 
 from .api import Elastic2D
 
-_RING_BASE = {"pair": 0, "pair_split": 0, "pair_cta": 0, "pair_fcta": 0, "pair_xr": 0, "tb": 0,
+_RING_BASE = {"tile": 0, "pair": 0, "pair_split": 0, "pair_cta": 0, "pair_fcta": 0, "pair_xr": 0, "tb": 0,
               "tb_cta": 0, "tb_bulk": 1, "bwd_ws": 0, "bwd_1b": 0, "bwd_bulk": 0, "bwd_cta": 0}
 _RING_SPACE = [
     {"ring": 4, "xr": 128, "occ": 0, "cta": 128}, {"ring": 4, "xr": 128, "occ": 0, "cta": 192},
@@ -56,13 +56,15 @@ _WS_SPACE = ([{"tb": 2, "tb_cta": 0, "bwd_ws": kt} for kt in (96, 128, 192)] +
               for one in (0, 1) for bc in (128, 192, 256)] +
              [{"tb": 2, "tb_cta": 0, "bwd_bulk": 1, "bwd_1b": 1, "bwd_cta": 256, "pair_xr": pxr}
               for pxr in (96, 128, 192)])
-_RING_DEFAULTS = {"ring": 4, "xr": 128, "occ": 0, "cta": 0, "tb": 0, "tb_cta": 0, "tb_bulk": 1,
+_RING_DEFAULTS = {"tile": 0, "ring": 4, "xr": 128, "occ": 0, "cta": 0, "tb": 0, "tb_cta": 0, "tb_bulk": 1,
                   "bwd_ws": 0, "bwd_1b": 0, "bwd_bulk": 0, "bwd_cta": 0}
 
 
 def default_space(boundary="random"):
     """Full option sets (every knob named, so no setting carries over between candidates)."""
     space = [dict(_RING_BASE, **c) for c in _RING_SPACE]
+    # the tile kernels (one launch per step, small batches and the PML)
+    space += [dict(_RING_BASE, **{**_RING_SPACE[0], "tile": rows}) for rows in (8, 16)]
     if boundary == "random":
         space = ([dict(_RING_DEFAULTS, **c) for c in _PAIR_SPACE] +
                  [{**_RING_DEFAULTS, **_RING_BASE, **c} for c in _TB_SPACE + _WS_SPACE] + space)

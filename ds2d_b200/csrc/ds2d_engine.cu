@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
@@ -26,6 +27,7 @@
 #include "ds2d_tblock.cuh"
 #include "ds2d_bwdws.cuh"
 #include "ds2d_bwdbulk.cuh"
+#include "ds2d_tile.cuh"
 
 using namespace ds2d;
 
@@ -305,10 +307,16 @@ struct ds2d_ctx {
   std::vector<int> h_nxp;    // padded window rows of each slot of the current batch
   int opt_pcg_switch = 970;  // ds2d_lsrtm_pcg: per-mille residual ratio that ends the network phase
   int opt_pcg_m = 8;         // ds2d_lsrtm_pcg: directions kept for explicit conjugation
+  // Tile kernels (ds2d_tile.cuh): option "tile" (-1 automatic, 0 off, 8 / 16 / 32 rows per CTA);
+  // an explicit launch-shape option selects the marching kernels it shapes.
+  int opt_tile = -1;
+  bool shape_set = false;
   // Acoustic Born pair (LSRTM): background, scattered and adjoint states, Born overlay.
   float *ac[10] = {};        // bvx bvz bs | dvx dvz ds | yx yz ys | e
   float *ac_split[6] = {};   // with a PML: split stress s_x, s_z of background | scattered | adjoint
   float *ac2[6] = {};        // second (ping-pong) buffers of bvx bvz bs | dvx dvz ds (fused steps)
+  float *ac_split2[6] = {};  // tile steps: second buffers of the split stress
+  float *ac_e2 = nullptr;    // tile steps: second Born source (the sets run one step apart)
   double *dot_part = nullptr, *dot_out = nullptr;  // FP64 inner-product scratch
   // Work vectors of the LSRTM solver (model- and data-space), grown on demand.
   struct Vec {
@@ -319,12 +327,13 @@ struct ds2d_ctx {
   Wave fw2{}, abk2{};  // ping-pong partners of fw / abk for the fused kernels
   Wave b1_2{}, b2_2{};  // ping-pong partners of the scattered sets (fused ELSRTM forward)
   float *ov_s2[3] = {nullptr, nullptr, nullptr};  // Born source of b1 for b2 (fused forward)
+  float *ov_t[2][3] = {};  // tile steps: second Born sources (the sets run one step apart)
   Wave *fw_cur = nullptr;  // buffer holding the latest forward state
   double batch_cells = 0, batch_wcells = 0;  // padded / interior cells of the current batch
   // CUDA graphs of whole batches (time loops included), keyed by everything baked into them.
   int opt_graph = 1;
   struct GraphEntry {
-    long long key[6];
+    std::array<long long, 5> key;
     cudaGraphExec_t exec;
     long long launches;
   };
@@ -413,9 +422,17 @@ int alloc_strips(ds2d_ctx *c, Strips &st, int steps) {
   return DS2D_OK;
 }
 
+// Drops the captured batches (their launches hold the options and buffers of their capture).
+// Every entry point waits for its work, so none is in flight.
+void clear_graphs(ds2d_ctx *c) {
+  for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
+  c->graphs.clear();
+}
+
 // Frees one arena allocation before the context's end (buffers whose size follows an option).
 void release(ds2d_ctx *c, void *p) {
   if (!p) return;
+  clear_graphs(c);
   cudaFree(p);
   auto &v = c->arena.ptrs;
   v.erase(std::remove(v.begin(), v.end(), p), v.end());
@@ -937,12 +954,141 @@ bool ac_rev_pair_on(const ds2d_ctx *c) {
   return ac_pair_on(c) && c->occ_ac_rev[ac_rev_cta(c) == 192 ? 0 : 1] > 0;
 }
 
+// ---- tile kernels ------------------------------------------------------------------------------
+constexpr int kTileRows[3] = {8, 16, 32};
+using FwdTileFn = void (*)(FwdTileArgs);
+using BwdTileFn = void (*)(BwdTileArgs);
+using AcTileFn = void (*)(AcFwdTileArgs);
+using AcRevTileFn = void (*)(AcRevTileArgs);
+template <bool kBorn>
+FwdTileFn fwd_tile_fn(bool pml, int tx) {
+  if (pml) return tx == 8 ? k_fwd_tile<true, 8, kBorn> : tx == 16 ? k_fwd_tile<true, 16, kBorn> : k_fwd_tile<true, 32, kBorn>;
+  return tx == 8 ? k_fwd_tile<false, 8, kBorn> : tx == 16 ? k_fwd_tile<false, 16, kBorn> : k_fwd_tile<false, 32, kBorn>;
+}
+template <bool kScat>
+BwdTileFn bwd_tile_fn(bool pml, int tx) {
+  if (pml) return tx == 8 ? k_bwd_tile<true, 8, kScat> : tx == 16 ? k_bwd_tile<true, 16, kScat> : k_bwd_tile<true, 32, kScat>;
+  return tx == 8 ? k_bwd_tile<false, 8, kScat> : tx == 16 ? k_bwd_tile<false, 16, kScat> : k_bwd_tile<false, 32, kScat>;
+}
+AcTileFn ac_tile_fn(bool pml, int tx) {
+  if (pml) return tx == 8 ? k_ac_tile<true, 8> : tx == 16 ? k_ac_tile<true, 16> : k_ac_tile<true, 32>;
+  return tx == 8 ? k_ac_tile<false, 8> : tx == 16 ? k_ac_tile<false, 16> : k_ac_tile<false, 32>;
+}
+AcRevTileFn ac_rev_tile_fn(bool pml, int tx) {
+  if (pml) return tx == 8 ? k_ac_rev_tile<true, 8> : tx == 16 ? k_ac_rev_tile<true, 16> : k_ac_rev_tile<true, 32>;
+  return tx == 8 ? k_ac_rev_tile<false, 8> : tx == 16 ? k_ac_rev_tile<false, 16> : k_ac_rev_tile<false, 32>;
+}
+size_t bwd_tile_bytes(int tx, bool scat) {
+  return scat ? std::max(bwd_tile_smem(tx), scat_tile_smem(tx)) : bwd_tile_smem(tx);
+}
+
+cudaError_t tile_attributes() {
+  cudaError_t e = cudaSuccess;
+  auto set = [&](auto fn, size_t bytes) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  for (bool pml : {false, true})
+    for (int tx : kTileRows) {
+      set(fwd_tile_fn<false>(pml, tx), fwd_tile_smem(tx));
+      set(fwd_tile_fn<true>(pml, tx), fwd_tile_smem(tx));
+      set(bwd_tile_fn<false>(pml, tx), bwd_tile_bytes(tx, false));
+      set(bwd_tile_fn<true>(pml, tx), bwd_tile_bytes(tx, true));
+      set(ac_tile_fn(pml, tx), ac_tile_smem(tx));
+      set(ac_rev_tile_fn(pml, tx), ac_rev_tile_smem(tx));
+    }
+  return e;
+}
+
+bool tile_ok(const ds2d_ctx *c) {
+  return c->opt_fused && c->ring_ok && c->d.nop == 4 && c->d.ild == c->d.ld;
+}
+// Where a context's steps run on the tile kernels.  The rule looks at the context's batch (padded
+// cells of all its slots), so every batch of a context, a last short one too, takes the same
+// kernels.  Measured on a B200 at 0.05-22 M cells, ms per call, tile against marching kernels:
+//  - PML: elastic 16 x 1201x401 (8.9 M) RTM 41.5 / 43.1, forward 13.1 / 13.3, ELSRTM 138 / 141,
+//    and 6-50x on small batches; acoustic L^T L 0.66 M 5.5 / 6.9, 21.9 M 42.8 / 55.4 (half
+//    steps).  The marching kernels pay the PML's predicates row by row: always the tiles.
+//  - random boundary, elastic: 0.66 M 3.6 / 8.1, 1.97 M 9.6 / 10.6, 2.22 M 8.0 / 7.8, 8.9 M
+//    28.3 / 17.5: the bulk-copy marching kernels win once they fill the chip, at 2 M cells.
+//  - random boundary, acoustic: 0.66 M 3.0 / 14.2, 2.63 M 10.9 / 16.3, 21.9 M 27.9 / 21.2: 6 M.
+constexpr double kTileElastic = 2e6, kTileAcoustic = 6e6;
+bool tile_on(const ds2d_ctx *c, bool acoustic) {
+  if (!tile_ok(c) || c->opt_tile == 0) return false;
+  if (c->opt_tile > 0) return true;
+  if (c->shape_set) return false;
+  return !c->d.rbc || (double)c->B * c->d.slot <= (acoustic ? kTileAcoustic : kTileElastic);
+}
+// Rows per CTA: the elastic steps are best at 8 (registers: 3 CTAs an SM); the acoustic ones, with a
+// third of the operands, at 16, and at 32 (least redundant work) once the tiles fill the chip
+// (0.09 M cells 14.8 / 12.9 / 14.3 ms at 8 / 16 / 32, 2.6 M 15.3 / 11.6 / 10.9).
+int tile_rows(const ds2d_ctx *c, bool acoustic) {
+  if (c->opt_tile > 0) return c->opt_tile;
+  return !acoustic ? 8 : (double)c->B * c->d.slot < 1e6 ? 16 : 32;
+}
+dim3 tile_grid(const ds2d_ctx *c, int tx, int slices) {
+  return dim3((c->d.nzp + kTileZ - 1) / kTileZ, (c->d.nxp + tx - 1) / tx, slices);
+}
+// Launches a tile kernel; `chain`: behind another tile kernel of the same pass, so its loads of
+// what no step writes may overlap that one (programmatic dependent launch).
+template <class A>
+void launch_tile(ds2d_ctx *c, const char *name, double bytes, void (*fn)(A), dim3 grid, size_t smem,
+                 const A &a, bool chain) {
+  int ev = -1;
+  if (c->prof.on) {
+    ev = c->prof.take();
+    cudaEventRecord(c->prof.pool[ev], c->stream);
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kTileT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = chain && ev < 0 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, fn, a);
+  c->last_launches++;
+  if (ev >= 0) {
+    cudaEventRecord(c->prof.pool[ev + 1], c->stream);
+    c->prof.recs.push_back(ProfRec{name, ev, bytes});
+  }
+}
+
+// Forward pass on k_fwd_tile; with strips, each launch saves those of the state it reads.
+int run_forward_tile(ds2d_ctx *c, int n, bool record, bool strips) {
+  const Dims &d = c->d;
+  const int tx = tile_rows(c, false), nst = strips ? 1 : 0;
+  Wave *cur = &c->fw, *nxt = &c->fw2;
+  FwdTileArgs t{};
+  t.n = n;
+  t.nset = 1;
+  t.nst = nst;
+  for (int it = 0; it < d.nt; it++) {
+    FwdFusedArgs &a = t.set[0];
+    a.d = d; a.a = *cur; a.b = *nxt; a.p = c->par; a.shots = c->d_shots; a.wavelet = c->wavelet;
+    a.it = it; a.rmap = c->d_rmap;
+    if (record) { a.rec_on = 1; a.rec_vz = c->rec[0]; a.rec_vx = c->rec[1]; }
+    if (strips) t.st[0] = StripSaveArgs{d, c->d_shots, cur->vx, cur->vz, c->st_a, it - 1};
+    launch_tile(c, "fwd_tile", kBytesFused * CELLS(n), fwd_tile_fn<false>(!d.rbc, tx),
+                tile_grid(c, tx, n * (1 + nst)), fwd_tile_smem(tx), t, it > 0);
+    std::swap(cur, nxt);
+  }
+  if (strips) strip_save(c, *cur, c->st_a, d.nt - 1, n);
+  c->fw_cur = cur;
+  CK(cudaGetLastError());
+  return DS2D_OK;
+}
+
 // Fused forward pass: one k_fwd_fused launch per step, ping-ponging fw <-> fw2.
 int run_forward_fused(ds2d_ctx *c, int n, bool record, bool strips) {
   const Dims &d = c->d;
   int rc;
   if (!c->fw2.vx && (rc = alloc_wave(c, c->fw2, false))) return rc;
   if ((rc = zero_wave(c, c->fw2, n))) return rc;
+  if (tile_on(c, false)) return run_forward_tile(c, n, record, strips);
   const int cta = fused_cta(c);
   int nstrips, tz;
   strip_split(d, cta, &nstrips, &tz);
@@ -1083,11 +1229,17 @@ int rtm_batch_body(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base);
 // Runs `body` (device work only: launches, async device copies and memsets on c->stream) as a
 // CUDA graph: captured on first use for `key`, replayed afterwards.  Direct launches when
 // graphs are off, when profiling, or on the legacy default stream (which cannot be captured).
+// A key names the call, its batch, the stream and the density array that k_setup reads; the other
+// options and buffers are those of the capture (a changed option or freed buffer drops the graphs).
+using GraphKey = std::array<long long, 5>;
+GraphKey graph_key(const ds2d_ctx *c, int kind, int n, int shot_base) {
+  return {kind, n, shot_base, (long long)(size_t)c->stream, (long long)(size_t)c->rho_all};
+}
 template <class F>
-int run_graph(ds2d_ctx *c, const long long (&key)[6], F &&body) {
+int run_graph(ds2d_ctx *c, const GraphKey &key, F &&body) {
   if (!c->opt_graph || c->prof.on || c->stream == nullptr) return body();
   for (const auto &g : c->graphs)
-    if (std::equal(key, key + 6, g.key)) {
+    if (key == g.key) {
       CK(cudaGraphLaunch(g.exec, c->stream));
       c->last_launches += g.launches;
       return DS2D_OK;
@@ -1103,7 +1255,7 @@ int run_graph(ds2d_ctx *c, const long long (&key)[6], F &&body) {
   }
   CK(e);
   ds2d_ctx::GraphEntry g{};
-  std::copy(key, key + 6, g.key);
+  g.key = key;
   const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
   cudaGraphDestroy(graph);
   CK(ie);
@@ -1119,7 +1271,7 @@ int rtm_batch(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base) {
     if (!c->fw2.vx && (rc = alloc_wave(c, c->fw2, false))) return rc;
     if (!c->abk2.vx && (rc = alloc_wave(c, c->abk2, true))) return rc;
   }
-  const long long key[6] = {2, n, shot_base, c->opt_fused + 2 * c->opt_ring + 32 * c->opt_occ + 64 * c->opt_cta, c->opt_xr + 1000LL * c->opt_pair_xr + 1000000LL * c->opt_pair_cta + 100000000LL * (c->opt_pair_fcta / 64 + 5 * c->opt_pair_split) + 1000000000LL * c->opt_pair + 10000000000LL * (c->opt_tb + 5 * (c->opt_tb_cta / 32)) + 1000000000000LL * (c->opt_bwd_ws / 32 + 8 * c->opt_bwd_1b + 16 * c->opt_bwd_bulk + 32 * c->opt_tb_bulk + 64 * (c->opt_bwd_cta / 64)), (long long)(size_t)c->stream};
+  const GraphKey key = graph_key(c, 2, n, shot_base);
   return run_graph(c, key, [&]() { return rtm_batch_body(c, shots, n, shot_base); });
 }
 
@@ -1150,13 +1302,21 @@ int rtm_batch_body(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base) {
     strip_split(d, cta, &nstrips, &tz);
     const int xr = std::max(8, c->opt_xr);
     dim3 fgrid(nstrips, (d.nxp + xr - 1) / xr, n);
+    const bool tile = tile_on(c, false);
     for (int it = d.nt - 1; it >= 0; --it) {
       BwdFusedArgs a{};
       a.d = d; a.ra = *cur; a.rb = *nxt; a.aa = *acur; a.ab = *anxt; a.p = c->par;
       a.shots = c->d_shots; a.rmap = c->d_rmap; a.res_vz = c->rec[0]; a.res_vx = c->rec[1];
       a.st = c->st_a; a.strips_on = strips; a.it = it; a.tz = tz; a.xr = xr;
       a.img = c->img_slot; a.img_plane = (long long)plane;
-      if (pair_bwd_on(c) && c->opt_pair_split) {
+      if (tile) {
+        const int tx = tile_rows(c, false);
+        BwdTileArgs t{};
+        t.b = a;
+        t.n = n;
+        launch_tile(c, "bwd_tile", kBytesBwdFused * CELLS(n), bwd_tile_fn<false>(!d.rbc, tx),
+                    tile_grid(c, tx, n), bwd_tile_bytes(tx, false), t, it < d.nt - 1);
+      } else if (pair_bwd_on(c) && c->opt_pair_split) {
         int pns, ptz;
         pair_split(d, kPairSplitT, &pns, &ptz);
         const int pxr = pair_xr(c, pns, std::min(c->occ_pair[5], c->occ_pair[6]));
@@ -1272,7 +1432,51 @@ int elsrtm_forward_fused(ds2d_ctx *c, int n, bool strips) {
   Wave *set[3][2] = {{&c->fw, &c->fw2}, {&c->b1, &c->b1_2}, {&c->b2, &c->b2_2}};
   float *const *ov[2] = {c->ov_s, c->ov_s2};  // Born source of the background / of b1
   int cur = 0;
-  for (int it = 0; it < d.nt; it++, cur ^= 1) {
+  if (tile_on(c, false)) {
+    // One launch advances all three sets, set m one step behind set m - 1 (its Born source of
+    // step t is read while the source of step t + 1 is written, so each has two buffers), and
+    // saves the strips of the states it reads.
+    for (auto &o : c->ov_t)
+      for (float *p : o) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
+    float *const *ovt[2][2] = {{c->ov_s, c->ov_t[0]}, {c->ov_s2, c->ov_t[1]}};
+    const int tx = tile_rows(c, false), nst = strips ? 2 : 0;
+    FwdTileArgs t{};
+    t.n = n;
+    t.nset = 3;
+    t.nst = nst;
+    for (int l = 0; l < d.nt + 2; l++) {
+      for (int m = 0; m < 3; m++) {
+        FwdFusedArgs &a = t.set[m];
+        const int it = l - m, side = it & 1;
+        a = FwdFusedArgs{};
+        a.it = it < d.nt ? it : -1;
+        if (a.it < 0) continue;
+        a.d = d; a.a = *set[m][side]; a.b = *set[m][side ^ 1]; a.p = c->par;
+        a.shots = c->d_shots; a.wavelet = c->wavelet; a.rmap = c->d_rmap;
+        if (m > 0) {
+          float *const *o = ovt[m - 1][side];
+          a.rec_on = 1; a.rec_vz = c->rec[2 * m]; a.rec_vx = c->rec[2 * m + 1];
+          a.ovi_txx = o[0]; a.ovi_tzz = o[1]; a.ovi_txz = o[2];
+        }
+        if (m < 2) {
+          float *const *o = ovt[m][side];
+          a.ovo_txx = o[0]; a.ovo_tzz = o[1]; a.ovo_txz = o[2];
+        }
+      }
+      for (int m = 0; m < nst; m++) {  // the state after step l - m - 1, which set m reads now
+        const int it = l - m;
+        const Wave &w = *set[m][it & 1];
+        t.st[m] = StripSaveArgs{d, c->d_shots, w.vx, w.vz, m ? c->st_b : c->st_a,
+                                it >= 1 && it <= d.nt ? it - 1 : -1};
+      }
+      launch_tile(c, "fwd_born_tile",
+                  (kBytesBornMode[1] + kBytesBornMode[2] + kBytesBornMode[3]) * CELLS(n),
+                  fwd_tile_fn<true>(!d.rbc, tx), tile_grid(c, tx, n * (3 + nst)),
+                  fwd_tile_smem(tx), t, l > 0);
+    }
+    cur = d.nt & 1;
+  }
+  for (int it = 0; it < d.nt && !tile_on(c, false); it++, cur ^= 1) {
     for (int m = 0; m < 3; m++) {
       FwdFusedArgs a{};
       a.d = d; a.a = *set[m][cur]; a.b = *set[m][cur ^ 1]; a.p = c->par; a.shots = c->d_shots;
@@ -1332,6 +1536,35 @@ int elsrtm_backward_fused(ds2d_ctx *c, int n, bool strips) {
   Wave *fc = &c->fw, *fn = &c->fw2, *ac = &c->abk, *an = &c->abk2, *bc = &c->b1, *bn = &c->b1_2;
   const size_t sm = sizeof(float) * 4 * bwd_ring_fields(!d.rbc) * kFB;
   const size_t sm2 = sizeof(float) * 4 * kBwdScatRingFields * kFB;
+  if (tile_on(c, false)) {
+    // One launch: the backward step `it` and the scattered set's reverse step it + 1, whose
+    // background velocities and adjoint stresses are the backward step's inputs.
+    const int tx = tile_rows(c, false);
+    for (int it = d.nt - 1; it >= -1; --it) {
+      BwdTileArgs t{};
+      t.n = n;
+      BwdFusedArgs &a = t.b;
+      a.it = it;
+      a.d = d; a.ra = *fc; a.rb = *fn; a.aa = *ac; a.ab = *an; a.p = c->par;
+      a.shots = c->d_shots; a.rmap = c->d_rmap; a.res_vz = c->rec[6]; a.res_vx = c->rec[7];
+      a.st = c->st_a; a.strips_on = strips; a.img = c->img_slot; a.img_plane = plane;
+      BwdScatArgs &b = t.sc;
+      b.it = it + 1 < d.nt ? it + 1 : -1;
+      b.d = d; b.ra = *bc; b.rb = *bn; b.atxx = ac->txx; b.atzz = ac->tzz; b.atxz = ac->txz;
+      b.p = c->par; b.shots = c->d_shots; b.st = c->st_b; b.strips_on = strips;
+      b.img = c->img_slot; b.img_plane = plane;
+      t.fvx = fc->vx;
+      t.fvz = fc->vz;
+      launch_tile(c, "bwd_scat_tile", (kBytesBwdFused + kBytesBwdScat) * CELLS(n),
+                  bwd_tile_fn<true>(!d.rbc, tx), tile_grid(c, tx, 2 * n), bwd_tile_bytes(tx, true),
+                  t, it < d.nt - 1);
+      std::swap(fc, fn);
+      std::swap(ac, an);
+      if (b.it >= 0) std::swap(bc, bn);
+    }
+    CK(cudaGetLastError());
+    return DS2D_OK;
+  }
   for (int it = d.nt - 1; it >= 0; --it) {
     BwdFusedArgs a{};
     a.d = d; a.ra = *fc; a.rb = *fn; a.aa = *ac; a.ab = *an; a.p = c->par;
@@ -1357,8 +1590,7 @@ int elsrtm_backward_fused(ds2d_ctx *c, int n, bool strips) {
   return DS2D_OK;
 }
 
-int elsrtm_batch(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base, int iter,
-                 double *mis_host) {
+int elsrtm_body(ds2d_ctx *c, int n, int shot_base, int iter) {
   const Dims &d = c->d;
   int rc;
   if ((rc = setup_batch(c, n, shot_base, true))) return rc;
@@ -1460,7 +1692,28 @@ int elsrtm_batch(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base, int 
     LAUNCH(k_image, igrid, blk, im);
   }
   CK(cudaGetLastError());
-  if ((rc = reduce_images(c, n, 7))) return rc;
+  return reduce_images(c, n, 7);
+}
+
+int elsrtm_batch(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base, int iter,
+                 double *mis_host) {
+  const Dims &d = c->d;
+  int rc;
+  // allocations must precede the graph capture
+  if (c->opt_fused) {
+    for (Wave *w : {&c->fw2, &c->b1_2, &c->b2_2})
+      if (!w->vx && (rc = alloc_wave(c, *w, false))) return rc;
+    if (!c->abk2.vx && (rc = alloc_wave(c, c->abk2, true))) return rc;
+    for (float *&p : c->ov_s2)
+      if (!p && (rc = alloc_slots(c, &p))) return rc;
+  }
+  if (tile_on(c, false))
+    for (auto &o : c->ov_t)
+      for (float *&p : o)
+        if (!p && (rc = alloc_slots(c, &p))) return rc;
+  rc = run_graph(c, graph_key(c, iter == 0 ? 3 : 4, n, shot_base),
+                 [&]() { return elsrtm_body(c, n, shot_base, iter); });
+  if (rc) return rc;
   std::vector<double> terms((size_t)n * d.max_ntr);
   CK(cudaMemcpyAsync(terms.data(), c->d_mis, terms.size() * sizeof(double), cudaMemcpyDeviceToHost,
                      c->stream));
@@ -1495,6 +1748,11 @@ int ensure_acoustic(ds2d_ctx *c) {
   if (c->opt_fused && c->ring_ok)
     for (float *&p : c->ac2)
       if (!p && (rc = alloc_slots(c, &p))) return rc;
+  if (tile_on(c, true)) {
+    if (!c->ac_e2 && (rc = alloc_slots(c, &c->ac_e2))) return rc;
+    for (float *&p : c->ac_split2)
+      if (!c->d.rbc && !p && (rc = alloc_slots(c, &p))) return rc;
+  }
   if (!c->img_slot) {  // per-shot gradient planes (same 7-plane size as the RTM images)
     size_t n = (size_t)7 * c->B * c->d.wnx * c->d.ild;
     if ((rc = alloc(c, (void **)&c->img_slot, n * sizeof(float)))) return rc;
@@ -1556,12 +1814,62 @@ int ac_ring_step(ds2d_ctx *c, int n, int set, int cur, int it, bool born_out, bo
   return DS2D_OK;
 }
 
+// Tile-step arguments of the buffer pair `set` (0 background, 1 scattered) from side `cur`.
+AcTileArgs ac_tile_args(ds2d_ctx *c, int set, int cur, int it) {
+  float *const *side[2] = {c->ac + 3 * set, c->ac2 + 3 * set};
+  AcTileArgs a{};
+  a.d = c->d; a.shots = c->d_shots; a.rmap = c->d_rmap; a.wavelet = c->wavelet; a.it = it;
+  a.vx = side[cur][0]; a.vz = side[cur][1]; a.s = side[cur][2];
+  a.vx_n = side[1 - cur][0]; a.vz_n = side[1 - cur][1]; a.s_n = side[1 - cur][2];
+  if (!c->d.rbc) {
+    float *const *sp[2] = {c->ac_split + 2 * set, c->ac_split2 + 2 * set};
+    a.sx = sp[cur][0]; a.sz = sp[cur][1];
+    a.sx_n = sp[1 - cur][0]; a.sz_n = sp[1 - cur][1];
+  }
+  a.b = c->par.b; a.lam = c->par.lam; a.m = c->par.dmp;
+  a.dampx = c->par.dampx; a.dampz = c->par.dampz;
+  return a;
+}
+
+// L m on the tile kernels: one launch per step, the scattered set one step behind the background.
+int ac_L_tile(ds2d_ctx *c, int n) {
+  const Dims &d = c->d;
+  const size_t bytes = sizeof(float) * (size_t)d.slot * n, nrec = (size_t)n * d.max_ntr * d.nt;
+  for (int i = 0; i < 6; i++) {
+    CK(cudaMemsetAsync(c->ac[i], 0, bytes, c->stream));
+    CK(cudaMemsetAsync(c->ac2[i], 0, bytes, c->stream));
+  }
+  for (float *p : c->ac_split2)
+    if (p) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
+  float *const e[2] = {c->ac[9], c->ac_e2};
+  for (float *p : e) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
+  for (int i = 0; i < 2; i++) CK(cudaMemsetAsync(c->rec[i], 0, nrec * 4, c->stream));
+  const int tx = tile_rows(c, true);
+  for (int l = 0; l <= d.nt; l++) {
+    AcFwdTileArgs t{};
+    t.n = n;
+    t.nset = 2;
+    t.st.it = -1;
+    t.set[0] = ac_tile_args(c, 0, l & 1, l < d.nt ? l : -1);
+    t.set[0].e_out = e[l & 1];
+    t.set[1] = ac_tile_args(c, 1, (l - 1) & 1, l - 1);
+    t.set[1].e_in = e[(l - 1) & 1];
+    t.set[1].rec_vz = c->rec[0];
+    t.set[1].rec_vx = c->rec[1];
+    launch_tile(c, "ac_tile", 0, ac_tile_fn(!d.rbc, tx), tile_grid(c, tx, 2 * n), ac_tile_smem(tx),
+                t, l > 0);
+  }
+  CK(cudaGetLastError());
+  return DS2D_OK;
+}
+
 // L m for the uploaded batch: scattered vz / vx into rec[0] / rec[1] (m = the window p_dmp).
 int ac_L_batch(ds2d_ctx *c, int n) {
   const Dims &d = c->d;
   size_t bytes = sizeof(float) * (size_t)d.slot * n;
   if (!d.rbc)
     for (float *p : c->ac_split) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
+  if (tile_on(c, true)) return ac_L_tile(c, n);
   if (d.rbc && c->opt_fused && c->ring_ok && c->ac2[0]) {
     // fused: per step one background launch (Born source out) and one scattered launch
     for (int i = 0; i < 10; i++)
@@ -1660,16 +1968,13 @@ void ac_LT_pml_reverse_step(ds2d_ctx *c, int n, const Dims &ds, int srow, int it
   LAUNCHP("ac_vel", 0, k_ac_vel, grid, blk, b);
 }
 
-// PML L^T with background checkpoints every K steps (option "ac_ckpt"): a forward pass keeps
-// snapshots 0 .. nseg-2 (the state before steps 0, K, 2K, ...); then, from the last segment to the
-// first, the segment's start state (the exact state for the last, a decoded snapshot for the
-// others) is replayed over its steps saving their strips into a K-step buffer, and the segment is
-// reversed with them.  Forward work: (nseg - 1) K + nt steps instead of nt.
-int ac_LT_batch_pml_ckpt(ds2d_ctx *c, int n, int K) {
+// Snapshot buffers of the checkpointed PML L^T (option "ac_ckpt").
+int ensure_ckpt(ds2d_ctx *c) {
   const Dims &d = c->d;
-  const int nseg = (d.nt + K - 1) / K;
+  const int K = c->opt_ac_ckpt;
+  if (d.rbc || K <= 0 || K >= d.nt) return DS2D_OK;
   const size_t esz = c->o.strip_precision == DS2D_STRIPS_F32 ? 4 : 2;
-  const int nsnap = std::max(1, nseg - 1);
+  const int nsnap = std::max(1, (d.nt + K - 1) / K - 1);
   const size_t need = (size_t)nsnap * kCkptFields * c->B * d.slot * esz;
   int rc;
   if (c->ckpt_bytes < need) {
@@ -1686,6 +1991,18 @@ int ac_LT_batch_pml_ckpt(ds2d_ctx *c, int n, int K) {
   if (!c->ckpt_amax &&
       (rc = alloc(c, (void **)&c->ckpt_amax, sizeof(unsigned) * kCkptFields * c->B)))
     return rc;
+  return DS2D_OK;
+}
+
+// PML L^T with background checkpoints every K steps (option "ac_ckpt"): a forward pass keeps
+// snapshots 0 .. nseg-2 (the state before steps 0, K, 2K, ...); then, from the last segment to the
+// first, the segment's start state (the exact state for the last, a decoded snapshot for the
+// others) is replayed over its steps saving their strips into a K-step buffer, and the segment is
+// reversed with them.  Forward work: (nseg - 1) K + nt steps instead of nt.
+int ac_LT_batch_pml_ckpt(ds2d_ctx *c, int n, int K) {
+  const Dims &d = c->d;
+  const int nseg = (d.nt + K - 1) / K;
+  int rc;
   dim3 grid = cell_grid(d, n), blk(32, 8);
   auto fwd_step = [&](int it) {
     AcArgs b = ac_args(c, 0, it, 1.f);
@@ -1713,11 +2030,69 @@ int ac_LT_batch_pml_ckpt(ds2d_ctx *c, int n, int K) {
   return reduce_images(c, n, 1);
 }
 
+// L^T r on the tile kernels: forward replay of the background (with a PML each launch saves the
+// strips of the state it reads), then one launch per reverse step.
+int ac_LT_tile(ds2d_ctx *c, int n) {
+  const Dims &d = c->d;
+  const size_t bytes = sizeof(float) * (size_t)d.slot * n;
+  const int tx = tile_rows(c, true), nst = d.rbc ? 0 : 1;
+  for (float *p : c->ac2) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
+  for (float *p : c->ac_split2)
+    if (p) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
+  for (int it = 0; it < d.nt; it++) {
+    AcFwdTileArgs t{};
+    t.n = n;
+    t.nset = 1;
+    t.set[0] = ac_tile_args(c, 0, it & 1, it);
+    t.st = StripSaveArgs{d, c->d_shots, t.set[0].vx, t.set[0].vz, c->st_a, it - 1};
+    launch_tile(c, "ac_tile", 0, ac_tile_fn(!d.rbc, tx), tile_grid(c, tx, n * (1 + nst)),
+                ac_tile_smem(tx), t, it > 0);
+  }
+  float *bk[2][3], *yk[2][5];
+  for (int i = 0; i < 3; i++) {
+    bk[d.nt & 1][i] = c->ac2[i];
+    bk[(d.nt & 1) ^ 1][i] = c->ac[i];
+    yk[0][i] = c->ac[6 + i];
+    yk[1][i] = c->ac2[3 + i];
+  }
+  std::swap(bk[0], bk[1]);  // bk[0]: the final state (ac after an even number of steps)
+  for (int i = 0; i < 2; i++) {
+    yk[0][3 + i] = c->ac_split[4 + i];
+    yk[1][3 + i] = c->ac_split2[4 + i];
+  }
+  if (!d.rbc) {
+    StripSaveArgs sv{d, c->d_shots, bk[0][0], bk[0][1], c->st_a, d.nt - 1};
+    LAUNCH(k_strip_save, dim3((d.lb + 255) / 256, 2, n), 256, sv);
+    // cells outside the interior are not rebuilt: both buffers keep them as the forward pass left
+    // them
+    for (int i = 0; i < 3; i++)
+      CK(cudaMemcpyAsync(bk[1][i], bk[0][i], bytes, cudaMemcpyDeviceToDevice, c->stream));
+  }
+  int cur = 0;
+  for (int it = d.nt - 1; it >= 0; --it, cur ^= 1) {
+    AcRevTileArgs a{};
+    float **y = yk[cur], **yn = yk[cur ^ 1], **b = bk[cur], **bn = bk[cur ^ 1];
+    a.d = d; a.shots = c->d_shots;
+    a.yx = y[0]; a.yz = y[1]; a.ys = y[2]; a.ysx = y[3]; a.ysz = y[4];
+    a.yx_n = yn[0]; a.yz_n = yn[1]; a.ys_n = yn[2]; a.ysx_n = yn[3]; a.ysz_n = yn[4];
+    a.vx = b[0]; a.vz = b[1]; a.s = b[2];
+    a.vx_n = bn[0]; a.vz_n = bn[1]; a.s_n = bn[2];
+    a.b = c->par.b; a.lam = c->par.lam; a.dampx = c->par.dampx; a.dampz = c->par.dampz;
+    a.wavelet = c->wavelet; a.grad = c->img_slot; a.it = it; a.rmap = c->d_rmap;
+    a.res_vz = c->rec[0]; a.res_vx = c->rec[1]; a.st = c->st_a;
+    launch_tile(c, "ac_rev_tile", kBytesAcRev * CELLS(n), ac_rev_tile_fn(!d.rbc, tx),
+                tile_grid(c, tx, n), ac_rev_tile_smem(tx), a, it < d.nt - 1);
+  }
+  CK(cudaGetLastError());
+  return reduce_images(c, n, 1);
+}
+
 int ac_LT_batch_pml(ds2d_ctx *c, int n) {
   const Dims &d = c->d;
   size_t bytes = sizeof(float) * (size_t)d.slot * n;
   for (float *p : c->ac_split) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
   if (c->opt_ac_ckpt > 0 && c->opt_ac_ckpt < d.nt) return ac_LT_batch_pml_ckpt(c, n, c->opt_ac_ckpt);
+  if (tile_on(c, true)) return ac_LT_tile(c, n);
   dim3 grid = cell_grid(d, n), blk(32, 8);
   for (int it = 0; it < d.nt; it++) {
     AcArgs b = ac_args(c, 0, it, 1.f);
@@ -1743,6 +2118,7 @@ int ac_LT_batch(ds2d_ctx *c, int n) {
   CK(cudaMemsetAsync(c->img_slot, 0, plane * sizeof(float), c->stream));
   dim3 grid = cell_grid(d, n), blk(32, 8);
   if (!d.rbc) return ac_LT_batch_pml(c, n);
+  if (tile_on(c, true)) return ac_LT_tile(c, n);
   const bool fused = c->opt_fused && c->ring_ok && c->ac2[0];
   if (fused) {
     // fused forward replay of the background, final state left in ac[0..2]
@@ -1843,15 +2219,23 @@ int ac_apply(ds2d_ctx *c, const ds2d_shot *shots, int n, bool adjoint, const flo
   for (int f = 0; f < n; f += c->B) {
     const int m = std::min(c->B, n - f);
     if ((rc = upload_batch(c, shots + f, m))) return rc;
-    if ((rc = setup_batch(c, m, f, !adjoint))) return rc;
     if (!adjoint) {
-      if ((rc = ac_L_batch(c, m))) return rc;
+      rc = run_graph(c, graph_key(c, 5, m, f), [&]() {
+        const int r = setup_batch(c, m, f, true);
+        return r ? r : ac_L_batch(c, m);
+      });
+      if (rc) return rc;
       CK(cudaMemcpyAsync(dz + f * per, c->rec[0], m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
       CK(cudaMemcpyAsync(dx + f * per, c->rec[1], m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
     } else {
       CK(cudaMemcpyAsync(c->rec[0], dz + f * per, m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
       CK(cudaMemcpyAsync(c->rec[1], dx + f * per, m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
-      if ((rc = ac_LT_batch(c, m))) return rc;
+      if ((rc = ensure_ckpt(c))) return rc;
+      rc = run_graph(c, graph_key(c, 6, m, f), [&]() {
+        const int r = setup_batch(c, m, f, false);
+        return r ? r : ac_LT_batch(c, m);
+      });
+      if (rc) return rc;
     }
     // upload_batch of the next batch overwrites d_shots / rmap: finish this batch first.
     CK(cudaStreamSynchronize(c->stream));
@@ -2061,6 +2445,7 @@ int ds2d_create(const ds2d_grid *grid, const ds2d_opts *opts, ds2d_ctx **out) {
           e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->occ_tb_bulk[i][K - 1],
                                                             tb_fn(K, cta, true), cta, sm);
       }
+    if (e == cudaSuccess) e = tile_attributes();
     int dev = 0;
     if (e == cudaSuccess) e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2116,8 +2501,7 @@ int ds2d_destroy(ds2d_ctx *c) {
   if (c->own) cudaStreamSynchronize(c->own);
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->aux) cudaStreamSynchronize(c->aux);
-  for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
-  c->graphs.clear();
+  clear_graphs(c);
   for (auto &v : c->vecs)
     if (v.p) cudaFree(v.p);
   c->arena.release();
@@ -2193,7 +2577,7 @@ int ds2d_forward(ds2d_ctx *c, const ds2d_shot *shots, int n, float *rec_vz, floa
     int m = std::min(c->B, n - f);
     if ((rc = upload_batch(c, shots + f, m))) return rc;
     if (c->opt_fused && !c->fw2.vx && (rc = alloc_wave(c, c->fw2, false))) return rc;
-    const long long key[6] = {1, m, f, c->opt_fused + 2 * c->opt_ring + 32 * c->opt_occ + 64 * c->opt_cta, c->opt_xr + 1000LL * c->opt_pair_xr + 1000000LL * c->opt_pair_cta + 100000000LL * (c->opt_pair_fcta / 64 + 5 * c->opt_pair_split) + 1000000000LL * c->opt_pair + 10000000000LL * (c->opt_tb + 5 * (c->opt_tb_cta / 32)) + 1000000000000LL * (c->opt_bwd_ws / 32 + 8 * c->opt_bwd_1b + 16 * c->opt_bwd_bulk + 32 * c->opt_tb_bulk + 64 * (c->opt_bwd_cta / 64)), (long long)(size_t)c->stream};
+    const GraphKey key = graph_key(c, 1, m, f);
     rc = run_graph(c, key, [&]() {
       int r;
       if ((r = setup_batch(c, m, f, false))) return r;
@@ -2604,7 +2988,16 @@ int ds2d_dot_f64(ds2d_ctx *c, const float *a, const float *b, long long n, doubl
 int ds2d_set_option(ds2d_ctx *c, const char *key, long long value) {
   if (!c || !key) return DS2D_E_ARG;
   std::string k(key);
-  if (k == "fused") {
+  // A graph holds the options of its capture ("graph" itself and the solver's options shape none).
+  if (k != "graph" && k.compare(0, 4, "pcg_") != 0) clear_graphs(c);
+  if (k != "graph" && k.compare(0, 4, "pcg_") != 0 && k != "adjoint_born" && k != "ac_ckpt" &&
+      k != "tile")
+    c->shape_set = true;
+  if (k == "tile") {
+    if (value != -1 && value != 0 && value != 8 && value != 16 && value != 32)
+      return fail(c, DS2D_E_ARG, "tile must be -1 (automatic), 0 (off), 8, 16 or 32 rows per CTA");
+    c->opt_tile = (int)value;
+  } else if (k == "fused") {
     c->opt_fused = value != 0;
   } else if (k == "adjoint_born") {
     c->opt_adjoint_born = value != 0;

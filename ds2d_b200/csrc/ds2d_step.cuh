@@ -375,17 +375,9 @@ struct StripSaveArgs {
   int it;
 };
 
-__global__ void __launch_bounds__(256) k_strip_save(StripSaveArgs a) {
-  const int s = blockIdx.z, comp = blockIdx.y;
-  const Dims d = slot_dims(a.d, a.shots[s]);
-  const int bo = blockIdx.x * 256 + threadIdx.x;
-  const bool valid = bo < d.lb;
-  float v = 0.f;
-  if (valid) {
-    int ix, iz;
-    band_cell(d, bo, ix, iz);
-    v = (comp ? a.vz : a.vx)[d.slot * s + (long long)ix * d.ld + iz];
-  }
+// Stores element bo (value v) of component comp; the 32 lanes of a warp hold one segment.
+__device__ __forceinline__ void strip_put(const StripSaveArgs &a, const Dims &d, int s, int comp,
+                                          int bo, float v, bool valid) {
   const long long row = ((long long)s * d.nt + a.it) * 2 + comp;
   const long long e = row * d.lb_max + bo;
   if (a.st.prec == 0) {
@@ -398,11 +390,25 @@ __global__ void __launch_bounds__(256) k_strip_save(StripSaveArgs a) {
   // Leading wavefront tails reach subnormal magnitudes, where m / 2^15 would underflow to 0;
   // clamping the scale at FLT_MIN keeps |q| <= 2^15 inside the fp16 range.
   const float sc = m > 0.f ? fmaxf(m * (1.0f / 32768.0f), 1.17549435e-38f) : 1.0f;
-  if ((threadIdx.x & 31) == 0 && bo < d.lb) a.st.scale[row * d.nseg_max + (bo >> 5)] = sc;
+  if ((threadIdx.x & 31) == 0 && valid) a.st.scale[row * d.nseg_max + (bo >> 5)] = sc;
   if (!valid) return;
   const float q = v / sc;
   if (a.st.prec == 1) ((__half *)a.st.data)[e] = __float2half_rn(q);
   else ((__nv_bfloat16 *)a.st.data)[e] = __float2bfloat16_rn(q);
+}
+
+__global__ void __launch_bounds__(256) k_strip_save(StripSaveArgs a) {
+  const int s = blockIdx.z, comp = blockIdx.y;
+  const Dims d = slot_dims(a.d, a.shots[s]);
+  const int bo = blockIdx.x * 256 + threadIdx.x;
+  const bool valid = bo < d.lb;
+  float v = 0.f;
+  if (valid) {
+    int ix, iz;
+    band_cell(d, bo, ix, iz);
+    v = (comp ? a.vz : a.vx)[d.slot * s + (long long)ix * d.ld + iz];
+  }
+  strip_put(a, d, s, comp, bo, v, valid);
 }
 
 // Zero-lag imaging, FD2DGPU.cu:3245-3263 doimage_gradient (x3 in reference mode) and

@@ -231,7 +231,10 @@ int ds2d_bandpass_filter_device(int nx, int nz, int x1, int x2, int z1, int z2, 
  * 0 = per-thread cp.async), "bwd_cta" (threads per CTA of the bulk-copy step: 128 / 192 / 256,
  * 0 = the width with the fewest threads per grid row), "bwd_1b" (1 = one barrier per row step:
  * the default; 0 = two), "bwd_ws" (0 off, or 96 / 128 / 192 threads per role of the
- * warp-specialised step). */
+ * warp-specialised step).  "tile": the tile kernels, one launch per time step with every row of a
+ * tile in parallel, for batches that do not fill the chip and for every PML step: -1 = automatic
+ * (the default: by boundary and padded cells of the context's slots, unless one of the launch-shape
+ * options above is set), 0 = off, 8 / 16 / 32 = on with that many rows per CTA. */
 int ds2d_set_option(ds2d_ctx *ctx, const char *key, long long value);
 
 /* Profiling (no counterpart in the reference, which has only a commented-out host timer,
