@@ -199,8 +199,9 @@ int ds2d_dot_f64_noalloc(const float *a, const float *b, long long n, void *stre
  * complex (k, k) multiply.  x1, x2 are accepted for the reference's signature and unused, as in
  * its live filter.  ds2d_bandpass_filter takes host arrays (copied in and out, like the
  * reference); ds2d_bandpass_filter_device filters device arrays in place on `stream`.  Either
- * image pointer may be NULL.  Both allocate their scratch per call (two DFT matrices and three
- * work planes, about 16 (nx^2 + nz^2 + 3 nx nz) bytes).  Errors via ds2d_last_error(NULL). */
+ * image pointer may be NULL.  Both allocate their scratch per call: about 36 nx nz bytes for
+ * transforms of up to 4096 points, two DFT matrices and three work planes (about
+ * 16 (nx^2 + nz^2 + 3 nx nz) bytes) beyond.  Errors via ds2d_last_error(NULL). */
 int ds2d_bandpass_filter(int nx, int nz, int x1, int x2, int z1, int z2, float *grad_pp,
                          float *grad_ps);
 int ds2d_bandpass_filter_device(int nx, int nz, int x1, int x2, int z1, int z2, float *grad_pp,

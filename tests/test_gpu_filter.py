@@ -49,3 +49,17 @@ def test_bandpass_rejects_bad_arguments(cuda_device):
     from ds2d_b200._lib import DS2DError
     with pytest.raises(DS2DError):
         bandpass_filter(np.zeros((8, 8), np.float32), np.zeros((8, 8), np.float32), 0, 0)
+
+
+# Lengths around the powers of two that the chirp transforms pad to, the shortest, the longest of
+# the in-memory transforms and one beyond them (dense products).
+@pytest.mark.parametrize("nx,nz,z1,z2", [(2, 2, 0, 3), (3, 2, 1, 2), (5, 8, 0, 2), (32, 33, 2, 9),
+                                         (33, 65, 0, 9), (4096, 3, 5, 60), (3, 4096, 0, 60),
+                                         (2049, 17, 0, 40), (4097, 6, 0, 60)])
+def test_bandpass_lengths(cuda_device, nx, nz, z1, z2):
+    rng = np.random.default_rng(nx + nz)
+    pp = rng.standard_normal((nx, nz)).astype(np.float32)
+    ps = 1e-3 * rng.standard_normal((nx, nz)).astype(np.float32)
+    fpp, fps = bandpass_filter(pp, ps, z1, z2)
+    assert rel(fpp, po.bandpass(pp, z1, z2)) < TOL
+    assert rel(fps, po.bandpass(ps, z1, z2)) < TOL
