@@ -850,6 +850,13 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tc(WgradArgs a, int *err)
 // contiguous range of chunks (split-K, FP32 atomics at the end).  The bias gradient is
 // k_bias_grad's.  Every wait is bounded.
 // ---------------------------------------------------------------------------------------------
+// dst[0..3] += the four FP32 bit patterns, one 16-byte reduction in L2.
+__device__ __forceinline__ void red_add4(float *dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n" ::"l"(dst), "f"(__uint_as_float(a)),
+               "f"(__uint_as_float(b)), "f"(__uint_as_float(c)), "f"(__uint_as_float(d))
+               : "memory");
+}
+
 constexpr int kWtStages = 4;
 constexpr int kWtHalo = kWgP + 2;                // x pixels per chunk
 // ring space of one x box (66 pixels x 16 B), padded so every box lands on a 128-byte boundary
@@ -991,9 +998,9 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tma(WgradArgs a,
               "=r"(r[7])
             : "r"(taddr));
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        if (co < a.cout) {
-#pragma unroll
-          for (int j = 0; j < 8; j++) atomicAdd(dst + c0 + j, __uint_as_float(r[j]));
+        if (co < a.cout) {  // 16-byte aligned: cin and every layer's offset are multiples of 4
+          red_add4(dst + c0, r[0], r[1], r[2], r[3]);
+          red_add4(dst + c0 + 4, r[4], r[5], r[6], r[7]);
         }
       }
     }
@@ -1024,6 +1031,15 @@ __global__ void __launch_bounds__(256) k_bias_grad(const bf16 *dz, int zcs, int 
       for (int q = 0; q < 8; q++)
         acc[q] += __uint_as_float((q & 1) ? (wv[q >> 1] & 0xffff0000u) : (wv[q >> 1] << 16));
     }
+  }
+  // lanes of a warp that hold the same group (g is a power of two, at least 4; threads without
+  // pixels add zeros), then one shared add per warp and group
+  if (g < 32) {
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+      for (int o = g; o < 32; o <<= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+  }
+  if (g >= 32 ? lp < per : (threadIdx.x & 31) < g) {
 #pragma unroll
     for (int q = 0; q < 8; q++) atomicAdd(&s_db[cg * 8 + q], acc[q]);
   }
@@ -1529,7 +1545,11 @@ int wgrad(ds2d_unet *u, const ds2d_unet::Layer &L, const bf16 *dz, int zcs, cons
       return unet_fail(u, DS2D_E_CUDA, "wgrad: cuTensorMapEncodeTiled failed");
     const long long tchunks = (long long)n * h * ((wd + kWgP - 1) / kWgP);
     const long long ttiles = (long long)((L.cout + kWgM - 1) / kWgM) * (L.cin_pad / kn) * 3;
-    long long ts = (4 * 148 + ttiles - 1) / ttiles;
+    // Splits of the pixel range: as many CTAs as are resident at once (TMEM and shared memory hold
+    // one per SM with 96 or 128 input channels, two below).  More only add epilogues, each of
+    // which adds its whole 128 x 3 kN tile to the gradient in L2.
+    const long long resident = 148 * (kn >= 96 ? 1 : 2);
+    long long ts = resident / ttiles;
     ts = ts > tchunks ? tchunks : (ts < 1 ? 1 : ts);
     a.chunks_per_cta = (int)((tchunks + ts - 1) / ts);
     ts = (tchunks + a.chunks_per_cta - 1) / a.chunks_per_cta;
@@ -1545,7 +1565,7 @@ int wgrad(ds2d_unet *u, const ds2d_unet::Layer &L, const bf16 *dz, int zcs, cons
     else
       k_conv3x3_wgrad_tma<16><<<tgrid, 128, wt_smem_bytes<16>(), u->stream>>>(a, tz, tx, u->d_err);
     const long long npx = (long long)n * h * wd;
-    const unsigned bb = nblk(npx * (L.cout / 8)) < 148u * 4 ? nblk(npx * (L.cout / 8)) : 148u * 4;
+    const unsigned bb = nblk(npx * (L.cout / 8)) < 148u * 2 ? nblk(npx * (L.cout / 8)) : 148u * 2;
     k_bias_grad<<<bb, 256, 0, u->stream>>>(dz, zcs, L.cout, npx, a.db);
     UCK(cudaGetLastError());
     return DS2D_OK;
