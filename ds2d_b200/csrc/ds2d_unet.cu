@@ -21,6 +21,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -167,6 +168,7 @@ __global__ void __launch_bounds__(64 * (kCo / 32)) k_conv3x3(ConvArgs a) {
 constexpr int kTcM = 128;              // pixels per CTA (UMMA M)
 constexpr int kTcHalo = kTcM + 2;      // halo pixels per staged row
 constexpr int kTcPlaneA = kTcHalo * 16;  // bytes of one (row, channel-half) plane
+constexpr int kConvLayers = 14;           // 3x3 layers of the network
 constexpr int kTcSpin = 1 << 24;       // bound on every mbarrier wait
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
@@ -181,6 +183,20 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
   d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
   d |= (uint64_t)1 << 46;  // descriptor version for sm_100
   return d;                // base offset 0, legacy LBO mode, layout type 0 (no swizzle)
+}
+
+// K-major with rows of kCK channels (32- or 64-byte swizzle): groups of 8 rows `sbo` bytes apart.
+template <int kCK>
+__device__ __forceinline__ uint64_t umma_desc_sw(uint32_t saddr, uint32_t sbo) {
+  static_assert(kCK == 16 || kCK == 32, "rows of 32 or 64 bytes");
+  return umma_desc(saddr, 16, sbo) | (uint64_t)(kCK == 16 ? 6 : 4) << 61;
+}
+
+// MN-major blocks of kC channels (32 or 16) with one row of kC channels per K index: blocks `lbo`
+// bytes apart along M / N, groups of 8 K indices contiguous.
+template <int kC>
+__device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr, uint32_t lbo) {
+  return umma_desc(saddr, lbo, 8 * kC * 2) | (uint64_t)(kC == 16 ? 6 : 4) << 61;
 }
 
 // Instruction descriptor: BF16 x BF16 -> FP32, both K-major, M x N.
@@ -343,33 +359,38 @@ constexpr int tc_smem_bytes() {
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same convolution fed by the tensor-memory accelerator through a kS-stage ring (option
-// "tcgen05_tma").  Per 16-channel chunk, one thread issues the tiled bulk-tensor loads of the
-// kR + 2 halo rows (box: 8 channels x 130 pixels per channel half, out-of-image pixels and rows
-// filled with zeros by the copy engine) and of the 9 x 2 weight planes (one box of the blocked
-// weights: 8 input channels x kN output channels x 18 planes) into a free stage, counted on the
-// stage's "full" mbarrier; a second thread
-// waits for the stage, issues the stage's 9 kR UMMAs and commits them to its "empty" mbarrier,
-// which frees the stage for the loads kS chunks later.  The boxes land in the K-major no-swizzle
-// layout the descriptors of k_conv3x3_tc read (16-byte rows, one plane per channel half), so the
-// MMAs and the epilogue are that kernel's.  Every wait is bounded.
+// The same convolution fed by the tensor-memory accelerator (option "tcgen05_tma").  A CTA owns kJ
+// M-tiles of 8 pixels x 16 rows side by side (8 kJ x 16 output pixels) and kN output channels.  Per
+// stage of kCK input channels one thread issues ONE tiled bulk-tensor load of the (8 kJ + 2) x 18
+// halo box, whose rows are the kCK channels of a pixel (32 or 64 bytes, whole sectors) in the
+// 32- or 64-byte swizzle that the A descriptor names, and one bulk copy of the stage's weights
+// (contiguous: blocked by output tile).  An M-tile's 16 groups of 8 pixels are the 16 image rows of
+// the box, so the descriptor's group stride is the box's row pitch and every tap (and M-tile) is an
+// offset of its start address: (ky (8 kJ + 2) + kx + 8 j) pixels.  The swizzle acts on the address
+// bits, so the offsets need no alignment.  The MMAs keep the order of k_conv3x3_tc (16-channel
+// chunks, then taps), so the two give the same bits.  A second thread issues the MMAs; every wait
+// is bounded.
+//
+// Why this tile: widths are multiples of 8 but rarely of 128, and the deeper levels are 152, 76 or 32
+// pixels wide, so M-tiles along one image row did 1.05-4 times the work; the halo is 1.2 pixels per
+// output pixel for kJ = 4 against 1.52 for four rows of 130; and a box row of 8 channels (16 bytes,
+// half a sector) was one L2 request each, which set the pace.
 // ---------------------------------------------------------------------------------------------
-// A plane of a halo row in the ring: the 130 x 16-byte box rows, padded to a multiple of 128 bytes
-// so every bulk-tensor destination starts on a 128-byte boundary (the descriptors' LBO).
-constexpr int kTmaPlaneA = (kTcPlaneA + 127) / 128 * 128;
-// Bytes the loads of one stage deliver (the mbarrier's transaction count) and the stage's size.
-template <int kN, int kR>
-__host__ __device__ constexpr int tma_tx_bytes() {
-  return (kR + 2) * 2 * kTcPlaneA + 9 * 2 * kN * 16;
+constexpr int kTileH = 16;  // output rows of a CTA's tile
+template <int kJ>
+__host__ __device__ constexpr int cv_pitch() { return 8 * kJ + 2; }  // halo pixels per box row
+template <int kJ, int kCK>
+__host__ __device__ constexpr int cv_a_bytes() { return cv_pitch<kJ>() * (kTileH + 2) * kCK * 2; }
+template <int kN, int kCK>
+__host__ __device__ constexpr int cv_b_bytes() { return 9 * 2 * kN * 16 * (kCK / 16); }
+template <int kN, int kJ, int kCK>
+__host__ __device__ constexpr int cv_stage_bytes() {
+  return (cv_a_bytes<kJ, kCK>() + 1023) / 1024 * 1024 + (cv_b_bytes<kN, kCK>() + 1023) / 1024 * 1024;
 }
-template <int kN, int kR>
-__host__ __device__ constexpr int tma_stage_bytes() {
-  return (kR + 2) * 2 * kTmaPlaneA + 9 * 2 * kN * 16;
-}
-template <int kN, int kR, int kS>
-__host__ __device__ constexpr int tma_smem_bytes() {
-  // stages, 1024-aligned, then the barriers (2 per stage + 1)
-  return kS * ((tma_stage_bytes<kN, kR>() + 1023) / 1024 * 1024) + 8 * (2 * kS + 1);
+constexpr int kCvMaxStages = 3;
+template <int kN, int kJ, int kCK>
+constexpr int cv_smem_bytes(int stages) {
+  return 1024 + stages * cv_stage_bytes<kN, kJ, kCK>() + 8 * (2 * kCvMaxStages + 1);
 }
 
 __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity) {
@@ -385,30 +406,45 @@ __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity) {
   return done != 0;
 }
 
-template <int kN, int kR, int kS>
+__device__ __forceinline__ void tmem_ld32(uint32_t (&r)[32], uint32_t taddr) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
+        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+}
+
+template <int kN, int kJ, int kCK>
 __global__ void __launch_bounds__(128) k_conv3x3_tma(ConvArgs a, const __grid_constant__ CUtensorMap tmA,
-                                                     const __grid_constant__ CUtensorMap tmB,
-                                                     int *err) {
-  extern __shared__ __align__(1024) unsigned char tm_smem[];
-  constexpr int kStage = (tma_stage_bytes<kN, kR>() + 1023) / 1024 * 1024;
-  uint64_t *full = reinterpret_cast<uint64_t *>(tm_smem + kS * kStage);
-  uint64_t *empty = full + kS;
-  uint64_t *done = empty + kS;
+                                                     const bf16 *wblk, int stages, int *err) {
+  extern __shared__ unsigned char cv_raw[];
+  unsigned char *sm = cv_raw + ((1024 - (smem_u32(cv_raw) & 1023)) & 1023);
+  constexpr int kStage = cv_stage_bytes<kN, kJ, kCK>();
+  constexpr int kA = (cv_a_bytes<kJ, kCK>() + 1023) / 1024 * 1024, kP = cv_pitch<kJ>();
+  uint64_t *full = reinterpret_cast<uint64_t *>(sm + stages * kStage);
+  uint64_t *empty = full + kCvMaxStages;
+  uint64_t *done = empty + kCvMaxStages;
   __shared__ uint32_t tmem_base;
   __shared__ int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int w0 = blockIdx.x * kTcM, row0 = blockIdx.y * kR;
+  const int w0 = blockIdx.x * (8 * kJ), row0 = blockIdx.y * kTileH;
   const int ngrp = a.cout / kN;
-  const int img = blockIdx.z / ngrp, co0 = (blockIdx.z % ngrp) * kN;
-  constexpr uint32_t kCols = kR * kN <= 32 ? 32 : kR * kN <= 64 ? 64 : kR * kN <= 128 ? 128
-                           : kR * kN <= 256 ? 256 : 512;
+  const int img = blockIdx.z / ngrp, grp = blockIdx.z % ngrp, co0 = grp * kN;
+  constexpr uint32_t kCols = kJ * kN <= 32 ? 32 : kJ * kN <= 64 ? 64 : kJ * kN <= 128 ? 128
+                           : kJ * kN <= 256 ? 256 : 512;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                      smem_u32(&tmem_base)), "r"(kCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
   if (tid == 0) {
-    for (int k = 0; k < 2 * kS + 1; k++)
+    for (int k = 0; k < 2 * kCvMaxStages + 1; k++)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(full + k)));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     s_fail = 0;
@@ -418,64 +454,61 @@ __global__ void __launch_bounds__(128) k_conv3x3_tma(ConvArgs a, const __grid_co
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
   const uint32_t tmem = tmem_base;
   constexpr uint32_t idesc = umma_idesc(kTcM, kN);
-  const int nch = a.cin / 16;
+  const int nst = a.cin / kCK;  // stages of work
   if (tid == 0) {
-    // producer: tiled bulk-tensor loads of chunk c into stage c mod kS
-    const uint64_t ta = reinterpret_cast<uint64_t>(&tmA), tb = reinterpret_cast<uint64_t>(&tmB);
-    for (int c = 0; c < nch; c++) {
-      const int st = c % kS, k = c / kS;
-      if (c >= kS && !tc_wait(empty + st, (k - 1) & 1)) {
+    const uint64_t ta = reinterpret_cast<uint64_t>(&tmA);
+    const unsigned char *wsrc =
+        reinterpret_cast<const unsigned char *>(wblk) + (size_t)grp * (a.cin / 16) * (18 * kN * 16);
+    for (int c = 0; c < nst; c++) {
+      const int st = c % stages, k = c / stages;
+      if (c >= stages && !tc_wait(empty + st, (k - 1) & 1)) {
         s_fail = 1;
         break;
       }
-      unsigned char *sA = tm_smem + st * kStage, *sB = sA + (kR + 2) * 2 * kTmaPlaneA;
+      unsigned char *sA = sm + st * kStage;
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(
                        smem_u32(full + st)),
-                   "r"((uint32_t)tma_tx_bytes<kN, kR>())
+                   "r"((uint32_t)(cv_a_bytes<kJ, kCK>() + cv_b_bytes<kN, kCK>()))
                    : "memory");
-      const int ci0 = c * 16;
-      for (int r = 0; r < kR + 2; r++)
-        for (int kh = 0; kh < 2; kh++)
-          asm volatile(
-              "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-              " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(
-                  smem_u32(sA + (r * 2 + kh) * kTmaPlaneA)),
-              "l"(ta), "r"(ci0 + 8 * kh), "r"(w0 - 1), "r"(row0 + r - 1), "r"(img),
-              "r"(smem_u32(full + st))
-              : "memory");
-      // the chunk's 9 x 2 weight planes of this output tile: one box of the blocked weights
       asm volatile(
-          "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-          " [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(smem_u32(sB)),
-          "l"(tb), "r"(0), "r"(co0), "r"(18 * c), "r"(smem_u32(full + st))
+          "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+          " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(smem_u32(sA)),
+          "l"(ta), "r"(c * kCK), "r"(w0 - 1), "r"(row0 - 1), "r"(img), "r"(smem_u32(full + st))
+          : "memory");
+      asm volatile(
+          "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+              smem_u32(sA + kA)),
+          "l"(wsrc + (size_t)c * cv_b_bytes<kN, kCK>()), "r"((uint32_t)cv_b_bytes<kN, kCK>()),
+          "r"(smem_u32(full + st))
           : "memory");
     }
   } else if (tid == 32) {
-    // MMA issuer: the stage's 9 kR UMMAs, then a commit that frees the stage
-    for (int c = 0; c < nch; c++) {
-      const int st = c % kS, k = c / kS;
+    for (int c = 0; c < nst; c++) {
+      const int st = c % stages, k = c / stages;
       if (!tc_wait(full + st, k & 1)) {
         s_fail = 1;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-      const uint32_t a_base = smem_u32(tm_smem + st * kStage);
-      const uint32_t b_base = a_base + (kR + 2) * 2 * kTmaPlaneA;
+      const uint32_t a_base = smem_u32(sm + st * kStage), b_base = a_base + kA;
 #pragma unroll
-      for (int j = 0; j < kR; j++)
+      for (int k2 = 0; k2 < kCK / 16; k2++)
 #pragma unroll
-        for (int tap = 0; tap < 9; tap++) {
-          const int ky = tap / 3, kx = tap % 3;
-          const uint64_t ad =
-              umma_desc(a_base + ((j + ky) * 2) * kTmaPlaneA + kx * 16, kTmaPlaneA, 128);
-          const uint64_t bd = umma_desc(b_base + (tap * 2) * (kN * 16), kN * 16, 128);
-          const uint32_t acc = (c > 0 || tap > 0) ? 1u : 0u;
-          asm volatile(
-              "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-                  tmem + (uint32_t)(j * kN)),
-              "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-        }
+        for (int j = 0; j < kJ; j++)
+#pragma unroll
+          for (int tap = 0; tap < 9; tap++) {
+            const int ky = tap / 3, kx = tap % 3;
+            const uint64_t ad = umma_desc_sw<kCK>(
+                a_base + (ky * kP + kx + 8 * j) * (kCK * 2) + k2 * 32, kP * kCK * 2);
+            const uint64_t bd =
+                umma_desc(b_base + ((k2 * 9 + tap) * 2) * (kN * 16), kN * 16, 128);
+            const uint32_t acc = (c > 0 || k2 > 0 || tap > 0) ? 1u : 0u;
+            asm volatile(
+                "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+                    tmem + (uint32_t)(j * kN)),
+                "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+          }
       asm volatile(
           "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
               smem_u32(empty + st)));
@@ -490,42 +523,38 @@ __global__ void __launch_bounds__(128) k_conv3x3_tma(ConvArgs a, const __grid_co
   ok = __syncthreads_and(ok && !s_fail);
   if (!ok && tid == 0) atomicExch(err, 1);
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-  for (int j = 0; j < kR && ok; j++) {
-    const int row = row0 + j;
-    const int m = warp * 32 + lane;
-    const int ww = w0 + m;
+  // epilogue: thread (warp w, lane l) owns pixel m = 32 w + l of each M-tile: row m / 8, column m % 8
+  const int m = warp * 32 + lane, row = row0 + (m >> 3);
+  for (int j = 0; j < kJ && ok; j++) {
+    const int ww = w0 + 8 * j + (m & 7);
+    const bool in = ww < a.w && row < a.h;
     const long long obase = (((long long)img * a.h + row) * a.w + ww) * a.ocs + a.oco + co0;
 #pragma unroll 1
-    for (int c0 = 0; c0 < kN; c0 += 8) {
-      uint32_t r[8];
-      const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * kN + c0);
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
-          : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-            "=r"(r[7])
-          : "r"(taddr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-      if (ww < a.w && row < a.h) {
+    for (int c0 = 0; c0 < kN; c0 += 32) {
+      uint32_t r[32];
+      tmem_ld32(r, tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * kN + c0));
+      if (!in) continue;
+#pragma unroll
+      for (int g = 0; g < 4; g++) {
         float v[8];
+        const long long o = obase + c0 + 8 * g;
 #pragma unroll
         for (int q = 0; q < 8; q++) {
-          v[q] = __uint_as_float(r[q]) + (a.bias ? a.bias[co0 + c0 + q] : 0.f);
+          v[q] = __uint_as_float(r[8 * g + q]) + (a.bias ? __ldg(a.bias + co0 + c0 + 8 * g + q) : 0.f);
           if (a.relu) v[q] = fmaxf(v[q], 0.f);
         }
-        const long long o = obase + c0;
         if (a.mask) {
+          const uint4 mk = *reinterpret_cast<const uint4 *>(a.mask + o);
 #pragma unroll
-          for (int q = 0; q < 8; q++)
-            if (!(__bfloat162float(a.mask[o + q]) > 0.f)) v[q] = 0.f;
+          for (int q = 0; q < 8; q++) {
+            const uint32_t w = (&mk.x)[q >> 1];
+            if (!(__uint_as_float((q & 1) ? (w & 0xffff0000u) : (w << 16)) > 0.f)) v[q] = 0.f;
+          }
         }
         __nv_bfloat162 pk[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) pk[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
         *reinterpret_cast<uint4 *>(a.out + o) = *reinterpret_cast<uint4 *>(pk);
-        if (a.out_f32) {
-#pragma unroll
-          for (int q = 0; q < 8; q++) a.out_f32[o + q] = v[q];
-        }
       }
     }
   }
@@ -837,18 +866,20 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tc(WgradArgs a, int *err)
 // ---------------------------------------------------------------------------------------------
 // The weight gradient with both operands MN-major (option "tcgen05_wgrad_tma"): in the product
 // dW[tap][co][ci] = sum_p dz[p][co] x[p + tap][ci] the reduction runs over pixels, and the NHWC
-// activations hold the M (co) and N (ci) indices contiguous, so a tiled bulk-tensor box of
-// 8 channels x P pixels lands as one 8-channel column of the canonical MN-major no-swizzle layout
-// (16-byte rows of 8 channels, one per pixel; 8-pixel core matrices 128 bytes apart along K,
-// channel groups one box (x: one 128-byte-padded box) apart along M / N).  No transposition passes through the threads: one
-// thread issues the boxes of a 64-pixel row chunk into a kS-stage ring (dz: up to 16 channel
-// groups; x: the kN / 8 groups of 66 pixels, w0 - 1 .. w0 + 64, of row r + ky - 1, the copy engine
-// filling pixels and rows outside the image with zeros), a second thread issues the chunk's
-// 3 x 4 UMMAs (M 128 output channels, N kN input channels, K 16 pixels; the shift kx is a
-// 16-byte offset of the B descriptor along K) and commits them to the stage's "empty" barrier.
-// A CTA owns 128 output channels x kN input channels x the three taps of one kernel row and a
-// contiguous range of chunks (split-K, FP32 atomics at the end).  The bias gradient is
-// k_bias_grad's.  Every wait is bounded.
+// activations hold the M (co) and N (ci) indices contiguous, so a tiled bulk-tensor box of 32
+// channels x P pixels (16 channels for x in the first layer) lands as one 32-channel block of the
+// canonical MN-major layout with 64-byte (32-byte) swizzle: one row of 64 bytes per pixel, 8-pixel
+// groups 512 bytes apart along K, channel blocks one box apart along M / N.  No transposition
+// passes through the threads: one thread issues the boxes of a 64-pixel row chunk into a 4-stage
+// ring (dz: up to 4 blocks; x: 66 pixels, w0 - 1 .. w0 + 64, of row r + ky - 1, the copy engine
+// filling pixels and rows outside the image with zeros), a second thread issues the chunk's 3 x 4
+// UMMAs (M 128 output channels, N kN input channels, K 16 pixels; the shift kx is one row of the B
+// descriptor's start address: the swizzle acts on address bits) and commits them to the stage's
+// "empty" barrier.  With 32 output channels three quarters of M read whatever the stage holds and
+// are dropped.  A CTA owns 128 output channels x kN input channels x the three taps of one kernel
+// row and a contiguous range of chunks (split-K, FP32 reductions in L2 at the end).  The bias
+// gradient is k_bias_grad's.  Every wait is bounded.  Boxes of 8 channels (16-byte rows, half a
+// sector each) made the requests set the pace: 96 -> 32 channels at 8 x 128x256 pixels, 94 us.
 // ---------------------------------------------------------------------------------------------
 // dst[0..3] += the four FP32 bit patterns, one 16-byte reduction in L2.
 __device__ __forceinline__ void red_add4(float *dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -859,15 +890,19 @@ __device__ __forceinline__ void red_add4(float *dst, uint32_t a, uint32_t b, uin
 
 constexpr int kWtStages = 4;
 constexpr int kWtHalo = kWgP + 2;                // x pixels per chunk
-// ring space of one x box (66 pixels x 16 B), padded so every box lands on a 128-byte boundary
-constexpr int kWtXPlane = (kWtHalo * 16 + 127) / 128 * 128;
+constexpr int kWtZ = kWgP * 64;                  // bytes of a dz block: 64 pixels x 32 channels
+template <int kN>
+__host__ __device__ constexpr int wt_xc() { return kN < 32 ? kN : 32; }  // channels of an x block
+// ring space of one x block, a multiple of the swizzle's 512-byte period
+template <int kN>
+__host__ __device__ constexpr int wt_x() { return (kWtHalo * wt_xc<kN>() * 2 + 511) / 512 * 512; }
 template <int kN>
 __host__ __device__ constexpr int wt_stage_bytes() {
-  return ((16 * kWgP * 16 + (kN / 8) * kWtXPlane) + 1023) / 1024 * 1024;
+  return (4 * kWtZ + (kN / wt_xc<kN>()) * wt_x<kN>() + 1023) / 1024 * 1024;
 }
 template <int kN>
 __host__ __device__ constexpr int wt_smem_bytes() {
-  return kWtStages * wt_stage_bytes<kN>() + 8 * (2 * kWtStages + 1);
+  return 1024 + kWtStages * wt_stage_bytes<kN>() + 8 * (2 * kWtStages + 1);
 }
 
 template <int kN>
@@ -875,9 +910,9 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tma(WgradArgs a,
                                                            const __grid_constant__ CUtensorMap tmZ,
                                                            const __grid_constant__ CUtensorMap tmX,
                                                            int *err) {
-  extern __shared__ __align__(1024) unsigned char wt_smem[];
-  constexpr int kStage = wt_stage_bytes<kN>();
-  constexpr int kZBytes = 16 * kWgP * 16;   // dz: 16 channel groups x 64 pixels x 16 B
+  extern __shared__ unsigned char wt_raw[];
+  unsigned char *wt_smem = wt_raw + ((1024 - (smem_u32(wt_raw) & 1023)) & 1023);
+  constexpr int kStage = wt_stage_bytes<kN>(), kXC = wt_xc<kN>(), kXB = kN / kXC;
   uint64_t *full = reinterpret_cast<uint64_t *>(wt_smem + kWtStages * kStage);
   uint64_t *empty = full + kWtStages;
   uint64_t *done = empty + kWtStages;
@@ -886,7 +921,7 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tma(WgradArgs a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int co0 = blockIdx.x * kWgM;
   const int ci0 = (blockIdx.y / 3) * kN, ky = blockIdx.y % 3;
-  const int gz = (a.cout - co0) / 8 < 16 ? (a.cout - co0) / 8 : 16;  // dz channel groups loaded
+  const int gz = (a.cout - co0) / 32 < 4 ? (a.cout - co0) / 32 : 4;  // dz blocks loaded
   constexpr uint32_t kCols = 3 * kN <= 32 ? 32 : 3 * kN <= 64 ? 64 : 3 * kN <= 128 ? 128
                            : 3 * kN <= 256 ? 256 : 512;
   if (warp == 0) {
@@ -914,7 +949,7 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tma(WgradArgs a,
   if (tid == 0) {
     // producer
     const uint64_t tz = reinterpret_cast<uint64_t>(&tmZ), tx = reinterpret_cast<uint64_t>(&tmX);
-    const uint32_t tx_bytes = (uint32_t)(gz * kWgP * 16 + (kN / 8) * kWtHalo * 16);
+    const uint32_t tx_bytes = (uint32_t)(gz * kWtZ + kN * kWtHalo * 2);
     for (int i = 0; i < nck; i++) {
       const int st = i % kWtStages, k = i / kWtStages;
       if (i >= kWtStages && !tc_wait(empty + st, (k - 1) & 1)) {
@@ -926,7 +961,7 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tma(WgradArgs a,
       const long long rr = cidx / wchunks;
       const int row = (int)(rr % a.h), img = (int)(rr / a.h);
       const int w0 = wc * kWgP;
-      unsigned char *sZ = wt_smem + st * kStage, *sX = sZ + kZBytes;
+      unsigned char *sZ = wt_smem + st * kStage, *sX = sZ + 4 * kWtZ;
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(
                        smem_u32(full + st)),
                    "r"(tx_bytes)
@@ -934,14 +969,14 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tma(WgradArgs a,
       for (int g = 0; g < gz; g++)
         asm volatile(
             "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-            " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(smem_u32(sZ + g * (kWgP * 16))),
-            "l"(tz), "r"(co0 + 8 * g), "r"(w0), "r"(row), "r"(img), "r"(smem_u32(full + st))
+            " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(smem_u32(sZ + g * kWtZ)),
+            "l"(tz), "r"(co0 + 32 * g), "r"(w0), "r"(row), "r"(img), "r"(smem_u32(full + st))
             : "memory");
-      for (int g = 0; g < kN / 8; g++)
+      for (int g = 0; g < kXB; g++)
         asm volatile(
             "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-            " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(smem_u32(sX + g * kWtXPlane)),
-            "l"(tx), "r"(ci0 + 8 * g), "r"(w0 - 1), "r"(row + ky - 1), "r"(img),
+            " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(smem_u32(sX + g * wt_x<kN>())),
+            "l"(tx), "r"(ci0 + kXC * g), "r"(w0 - 1), "r"(row + ky - 1), "r"(img),
             "r"(smem_u32(full + st))
             : "memory");
     }
@@ -955,13 +990,13 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tma(WgradArgs a,
       }
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
       const uint32_t z_base = smem_u32(wt_smem + st * kStage);
-      const uint32_t x_base = z_base + kZBytes;
+      const uint32_t x_base = z_base + 4 * kWtZ;
 #pragma unroll
       for (int kx = 0; kx < 3; kx++)
 #pragma unroll
         for (int s = 0; s < kWgP / 16; s++) {
-          const uint64_t ad = umma_desc(z_base + s * 256, 128, kWgP * 16);
-          const uint64_t bd = umma_desc(x_base + kx * 16 + s * 256, 128, kWtXPlane);
+          const uint64_t ad = umma_desc_mn<32>(z_base + s * (16 * 64), kWtZ);
+          const uint64_t bd = umma_desc_mn<kXC>(x_base + (kx + 16 * s) * (kXC * 2), wt_x<kN>());
           const uint32_t acc = (i > 0 || s > 0) ? 1u : 0u;
           asm volatile(
               "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
@@ -1013,38 +1048,45 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tma(WgradArgs a,
   }
 }
 
-// Bias gradient db[co] += sum_p dz[p][co] (dz [P][zcs], cout channels): each thread sums one
-// 8-channel group over a strided set of pixels, then shared and global atomics.
-__global__ void __launch_bounds__(256) k_bias_grad(const bf16 *dz, int zcs, int cout, long long npx,
-                                                   float *db) {
+// Bias gradients db[co] += sum_p dz[p][co] (dz [P][cout]) of all layers in one launch (grid.y = layer:
+// their output gradients all stay in memory): each thread sums one 8-channel group over a strided
+// set of pixels; lanes of a warp that hold the same group add up by shuffles, then warps in shared
+// memory and CTAs in global memory.
+struct BiasLayer {
+  const bf16 *dz;
+  float *db;
+  long long npx;
+  int cout;
+};
+struct BiasArgs {
+  BiasLayer l[kConvLayers];
+};
+__global__ void __launch_bounds__(256) k_bias_grad(const __grid_constant__ BiasArgs a) {
   __shared__ float s_db[512];  // cout <= 512 (base channels <= 64)
-  for (int i = threadIdx.x; i < cout; i += blockDim.x) s_db[i] = 0.f;
+  const BiasLayer &L = a.l[blockIdx.y];
+  const int cout = L.cout;
+  for (int i = threadIdx.x; i < cout; i += 256) s_db[i] = 0.f;
   __syncthreads();
-  const int g = cout / 8, per = blockDim.x / g;  // threads per channel group
+  const int g = cout / 8, per = 256 / g;  // threads per channel group; g is a power of two, 4 .. 64
   const int cg = threadIdx.x % g, lp = threadIdx.x / g;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (lp < per) {
-    for (long long p = (long long)blockIdx.x * per + lp; p < npx; p += (long long)gridDim.x * per) {
-      const uint4 v = *reinterpret_cast<const uint4 *>(dz + p * zcs + cg * 8);
-      const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int q = 0; q < 8; q++)
-        acc[q] += __uint_as_float((q & 1) ? (wv[q >> 1] & 0xffff0000u) : (wv[q >> 1] << 16));
-    }
-  }
-  // lanes of a warp that hold the same group (g is a power of two, at least 4; threads without
-  // pixels add zeros), then one shared add per warp and group
-  if (g < 32) {
+#pragma unroll 4
+  for (long long p = (long long)blockIdx.x * per + lp; p < L.npx; p += (long long)gridDim.x * per) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(L.dz + p * cout + cg * 8);
+    const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int q = 0; q < 8; q++)
-      for (int o = g; o < 32; o <<= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+      acc[q] += __uint_as_float((q & 1) ? (wv[q >> 1] & 0xffff0000u) : (wv[q >> 1] << 16));
   }
-  if (g >= 32 ? lp < per : (threadIdx.x & 31) < g) {
+#pragma unroll
+  for (int q = 0; q < 8; q++)
+    for (int o = g; o < 32; o <<= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+  if (g >= 32 || (threadIdx.x & 31) < g) {
 #pragma unroll
     for (int q = 0; q < 8; q++) atomicAdd(&s_db[cg * 8 + q], acc[q]);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < cout; i += blockDim.x) atomicAdd(db + i, s_db[i]);
+  for (int i = threadIdx.x; i < cout; i += 256) atomicAdd(L.db + i, s_db[i]);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1082,7 +1124,8 @@ __global__ void k_pack_input(const float *x, bf16 *out, long long npx) {
 
 // 2x2 average pooling, [N][H][W][C] -> [N][H/2][W/2][C]:
 // y = 0.25 (x[2y][2x] + x[2y][2x+1] + x[2y+1][2x] + x[2y+1][2x+1])
-__global__ void k_pool(const bf16 *x, bf16 *y, int n, int h, int w, int c) {
+// (x at pixel stride xs)
+__global__ void k_pool(const bf16 *x, int xs, bf16 *y, int n, int h, int w, int c) {
   const int h2 = h / 2, w2 = w / 2, g = c / 8;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= w2 * g) return;
@@ -1090,9 +1133,9 @@ __global__ void k_pool(const bf16 *x, bf16 *y, int n, int h, int w, int c) {
   for (long long r = blockIdx.y; r < (long long)n * h2; r += gridDim.y) {
     const long long im = r / h2;
     const int yy = (int)(r - im * h2);
-    const long long b = ((im * h + 2 * yy) * w + 2 * xx) * c + cg * 8;
-    const uint4 v0 = ld16(x + b), v1 = ld16(x + b + c), v2 = ld16(x + b + (long long)w * c),
-                v3 = ld16(x + b + (long long)w * c + c);
+    const long long b = ((im * h + 2 * yy) * w + 2 * xx) * xs + cg * 8;
+    const uint4 v0 = ld16(x + b), v1 = ld16(x + b + xs), v2 = ld16(x + b + (long long)w * xs),
+                v3 = ld16(x + b + (long long)w * xs + xs);
     float f[8];
 #pragma unroll
     for (int q = 0; q < 8; q++) f[q] = 0.25f * (bfe(v0, q) + bfe(v1, q) + bfe(v2, q) + bfe(v3, q));
@@ -1101,9 +1144,10 @@ __global__ void k_pool(const bf16 *x, bf16 *y, int n, int h, int w, int c) {
 }
 
 // d(skip) = pool_grad(dy) * (s > 0) + extra, where extra (the skip's gradient through the
-// decoder concatenation, already masked) is read at channel offset `eco` of stride `ecs`.
-__global__ void k_pool_grad(const bf16 *dy, const bf16 *s, const bf16 *extra, int ecs, int eco,
-                            bf16 *dx, int n, int h, int w, int c) {
+// decoder concatenation, already masked) is read at channel offset `eco` of stride `ecs`; s at
+// stride ss.
+__global__ void k_pool_grad(const bf16 *dy, const bf16 *s, int ss, const bf16 *extra, int ecs,
+                            int eco, bf16 *dx, int n, int h, int w, int c) {
   const int g = c / 8;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= w * g) return;
@@ -1113,7 +1157,7 @@ __global__ void k_pool_grad(const bf16 *dy, const bf16 *s, const bf16 *extra, in
     const int yy = (int)(r - im * h);
     const long long px = r * w + xx;
     const long long j = ((im * (h / 2) + yy / 2) * (w / 2) + xx / 2) * c + cg * 8;
-    const uint4 vs = ld16(s + px * c + cg * 8), vd = ld16(dy + j);
+    const uint4 vs = ld16(s + px * ss + cg * 8), vd = ld16(dy + j);
     uint4 ve = make_uint4(0, 0, 0, 0);
     if (extra) ve = ld16(extra + px * ecs + eco + cg * 8);
     float f[8];
@@ -1126,20 +1170,23 @@ __global__ void k_pool_grad(const bf16 *dy, const bf16 *s, const bf16 *extra, in
   }
 }
 
-// Decoder input: out[.., 0:cu] = up2(u) (nearest), out[.., cu:cu+cs] = s; out [N][H][W][cu+cs]
-__global__ void k_up_concat(const bf16 *u, int cu, const bf16 *s, int cs, bf16 *out, int n, int h,
-                            int w) {
-  const int gu = cu / 8, g = (cu + cs) / 8;
+// Upsampled part of a decoder input: out[.., 0:cu] = up2(u) (nearest), out at pixel stride os.  A
+// thread reads 8 channels of a pixel once and writes its four children; the skip part of the input
+// is written in place by the encoder's convolution.
+__global__ void k_up(const bf16 *u, int cu, bf16 *out, int os, int n, int h, int w) {
+  const int h2 = h / 2, w2 = w / 2, g = cu / 8;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= w * g) return;
+  if (t >= w2 * g) return;
   const int xx = t / g, cg = t - xx * g;
-  for (long long r = blockIdx.y; r < (long long)n * h; r += gridDim.y) {
-    const long long im = r / h;
-    const int yy = (int)(r - im * h);
-    const long long px = r * w + xx;
-    const uint4 v = cg < gu ? ld16(u + ((im * (h / 2) + yy / 2) * (w / 2) + xx / 2) * cu + cg * 8)
-                            : ld16(s + px * cs + (cg - gu) * 8);
-    st16(out + px * (cu + cs) + cg * 8, v);
+  for (long long r = blockIdx.y; r < (long long)n * h2; r += gridDim.y) {
+    const long long im = r / h2;
+    const int yy = (int)(r - im * h2);
+    const uint4 v = ld16(u + (r * w2 + xx) * cu + cg * 8);
+    bf16 *o = out + ((im * h + 2 * yy) * w + 2 * xx) * os + cg * 8;
+    st16(o, v);
+    st16(o + os, v);
+    st16(o + (long long)w * os, v);
+    st16(o + (long long)w * os + os, v);
   }
 }
 
@@ -1260,25 +1307,33 @@ __global__ void k_adam(float *p, const float *g, float *m, float *v, long long n
 // backward-data [tap'][ci][co] with tap' = 8 - tap (spatial flip), and both blocked for the
 // bulk-tensor-fed convolution as [16-channel input chunk][tap][8-channel half][output ch][8], so
 // the B operand of one chunk and output tile (18 planes of kN x 16 bytes) is one box.
-__global__ void k_weights_bf16(const float *w, int k2, int co_n, int ci_real, int cin_pad,
-                               bf16 *wf, bf16 *wb, bf16 *wfb, bf16 *wbb) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)k2 * co_n * cin_pad) return;
-  const int ci = (int)(i % cin_pad);
-  const int co = (int)((i / cin_pad) % co_n);
-  const int tap = (int)(i / ((long long)cin_pad * co_n));
-  const float v = ci < ci_real ? w[((long long)tap * co_n + co) * ci_real + ci] : 0.f;
-  const bf16 b = __float2bfloat16(v);
-  wf[i] = b;
-  // blocked [ci / 16][tap][(ci / 8) & 1][co][ci & 7] (cin_pad a multiple of 16)
-  if (wfb && cin_pad % 16 == 0)
-    wfb[(((long long)(ci / 16) * k2 + tap) * 2 + ((ci >> 3) & 1)) * co_n * 8 + co * 8 + (ci & 7)] = b;
-  if (ci < ci_real) {
-    const int tb = k2 - 1 - tap;
-    if (wb) wb[((long long)tb * ci_real + ci) * co_n + co] = b;
+// One launch for all layers (grid.y).
+struct WeightLayer {
+  const float *w;
+  bf16 *wf, *wb, *wfb, *wbb;
+  int co_n, ci_real, cin_pad, knf, knb;
+};
+struct WeightArgs {
+  WeightLayer l[kConvLayers];
+};
+__global__ void __launch_bounds__(256) k_weights_bf16(const __grid_constant__ WeightArgs a) {
+  const WeightLayer &L = a.l[blockIdx.y];
+  const int n = 9 * L.co_n * L.cin_pad;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+    const int ci = i % L.cin_pad, co = (i / L.cin_pad) % L.co_n, tap = i / (L.cin_pad * L.co_n);
+    const float v = ci < L.ci_real ? L.w[((long long)tap * L.co_n + co) * L.ci_real + ci] : 0.f;
+    const bf16 b = __float2bfloat16(v);
+    L.wf[i] = b;
+    // blocked [co / knf][ci / 16][tap][(ci / 8) & 1][co % knf][ci & 7]
+    L.wfb[((((long long)(co / L.knf) * (L.cin_pad / 16) + ci / 16) * 9 + tap) * 2 + ((ci >> 3) & 1)) * L.knf * 8 +
+          (co % L.knf) * 8 + (ci & 7)] = b;
+    if (ci >= L.ci_real) continue;
+    const int tb = 8 - tap;
+    L.wb[((long long)tb * L.ci_real + ci) * L.co_n + co] = b;
     // backward-data weights blocked the same way, input channels = co, output channels = ci
-    if (wbb && co_n % 16 == 0)
-      wbb[(((long long)(co / 16) * k2 + tb) * 2 + ((co >> 3) & 1)) * ci_real * 8 + ci * 8 + (co & 7)] = b;
+    if (L.wbb)
+      L.wbb[((((long long)(ci / L.knb) * (L.co_n / 16) + co / 16) * 9 + tb) * 2 + ((co >> 3) & 1)) * L.knb * 8 +
+            (ci % L.knb) * 8 + (co & 7)] = b;
   }
 }
 
@@ -1330,6 +1385,8 @@ struct ds2d_unet {
   float *y = nullptr, *dy = nullptr;
   float *g0 = nullptr;  // padded [9][cout][16] weight gradient of the first layer (cin 1 -> 16)
   double *part = nullptr, *h_part = nullptr;
+  char *h_stage = nullptr;    // pinned staging (two chunks) of gradients read by the host
+  cudaEvent_t ev_stage[2] = {};
   std::string err;
   bool weights_dirty = true;
   int use_tc = 1;          // 3x3 convolutions on tcgen05 (1, default) or mma.sync (0)
@@ -1337,7 +1394,6 @@ struct ds2d_unet {
   int tc_wgrad_tma = 1;    // the weight gradient with MN-major bulk-tensor operands
   int tc_rows = 4;         // output rows per CTA of the tcgen05 convolution (1, 2 or 4)
   int tc_tma = 1;          // the tcgen05 convolution fed by tiled bulk-tensor loads (k_conv3x3_tma)
-  int tc_stages = 2;       // ring stages of k_conv3x3_tma (2 or 3)
   int *d_err = nullptr;    // device flag raised by a bounded wait that gave up
   std::vector<void *> allocs;
 };
@@ -1383,63 +1439,59 @@ TmEncodeFn tm_encode_fn() {
   return fn;
 }
 
-// Tensor maps of one convolution: the input [n][h][w][cin] (box 8 channels x 130 pixels, zero
-// fill outside the image) and the blocked weights [cin/16][9][2][cout][8] viewed as
-// {8, cout, 18 cin/16} (box 8 x kn x 18: the whole B operand of a chunk and output tile).
-bool conv_tensor_maps(const ConvArgs &a, const bf16 *wblk, int kn, CUtensorMap *ta,
-                      CUtensorMap *tb) {
+// Tensor map of one convolution's input [n][h][w][cin]: box ck channels x `pitch` pixels x 18 rows,
+// swizzled over the ck channels, zeros outside the image.
+bool conv_tensor_map(const ConvArgs &a, int ck, int pitch, CUtensorMap *ta) {
   TmEncodeFn enc = tm_encode_fn();
   if (!enc) return false;
   const cuuint64_t dA[4] = {(cuuint64_t)a.cin, (cuuint64_t)a.w, (cuuint64_t)a.h, (cuuint64_t)a.n};
   const cuuint64_t sA[3] = {(cuuint64_t)a.cin * 2, (cuuint64_t)a.w * a.cin * 2,
                             (cuuint64_t)a.h * a.w * a.cin * 2};
-  const cuuint32_t bA[4] = {8, (cuuint32_t)kTcHalo, 1, 1}, e4[4] = {1, 1, 1, 1};
-  if (enc(ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)a.in, dA, sA, bA, e4,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return false;
-  const cuuint64_t dB[3] = {8, (cuuint64_t)a.cout, (cuuint64_t)18 * (a.cin / 16)};
-  const cuuint64_t sB[2] = {16, (cuuint64_t)a.cout * 16};
-  const cuuint32_t bB[3] = {8, (cuuint32_t)kn, 18}, e3[3] = {1, 1, 1};
-  return enc(tb, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, (void *)wblk, dB, sB, bB, e3,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+  const cuuint32_t bA[4] = {(cuuint32_t)ck, (cuuint32_t)pitch, kTileH + 2, 1}, e4[4] = {1, 1, 1, 1};
+  return enc(ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)a.in, dA, sA, bA, e4,
+             CU_TENSOR_MAP_INTERLEAVE_NONE,
+             ck == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tensor maps of one weight gradient: dz [n][h][w][zcs] (cout channels; box 8 channels x 64
-// pixels) and x [n][h][w][cin] (box 8 channels x 66 pixels), zero fill outside the image.
-bool wgrad_tensor_maps(const WgradArgs &a, CUtensorMap *tz, CUtensorMap *tx) {
+// Output channels of one tile: 128, 64, 96 (one tile for a 96-channel output, so its input is read
+// once) or 32.
+int conv_kn(int cout) {
+  return cout % 128 == 0 ? 128 : cout % 64 == 0 ? 64 : cout % 96 == 0 ? 96 : 32;
+}
+
+// Tensor maps of one weight gradient: dz [n][h][w][zcs] (cout channels; box 32 channels x 64
+// pixels) and x [n][h][w][cin] (box xc channels x 66 pixels), swizzled over the box's channels, zero
+// fill outside the image.
+bool wgrad_tensor_maps(const WgradArgs &a, int xc, CUtensorMap *tz, CUtensorMap *tx) {
   TmEncodeFn enc = tm_encode_fn();
   if (!enc) return false;
   const cuuint32_t e4[4] = {1, 1, 1, 1};
-  const cuuint64_t dZ[4] = {(cuuint64_t)a.cout, (cuuint64_t)a.w, (cuuint64_t)a.h, (cuuint64_t)a.n};
-  const cuuint64_t sZ[3] = {(cuuint64_t)a.zcs * 2, (cuuint64_t)a.w * a.zcs * 2,
-                            (cuuint64_t)a.h * a.w * a.zcs * 2};
-  const cuuint32_t bZ[4] = {8, (cuuint32_t)kWgP, 1, 1};
-  if (enc(tz, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)a.dz, dZ, sZ, bZ, e4,
-          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-          CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return false;
-  const cuuint64_t dX[4] = {(cuuint64_t)a.cin, (cuuint64_t)a.w, (cuuint64_t)a.h, (cuuint64_t)a.n};
-  const cuuint64_t sX[3] = {(cuuint64_t)a.cin * 2, (cuuint64_t)a.w * a.cin * 2,
-                            (cuuint64_t)a.h * a.w * a.cin * 2};
-  const cuuint32_t bX[4] = {8, (cuuint32_t)kWtHalo, 1, 1};
-  return enc(tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)a.x, dX, sX, bX, e4,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  auto map = [&](CUtensorMap *t, const bf16 *p, int c, int cs, int bc, int bp) {
+    const cuuint64_t d[4] = {(cuuint64_t)c, (cuuint64_t)a.w, (cuuint64_t)a.h, (cuuint64_t)a.n};
+    const cuuint64_t s[3] = {(cuuint64_t)cs * 2, (cuuint64_t)a.w * cs * 2, (cuuint64_t)a.h * a.w * cs * 2};
+    const cuuint32_t b[4] = {(cuuint32_t)bc, (cuuint32_t)bp, 1, 1};
+    return enc(t, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)p, d, s, b, e4,
+               CU_TENSOR_MAP_INTERLEAVE_NONE,
+               bc == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
+               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  return map(tz, a.dz, a.cout, a.zcs, 32, kWgP) && map(tx, a.x, a.cin, a.cin, xc, kWtHalo);
 }
 
-template <int kN, int kR, int kS>
-void launch_tma(dim3 grid, const ConvArgs &a, const CUtensorMap &ta, const CUtensorMap &tb,
-                ds2d_unet *u) {
-  k_conv3x3_tma<kN, kR, kS><<<grid, 128, tma_smem_bytes<kN, kR, kS>(), u->stream>>>(a, ta, tb,
-                                                                                    u->d_err);
-}
-
-template <int kN, int kR, int kS>
-cudaError_t tma_attr() {
-  return cudaFuncSetAttribute(k_conv3x3_tma<kN, kR, kS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              tma_smem_bytes<kN, kR, kS>());
+template <int kN, int kJ, int kCK>
+int launch_conv(ds2d_unet *u, const ConvArgs &a, const bf16 *wblk, int stages) {
+  CUtensorMap ta;
+  if (!conv_tensor_map(a, kCK, cv_pitch<kJ>(), &ta))
+    return unet_fail(u, DS2D_E_CUDA, "conv: cuTensorMapEncodeTiled failed");
+  stages = std::min(stages, a.cin / kCK);
+  while (stages > 1 && cv_smem_bytes<kN, kJ, kCK>(stages) > 226 * 1024) stages--;
+  const dim3 grid((a.w + 8 * kJ - 1) / (8 * kJ), (a.h + kTileH - 1) / kTileH, a.n * (a.cout / kN));
+  const int smem = cv_smem_bytes<kN, kJ, kCK>(stages);
+  UCK(cudaFuncSetAttribute(k_conv3x3_tma<kN, kJ, kCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k_conv3x3_tma<kN, kJ, kCK><<<grid, 128, smem, u->stream>>>(a, ta, wblk, stages, u->d_err);
+  UCK(cudaGetLastError());
+  return DS2D_OK;
 }
 
 int conv(ds2d_unet *u, const ds2d_unet::Layer &L, const bf16 *in, const bf16 *w, int cin, int cout,
@@ -1447,37 +1499,19 @@ int conv(ds2d_unet *u, const ds2d_unet::Layer &L, const bf16 *in, const bf16 *w,
          int n, int h, int wd) {
   ConvArgs a{in, w, bias, out, out_f32, mask, n, h, wd, cin, cout, ocs, oco, relu};
   if (u->use_tc && u->tc_tma && cout % 32 == 0 && cin % 16 == 0) {
-    // tcgen05, operands by tiled bulk-tensor loads through a ring; output tiles of 128, 64, 96
-    // (one tile for a 96-channel output, so its input is read once) or 32 channels
-    const int kn = cout % 128 == 0 ? 128 : cout % 64 == 0 ? 64 : cout % 96 == 0 ? 96 : 32;
+    // tcgen05, operands by bulk-tensor loads
+    const int kn = conv_kn(cout);
     const bf16 *wblk = w == L.wf ? L.wfb : (w == L.wb ? L.wbb : nullptr);
-    CUtensorMap ta, tb;
-    if (!wblk || !conv_tensor_maps(a, wblk, kn, &ta, &tb))
-      return unet_fail(u, DS2D_E_CUDA, "conv: cuTensorMapEncodeTiled failed");
-    // rows per CTA: 4 with option "tcgen05_rows" 4, else 2; ring stages: option "tcgen05_stages"
-    const int kr = u->tc_rows == 4 ? 4 : 2, ks = u->tc_stages;
-    dim3 grid((wd + kTcM - 1) / kTcM, (h + kr - 1) / kr, n * (cout / kn));
-    const int v = kn == 96 ? (ks == 2 ? 12 : 13)  // 96 channels: two rows per CTA (TMEM)
-                           : (kn == 128 ? 0 : kn == 64 ? 4 : 8) + (kr == 4 ? 2 : 0) + (ks == 2 ? 1 : 0);
-    if (kn == 96) grid.y = (h + 1) / 2;
-    switch (v) {
-      case 0: launch_tma<128, 2, 3>(grid, a, ta, tb, u); break;
-      case 1: launch_tma<128, 2, 2>(grid, a, ta, tb, u); break;
-      case 2: launch_tma<128, 4, 3>(grid, a, ta, tb, u); break;
-      case 3: launch_tma<128, 4, 2>(grid, a, ta, tb, u); break;
-      case 4: launch_tma<64, 2, 3>(grid, a, ta, tb, u); break;
-      case 5: launch_tma<64, 2, 2>(grid, a, ta, tb, u); break;
-      case 6: launch_tma<64, 4, 3>(grid, a, ta, tb, u); break;
-      case 7: launch_tma<64, 4, 2>(grid, a, ta, tb, u); break;
-      case 8: launch_tma<32, 2, 3>(grid, a, ta, tb, u); break;
-      case 9: launch_tma<32, 2, 2>(grid, a, ta, tb, u); break;
-      case 10: launch_tma<32, 4, 3>(grid, a, ta, tb, u); break;
-      case 11: launch_tma<32, 4, 2>(grid, a, ta, tb, u); break;
-      case 12: launch_tma<96, 2, 2>(grid, a, ta, tb, u); break;
-      default: launch_tma<96, 2, 3>(grid, a, ta, tb, u); break;
-    }
-    UCK(cudaGetLastError());
-    return DS2D_OK;
+    if (!wblk) return unet_fail(u, DS2D_E_STATE, "conv: no blocked weights");
+    // Tiles of 8 or 16 pixels x 16 rows and one or two stages: small CTAs, several per SM, whose
+    // loads, MMAs and epilogues interleave.  2008x608 forward / training gradients on 8 x 128x256, ms
+    // (0.94 / 1.33 as chosen): 128 channels 16 pixels 0.97 / 1.39, stages of 32 channels 1.01 /
+    // 1.31; 64 channels 32 pixels 1.01 / 1.37; 32 channels 32 pixels 0.98 / 1.36, two stages 0.97
+    // / 1.33; 96 channels 8 pixels 1.05 / 1.34.
+    if (kn == 128) return launch_conv<128, 1, 16>(u, a, wblk, 2);
+    if (kn == 96) return launch_conv<96, 2, 16>(u, a, wblk, 2);
+    if (kn == 64) return launch_conv<64, 1, 16>(u, a, wblk, 1);
+    return launch_conv<32, 2, 16>(u, a, wblk, 1);
   }
   if (u->use_tc && cout % 32 == 0) {
     const int kn = cout % 128 == 0 ? 128 : (cout % 64 == 0 ? 64 : 32);
@@ -1541,7 +1575,7 @@ int wgrad(ds2d_unet *u, const ds2d_unet::Layer &L, const bf16 *dz, int zcs, cons
     const int kn = L.cin_pad % 128 == 0 ? 128 : L.cin_pad % 64 == 0 ? 64
                  : L.cin_pad % 96 == 0 ? 96 : L.cin_pad % 32 == 0 ? 32 : 16;
     CUtensorMap tz, tx;
-    if (!wgrad_tensor_maps(a, &tz, &tx))
+    if (!wgrad_tensor_maps(a, kn < 32 ? kn : 32, &tz, &tx))
       return unet_fail(u, DS2D_E_CUDA, "wgrad: cuTensorMapEncodeTiled failed");
     const long long tchunks = (long long)n * h * ((wd + kWgP - 1) / kWgP);
     const long long ttiles = (long long)((L.cout + kWgM - 1) / kWgM) * (L.cin_pad / kn) * 3;
@@ -1564,9 +1598,6 @@ int wgrad(ds2d_unet *u, const ds2d_unet::Layer &L, const bf16 *dz, int zcs, cons
       k_conv3x3_wgrad_tma<32><<<tgrid, 128, wt_smem_bytes<32>(), u->stream>>>(a, tz, tx, u->d_err);
     else
       k_conv3x3_wgrad_tma<16><<<tgrid, 128, wt_smem_bytes<16>(), u->stream>>>(a, tz, tx, u->d_err);
-    const long long npx = (long long)n * h * wd;
-    const unsigned bb = nblk(npx * (L.cout / 8)) < 148u * 2 ? nblk(npx * (L.cout / 8)) : 148u * 2;
-    k_bias_grad<<<bb, 256, 0, u->stream>>>(dz, zcs, L.cout, npx, a.db);
     UCK(cudaGetLastError());
     return DS2D_OK;
   }
@@ -1598,12 +1629,13 @@ int wgrad(ds2d_unet *u, const ds2d_unet::Layer &L, const bf16 *dz, int zcs, cons
 
 int refresh_weights(ds2d_unet *u) {
   if (!u->weights_dirty) return DS2D_OK;
-  for (auto &L : u->layers) {
-    if (L.k != 3) continue;
-    const long long n = 9LL * L.cout * L.cin_pad;
-    k_weights_bf16<<<nblk(n), 256, 0, u->stream>>>(u->params + L.w_off, 9, L.cout, L.cin,
-                                                   L.cin_pad, L.wf, L.wb, L.wfb, L.wbb);
-  }
+  WeightArgs a{};
+  int k = 0;
+  for (auto &L : u->layers)
+    if (L.k == 3)  // the first layer has no backward-data convolution (its input is the image)
+      a.l[k++] = WeightLayer{u->params + L.w_off, L.wf, L.wb, L.wfb, L.cin % 32 == 0 ? L.wbb : nullptr,
+                             L.cout, L.cin, L.cin_pad, conv_kn(L.cout), conv_kn(L.cin)};
+  k_weights_bf16<<<dim3(592, k), 256, 0, u->stream>>>(a);
   UCK(cudaGetLastError());
   u->weights_dirty = false;
   return DS2D_OK;
@@ -1619,6 +1651,29 @@ int check_wait_flag(ds2d_unet *u) {
     return unet_fail(u, DS2D_E_CUDA, "tensor-core convolution: a bounded wait gave up");
   }
   return DS2D_OK;
+}
+
+// Device array into a pageable host array through two pinned chunks, one filling while the host
+// empties the other (a pageable copy of the gradients took 1.0 ms of a 4.2 ms training step, this
+// 0.8, most of it the page faults of a fresh array).
+constexpr size_t kStageChunk = 256 << 10;
+int to_host(ds2d_unet *u, void *dst, const void *src, size_t bytes) {
+  const size_t n = (bytes + kStageChunk - 1) / kStageChunk;
+  auto empty = [&](size_t i) {
+    UCK(cudaEventSynchronize(u->ev_stage[i & 1]));
+    std::memcpy((char *)dst + i * kStageChunk, u->h_stage + (i & 1) * kStageChunk,
+                std::min(kStageChunk, bytes - i * kStageChunk));
+    return (int)DS2D_OK;
+  };
+  int rc;
+  for (size_t i = 0; i < n; i++) {
+    UCK(cudaMemcpyAsync(u->h_stage + (i & 1) * kStageChunk, (const char *)src + i * kStageChunk,
+                        std::min(kStageChunk, bytes - i * kStageChunk), cudaMemcpyDeviceToHost,
+                        u->stream));
+    UCK(cudaEventRecord(u->ev_stage[i & 1], u->stream));
+    if (i > 0 && (rc = empty(i - 1))) return rc;
+  }
+  return n ? empty(n - 1) : (int)DS2D_OK;
 }
 
 int check_shape(ds2d_unet *u, int n, int h, int w) {
@@ -1645,12 +1700,14 @@ int forward(ds2d_unet *u, const float *x, int n, int h, int w) {
     if ((rc = conv(u, La, u->act[src].p, La.wf, cin, c[l], u->params + La.b_off, u->act[ea[l]].p,
                    c[l], 0, nullptr, nullptr, 1, n, hh, ww)))
       return rc;
-    if ((rc = conv(u, Lb, u->act[ea[l]].p, Lb.wf, c[l], c[l], u->params + Lb.b_off,
-                   u->act[eb[l]].p, c[l], 0, nullptr, nullptr, 1, n, hh, ww)))
+    // levels 1-3: the skip goes straight into its channels of the decoder's input
+    const auto &E = u->act[eb[l]];
+    if ((rc = conv(u, Lb, u->act[ea[l]].p, Lb.wf, c[l], c[l], u->params + Lb.b_off, E.p, E.c, 0,
+                   nullptr, nullptr, 1, n, hh, ww)))
       return rc;
     if (l < 3) {
       k_pool<<<row_grid((long long)n * (hh / 2), (ww / 2) * (c[l] / 8)), 256, 0, u->stream>>>(
-          u->act[eb[l]].p, u->act[pl[l]].p, n, hh, ww, c[l]);
+          E.p, E.c, u->act[pl[l]].p, n, hh, ww, c[l]);
       src = pl[l];
       hh /= 2;
       ww /= 2;
@@ -1664,8 +1721,8 @@ int forward(ds2d_unet *u, const float *x, int n, int h, int w) {
     hh *= 2;
     ww *= 2;
     const int cc = cprev + c[l];
-    k_up_concat<<<row_grid((long long)n * hh, ww * (cc / 8)), 256, 0, u->stream>>>(
-        u->act[prev].p, cprev, u->act[eb[l]].p, c[l], u->act[ca[l]].p, n, hh, ww);
+    k_up<<<row_grid((long long)n * (hh / 2), (ww / 2) * (cprev / 8)), 256, 0, u->stream>>>(
+        u->act[prev].p, cprev, u->act[ca[l]].p, cc, n, hh, ww);
     const int li = 8 + 2 * (2 - l);
     const auto &La = u->layers[li], &Lb = u->layers[li + 1];
     if ((rc = conv(u, La, u->act[ca[l]].p, La.wf, cc, c[l], u->params + La.b_off, u->act[da[l]].p,
@@ -1697,7 +1754,7 @@ int backward(ds2d_unet *u, int n, int h, int w) {
   UCK(cudaMemsetAsync(u->grads, 0, sizeof(float) * u->nparam, u->stream));
   const auto &Lo = u->layers.back();
   {
-    const unsigned ob = nblk(npx) < 148u * 8 ? nblk(npx) : 148u * 8;  // grid-stride over pixels
+    const unsigned ob = nblk(npx) < 148u * 3 ? nblk(npx) : 148u * 3;  // grid-stride over pixels
     if (c[0] == 32)
       k_out_bwd<32><<<ob, 256, 0, u->stream>>>(u->act[U::D1B].p, u->dy, u->params + Lo.w_off,
                                                u->grad[U::D1B].p, u->grads + Lo.w_off,
@@ -1742,7 +1799,7 @@ int backward(ds2d_unet *u, int n, int h, int w) {
       // skip gradient: pool path (from level l+1's input) + concat path (channels cprev..)
       const int cprev = l == 2 ? c[3] : c[l + 1];
       k_pool_grad<<<row_grid((long long)n * hh, ww * (c[l] / 8)), 256, 0, u->stream>>>(
-          u->grad[pl[l]].p, u->act[eb[l]].p, u->grad[ca[l]].p, cprev + c[l], cprev,
+          u->grad[pl[l]].p, u->act[eb[l]].p, u->act[eb[l]].c, u->grad[ca[l]].p, cprev + c[l], cprev,
           u->grad[eb[l]].p, n, hh, ww, c[l]);
     }
     const int src = l == 0 ? U::IN : pl[l - 1];
@@ -1767,6 +1824,17 @@ int backward(ds2d_unet *u, int n, int h, int w) {
       return rc;
     hh *= 2;
     ww *= 2;
+  }
+  if (u->use_tc && u->tc_wgrad && u->tc_wgrad_tma) {  // the other weight-gradient kernels add theirs
+    static const int slot[kConvLayers] = {U::E1A, U::E1B, U::E2A, U::E2B, U::E3A, U::E3B, U::E4A,
+                                          U::E4B, U::D3A, U::D3B, U::D2A, U::D2B, U::D1A, U::D1B};
+    static const int level[kConvLayers] = {0, 0, 1, 1, 2, 2, 3, 3, 2, 2, 1, 1, 0, 0};
+    BiasArgs b{};
+    for (int i = 0; i < kConvLayers; i++) {
+      const auto &L = u->layers[i];
+      b.l[i] = BiasLayer{u->grad[slot[i]].p, u->grads + L.b_off, npx >> (2 * level[i]), L.cout};
+    }
+    k_bias_grad<<<dim3(148, kConvLayers), 256, 0, u->stream>>>(b);
   }
   UCK(cudaGetLastError());
   return DS2D_OK;
@@ -1835,7 +1903,8 @@ int ds2d_unet_create(int base, int max_n, int max_h, int max_w, int device, ds2d
     const long long px = px0 >> (2 * lev);
     u->act[slot].c = ch;
     u->grad[slot].c = ch;
-    A((void **)&u->act[slot].p, sizeof(bf16) * px * ch);
+    if (slot != U::E1B && slot != U::E2B && slot != U::E3B)
+      A((void **)&u->act[slot].p, sizeof(bf16) * px * ch);
     A((void **)&u->grad[slot].p, sizeof(bf16) * px * ch);
   };
   act(U::IN, 0, 16);
@@ -1846,6 +1915,12 @@ int ds2d_unet_create(int base, int max_n, int max_h, int max_w, int device, ds2d
   act(U::C3, 2, c[3] + c[2]); act(U::D3A, 2, c[2]); act(U::D3B, 2, c[2]);
   act(U::C2, 1, c[2] + c[1]); act(U::D2A, 1, c[1]); act(U::D2B, 1, c[1]);
   act(U::C1, 0, c[1] + c[0]); act(U::D1A, 0, c[0]); act(U::D1B, 0, c[0]);
+  // the skips are the last channels of the decoder inputs (pixel stride = channels of both)
+  auto skip = [&](int slot, int cat, int cu) {
+    u->act[slot].p = u->act[cat].p ? u->act[cat].p + cu : nullptr;
+    u->act[slot].c = u->act[cat].c;
+  };
+  skip(U::E1B, U::C1, c[1]); skip(U::E2B, U::C2, c[2]); skip(U::E3B, U::C3, c[3]);
   A((void **)&u->y, sizeof(float) * px0);
   A((void **)&u->dy, sizeof(float) * px0);
   A((void **)&u->part, sizeof(double) * kRedBlocks);
@@ -1872,12 +1947,6 @@ int ds2d_unet_create(int base, int max_n, int max_h, int max_w, int device, ds2d
     if (ea == cudaSuccess)
       ea = cudaFuncSetAttribute(k_conv3x3_tc<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 tc_smem_bytes<64, 4>());
-    for (cudaError_t (*f)() : {tma_attr<128, 2, 3>, tma_attr<128, 2, 2>, tma_attr<128, 4, 3>,
-                              tma_attr<128, 4, 2>, tma_attr<64, 2, 3>, tma_attr<64, 2, 2>,
-                              tma_attr<64, 4, 3>, tma_attr<64, 4, 2>, tma_attr<32, 2, 3>,
-                              tma_attr<32, 2, 2>, tma_attr<32, 4, 3>, tma_attr<32, 4, 2>,
-                              tma_attr<96, 2, 2>, tma_attr<96, 2, 3>})
-      if (ea == cudaSuccess) ea = f();
     if (ea == cudaSuccess)
       ea = cudaFuncSetAttribute(k_conv3x3_tc<32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 tc_smem_bytes<32, 4>());
@@ -1905,8 +1974,13 @@ int ds2d_unet_create(int base, int max_n, int max_h, int max_w, int device, ds2d
     if (ea != cudaSuccess)
       rc = unet_fail(u, DS2D_E_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(ea));
   }
-  if (rc == DS2D_OK && cudaMallocHost((void **)&u->h_part, sizeof(double) * kRedBlocks) != cudaSuccess)
+  // one pinned block: the two staging chunks, then the loss partials
+  if (rc == DS2D_OK && cudaMallocHost((void **)&u->h_stage, 2 * kStageChunk + sizeof(double) * kRedBlocks) != cudaSuccess)
     rc = unet_fail(u, DS2D_E_NOMEM, "cudaMallocHost");
+  if (rc == DS2D_OK) u->h_part = reinterpret_cast<double *>(u->h_stage + 2 * kStageChunk);
+  for (cudaEvent_t &ev : u->ev_stage)
+    if (rc == DS2D_OK && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess)
+      rc = unet_fail(u, DS2D_E_CUDA, "cudaEventCreate");
   if (rc != DS2D_OK) {
     g_unet_err = u->err;
     ds2d_unet_destroy(u);
@@ -1921,7 +1995,9 @@ int ds2d_unet_destroy(ds2d_unet *u) {
   cudaSetDevice(u->device);
   if (u->stream) cudaStreamSynchronize(u->stream);
   for (void *p : u->allocs) cudaFree(p);
-  if (u->h_part) cudaFreeHost(u->h_part);
+  if (u->h_stage) cudaFreeHost(u->h_stage);
+  for (cudaEvent_t e : u->ev_stage)
+    if (e) cudaEventDestroy(e);
   delete u;
   return DS2D_OK;
 }
@@ -1951,9 +2027,7 @@ int ds2d_unet_set_params(ds2d_unet *u, const float *host, long long n) {
 int ds2d_unet_get_params(ds2d_unet *u, float *host, long long n) {
   if (!u || !host || n != u->nparam) return unet_fail(u, DS2D_E_ARG, "get_params: size mismatch");
   cudaSetDevice(u->device);
-  UCK(cudaMemcpyAsync(host, u->params, sizeof(float) * n, cudaMemcpyDeviceToHost, u->stream));
-  UCK(cudaStreamSynchronize(u->stream));
-  return DS2D_OK;
+  return to_host(u, host, u->params, sizeof(float) * n);
 }
 
 int ds2d_unet_forward(ds2d_unet *u, const float *x, float *y, int n, int h, int w) {
@@ -1987,7 +2061,6 @@ int ds2d_unet_set_option(ds2d_unet *u, const char *key, long long value) {
   if (std::string(key) == "tcgen05_stages") {
     if (value != 2 && value != 3)
       return unet_fail(u, DS2D_E_ARG, "tcgen05_stages must be 2 or 3");
-    u->tc_stages = (int)value;
     return DS2D_OK;
   }
   if (std::string(key) == "tcgen05_rows") {
@@ -2011,11 +2084,12 @@ int ds2d_unet_loss_grad(ds2d_unet *u, const float *x, const float *target, int n
   if ((rc = backward(u, n, h, w))) return rc;
   UCK(cudaMemcpyAsync(u->h_part, u->part, sizeof(double) * kRedBlocks, cudaMemcpyDeviceToHost,
                       u->stream));
-  if (grads_host)
-    UCK(cudaMemcpyAsync(grads_host, u->grads, sizeof(float) * u->nparam, cudaMemcpyDeviceToHost,
-                        u->stream));
-  UCK(cudaStreamSynchronize(u->stream));
-  if (u->use_tc && (rc = check_wait_flag(u))) return rc;
+  if (grads_host && (rc = to_host(u, grads_host, u->grads, sizeof(float) * u->nparam))) return rc;
+  if (u->use_tc) {  // waits for the stream
+    if ((rc = check_wait_flag(u))) return rc;
+  } else {
+    UCK(cudaStreamSynchronize(u->stream));
+  }
   if (loss) {
     double s = 0;
     for (int i = 0; i < kRedBlocks; i++) s += u->h_part[i];

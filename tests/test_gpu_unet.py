@@ -236,3 +236,35 @@ def test_unet_mn_major_weight_gradients_agree_with_mma_sync(cuda_device):
     for k, v in grads[0].items():
         if np.linalg.norm(v) > 0:
             assert rel(grads[1][k], v) < 1e-4, (k, rel(grads[1][k], v))
+
+
+# Widths and heights around the 8- and 16-pixel x 16-row tiles of the convolution and the 64-pixel
+# chunks of the weight gradient, at every level of the network (the deepest is 1/8 of the image).
+@pytest.mark.parametrize("base,n,h,w", [(32, 1, 8, 8), (32, 3, 136, 72), (32, 1, 8, 520),
+                                        (32, 2, 264, 16), (64, 2, 40, 136)])
+def test_unet_tiles_equal_staged(cuda_device, base, n, h, w):
+    """The bulk-tensor-fed convolution issues the thread-staged kernel's MMAs in the same order, so
+    the forward pass has the same bits; the weight gradients sum the same products split otherwise
+    (FP32, about 1e5 terms: 1e-5)."""
+    import torch
+    from ds2d_b200.unet import UNet, he_normal, unflatten
+    g = torch.Generator(device="cuda").manual_seed(h + w)
+    x = torch.randn((n, h, w), generator=g, device="cuda")
+    t = torch.randn((n, h, w), generator=g, device="cuda")
+    out = []
+    with UNet(base=base, max_n=n, max_h=h, max_w=w) as net:
+        net.set_params(he_normal(5, base))
+        for tma in (1, 0):
+            net.set_option("tcgen05_tma", tma)
+            net.set_option("tcgen05_wgrad_tma", tma)
+            y = torch.empty_like(x)
+            net.forward(x.data_ptr(), y.data_ptr(), n, h, w)
+            loss, grads = net.loss_grad(x.data_ptr(), t.data_ptr(), n, h, w, want_grads=True)
+            torch.cuda.synchronize()
+            out.append((y.cpu().numpy(), loss, unflatten(grads, base)))
+    (y0, l0, g0), (y1, l1, g1) = out
+    np.testing.assert_array_equal(y0, y1)
+    assert l0 == l1
+    for k in g0:
+        ref = np.linalg.norm(g1[k].astype(np.float64))
+        assert np.linalg.norm(g0[k].astype(np.float64) - g1[k]) <= 1e-5 * ref, k
