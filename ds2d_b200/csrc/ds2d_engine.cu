@@ -960,42 +960,66 @@ using FwdTileFn = void (*)(FwdTileArgs);
 using BwdTileFn = void (*)(BwdTileArgs);
 using AcTileFn = void (*)(AcFwdTileArgs);
 using AcRevTileFn = void (*)(AcRevTileArgs);
+// Shapes by rows per CTA: the elastic steps keep two stage-1 rows a thread (registers), the acoustic
+// ones 320 threads.
+using TileE8 = TileCfg<8, 8>;
+using TileE16 = TileCfg<16, 12>;
+using TileE32 = TileCfg<32, 20>;
+using TileA8 = TileCfg<8, 8>;
+using TileA16 = TileCfg<16, 8>;
+using TileA32 = TileCfg<32, 8>;
+template <class Fn>
+struct TileKernel {
+  Fn fn;
+  int threads;
+  size_t smem;
+};
+template <class C, bool kBorn>
+TileKernel<FwdTileFn> fwd_tile_c(bool pml) {
+  return {pml ? k_fwd_tile<true, C, kBorn> : k_fwd_tile<false, C, kBorn>, C::T, fwd_tile_smem<C>()};
+}
 template <bool kBorn>
-FwdTileFn fwd_tile_fn(bool pml, int tx) {
-  if (pml) return tx == 8 ? k_fwd_tile<true, 8, kBorn> : tx == 16 ? k_fwd_tile<true, 16, kBorn> : k_fwd_tile<true, 32, kBorn>;
-  return tx == 8 ? k_fwd_tile<false, 8, kBorn> : tx == 16 ? k_fwd_tile<false, 16, kBorn> : k_fwd_tile<false, 32, kBorn>;
+TileKernel<FwdTileFn> fwd_tile_k(bool pml, int tx) {
+  return tx == 8 ? fwd_tile_c<TileE8, kBorn>(pml) : tx == 16 ? fwd_tile_c<TileE16, kBorn>(pml) : fwd_tile_c<TileE32, kBorn>(pml);
+}
+template <class C, bool kScat>
+TileKernel<BwdTileFn> bwd_tile_c(bool pml) {
+  return {pml ? k_bwd_tile<true, C, kScat> : k_bwd_tile<false, C, kScat>, C::T,
+          kScat ? std::max(bwd_tile_smem<C>(), scat_tile_smem<C>()) : bwd_tile_smem<C>()};
 }
 template <bool kScat>
-BwdTileFn bwd_tile_fn(bool pml, int tx) {
-  if (pml) return tx == 8 ? k_bwd_tile<true, 8, kScat> : tx == 16 ? k_bwd_tile<true, 16, kScat> : k_bwd_tile<true, 32, kScat>;
-  return tx == 8 ? k_bwd_tile<false, 8, kScat> : tx == 16 ? k_bwd_tile<false, 16, kScat> : k_bwd_tile<false, 32, kScat>;
+TileKernel<BwdTileFn> bwd_tile_k(bool pml, int tx) {
+  return tx == 8 ? bwd_tile_c<TileE8, kScat>(pml) : tx == 16 ? bwd_tile_c<TileE16, kScat>(pml) : bwd_tile_c<TileE32, kScat>(pml);
 }
-AcTileFn ac_tile_fn(bool pml, int tx) {
-  if (pml) return tx == 8 ? k_ac_tile<true, 8> : tx == 16 ? k_ac_tile<true, 16> : k_ac_tile<true, 32>;
-  return tx == 8 ? k_ac_tile<false, 8> : tx == 16 ? k_ac_tile<false, 16> : k_ac_tile<false, 32>;
+template <class C>
+TileKernel<AcTileFn> ac_tile_c(bool pml) {
+  return {pml ? k_ac_tile<true, C> : k_ac_tile<false, C>, C::T, ac_tile_smem<C>()};
 }
-AcRevTileFn ac_rev_tile_fn(bool pml, int tx) {
-  if (pml) return tx == 8 ? k_ac_rev_tile<true, 8> : tx == 16 ? k_ac_rev_tile<true, 16> : k_ac_rev_tile<true, 32>;
-  return tx == 8 ? k_ac_rev_tile<false, 8> : tx == 16 ? k_ac_rev_tile<false, 16> : k_ac_rev_tile<false, 32>;
+TileKernel<AcTileFn> ac_tile_k(bool pml, int tx) {
+  return tx == 8 ? ac_tile_c<TileA8>(pml) : tx == 16 ? ac_tile_c<TileA16>(pml) : ac_tile_c<TileA32>(pml);
 }
-size_t bwd_tile_bytes(int tx, bool scat) {
-  return scat ? std::max(bwd_tile_smem(tx), scat_tile_smem(tx)) : bwd_tile_smem(tx);
+template <class C>
+TileKernel<AcRevTileFn> ac_rev_tile_c(bool pml) {
+  return {pml ? k_ac_rev_tile<true, C> : k_ac_rev_tile<false, C>, C::T, ac_rev_tile_smem<C>()};
+}
+TileKernel<AcRevTileFn> ac_rev_tile_k(bool pml, int tx) {
+  return tx == 8 ? ac_rev_tile_c<TileA8>(pml) : tx == 16 ? ac_rev_tile_c<TileA16>(pml) : ac_rev_tile_c<TileA32>(pml);
 }
 
 cudaError_t tile_attributes() {
   cudaError_t e = cudaSuccess;
-  auto set = [&](auto fn, size_t bytes) {
+  auto set = [&](auto k) {
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
   };
   for (bool pml : {false, true})
     for (int tx : kTileRows) {
-      set(fwd_tile_fn<false>(pml, tx), fwd_tile_smem(tx));
-      set(fwd_tile_fn<true>(pml, tx), fwd_tile_smem(tx));
-      set(bwd_tile_fn<false>(pml, tx), bwd_tile_bytes(tx, false));
-      set(bwd_tile_fn<true>(pml, tx), bwd_tile_bytes(tx, true));
-      set(ac_tile_fn(pml, tx), ac_tile_smem(tx));
-      set(ac_rev_tile_fn(pml, tx), ac_rev_tile_smem(tx));
+      set(fwd_tile_k<false>(pml, tx));
+      set(fwd_tile_k<true>(pml, tx));
+      set(bwd_tile_k<false>(pml, tx));
+      set(bwd_tile_k<true>(pml, tx));
+      set(ac_tile_k(pml, tx));
+      set(ac_rev_tile_k(pml, tx));
     }
   return e;
 }
@@ -1006,34 +1030,39 @@ bool tile_ok(const ds2d_ctx *c) {
 // Where a context's steps run on the tile kernels.  The rule looks at the context's batch (padded
 // cells of all its slots), so every batch of a context, a last short one too, takes the same
 // kernels.  Measured on a B200 at 0.05-22 M cells, ms per call, tile against marching kernels:
-//  - PML: elastic 16 x 1201x401 (8.9 M) RTM 41.5 / 43.1, forward 13.1 / 13.3, ELSRTM 138 / 141,
-//    and 6-50x on small batches; acoustic L^T L 0.66 M 5.5 / 6.9, 21.9 M 42.8 / 55.4 (half
+//  - PML: elastic 16 x 1201x401 (8.9 M) RTM 34.0 / 43.1, forward 12.2 / 13.4, ELSRTM 113 / 141,
+//    and 6-50x on small batches; acoustic L^T L 0.66 M 5.7 / 6.9, 21.9 M 37.1 / 56.3 (half
 //    steps).  The marching kernels pay the PML's predicates row by row: always the tiles.
-//  - random boundary, elastic: 0.66 M 3.6 / 8.1, 1.97 M 9.6 / 10.6, 2.22 M 8.0 / 7.8, 8.9 M
-//    28.3 / 17.5: the bulk-copy marching kernels win once they fill the chip, at 2 M cells.
-//  - random boundary, acoustic: 0.66 M 3.0 / 14.2, 2.63 M 10.9 / 16.3, 21.9 M 27.9 / 21.2: 6 M.
-constexpr double kTileElastic = 2e6, kTileAcoustic = 6e6;
+//  - random boundary, elastic: 0.66 M 3.2 / 8.1, 2.22 M 7.2 / 7.9, 8.9 M 24.6 / 17.5: the
+//    bulk-copy marching kernels win once they fill the chip, between 2.2 and 8.9 M cells.
+//  - random boundary, acoustic: 0.66 M 2.9 / 14.2, 2.63 M 10.6 / 16.3, 21.9 M 25.8 / 21.3: 6 M.
+constexpr double kTileElastic = 3e6, kTileAcoustic = 6e6;
 bool tile_on(const ds2d_ctx *c, bool acoustic) {
   if (!tile_ok(c) || c->opt_tile == 0) return false;
   if (c->opt_tile > 0) return true;
   if (c->shape_set) return false;
   return !c->d.rbc || (double)c->B * c->d.slot <= (acoustic ? kTileAcoustic : kTileElastic);
 }
-// Rows per CTA: the elastic steps are best at 8 (registers: 3 CTAs an SM); the acoustic ones, with a
-// third of the operands, at 16, and at 32 (least redundant work) once the tiles fill the chip
-// (0.09 M cells 14.8 / 12.9 / 14.3 ms at 8 / 16 / 32, 2.6 M 15.3 / 11.6 / 10.9).
+// Rows per CTA.  Fewer rows are more CTAs, for batches that do not fill the chip (0.05 M cells
+// forward 9.6 / 11.8 / 11.3 ms at 8 / 16 / 32 rows); more rows are less redundant work: ELSRTM of
+// 0.19 M cells 29.7 / 27.0 / 25.0, of 8.9 M 125 / 115 / 113, RTM with the random boundary (whose
+// steps have no strip or PML operands) 0.66 M 3.54 / 3.18 / 3.31.  Acoustic: 0.09 M 11.3 / 11.2
+// / 14.4, 2.6 M 16.2 / 13.4 / 10.6.
 int tile_rows(const ds2d_ctx *c, bool acoustic) {
   if (c->opt_tile > 0) return c->opt_tile;
-  return !acoustic ? 8 : (double)c->B * c->d.slot < 1e6 ? 16 : 32;
+  const double cells = (double)c->B * c->d.slot;
+  if (acoustic) return cells < 0.5e6 ? 16 : 32;
+  return cells < 0.12e6 ? 8 : c->d.rbc ? 16 : 32;
 }
 dim3 tile_grid(const ds2d_ctx *c, int tx, int slices) {
-  return dim3((c->d.nzp + kTileZ - 1) / kTileZ, (c->d.nxp + tx - 1) / tx, slices);
+  const int upd = 2 * c->d.nop;  // tiles cover the updated cells
+  return dim3((c->d.nzp - upd + kTileZ - 1) / kTileZ, (c->d.nxp - upd + tx - 1) / tx, slices);
 }
 // Launches a tile kernel; `chain`: behind another tile kernel of the same pass, so its loads of
 // what no step writes may overlap that one (programmatic dependent launch).
 template <class A>
-void launch_tile(ds2d_ctx *c, const char *name, double bytes, void (*fn)(A), dim3 grid, size_t smem,
-                 const A &a, bool chain) {
+void launch_tile(ds2d_ctx *c, const char *name, double bytes, const TileKernel<void (*)(A)> &k,
+                 dim3 grid, const A &a, bool chain) {
   int ev = -1;
   if (c->prof.on) {
     ev = c->prof.take();
@@ -1041,15 +1070,15 @@ void launch_tile(ds2d_ctx *c, const char *name, double bytes, void (*fn)(A), dim
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(kTileT);
-  cfg.dynamicSmemBytes = smem;
+  cfg.blockDim = dim3(k.threads);
+  cfg.dynamicSmemBytes = k.smem;
   cfg.stream = c->stream;
   cudaLaunchAttribute at{};
   at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = chain && ev < 0 ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, fn, a);
+  cudaLaunchKernelEx(&cfg, k.fn, a);
   c->last_launches++;
   if (ev >= 0) {
     cudaEventRecord(c->prof.pool[ev + 1], c->stream);
@@ -1072,8 +1101,8 @@ int run_forward_tile(ds2d_ctx *c, int n, bool record, bool strips) {
     a.it = it; a.rmap = c->d_rmap;
     if (record) { a.rec_on = 1; a.rec_vz = c->rec[0]; a.rec_vx = c->rec[1]; }
     if (strips) t.st[0] = StripSaveArgs{d, c->d_shots, cur->vx, cur->vz, c->st_a, it - 1};
-    launch_tile(c, "fwd_tile", kBytesFused * CELLS(n), fwd_tile_fn<false>(!d.rbc, tx),
-                tile_grid(c, tx, n * (1 + nst)), fwd_tile_smem(tx), t, it > 0);
+    launch_tile(c, "fwd_tile", kBytesFused * CELLS(n), fwd_tile_k<false>(!d.rbc, tx),
+                tile_grid(c, tx, n * (1 + nst)), t, it > 0);
     std::swap(cur, nxt);
   }
   if (strips) strip_save(c, *cur, c->st_a, d.nt - 1, n);
@@ -1314,8 +1343,8 @@ int rtm_batch_body(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base) {
         BwdTileArgs t{};
         t.b = a;
         t.n = n;
-        launch_tile(c, "bwd_tile", kBytesBwdFused * CELLS(n), bwd_tile_fn<false>(!d.rbc, tx),
-                    tile_grid(c, tx, n), bwd_tile_bytes(tx, false), t, it < d.nt - 1);
+        launch_tile(c, "bwd_tile", kBytesBwdFused * CELLS(n), bwd_tile_k<false>(!d.rbc, tx),
+                    tile_grid(c, tx, n), t, it < d.nt - 1);
       } else if (pair_bwd_on(c) && c->opt_pair_split) {
         int pns, ptz;
         pair_split(d, kPairSplitT, &pns, &ptz);
@@ -1471,8 +1500,7 @@ int elsrtm_forward_fused(ds2d_ctx *c, int n, bool strips) {
       }
       launch_tile(c, "fwd_born_tile",
                   (kBytesBornMode[1] + kBytesBornMode[2] + kBytesBornMode[3]) * CELLS(n),
-                  fwd_tile_fn<true>(!d.rbc, tx), tile_grid(c, tx, n * (3 + nst)),
-                  fwd_tile_smem(tx), t, l > 0);
+                  fwd_tile_k<true>(!d.rbc, tx), tile_grid(c, tx, n * (3 + nst)), t, l > 0);
     }
     cur = d.nt & 1;
   }
@@ -1556,8 +1584,7 @@ int elsrtm_backward_fused(ds2d_ctx *c, int n, bool strips) {
       t.fvx = fc->vx;
       t.fvz = fc->vz;
       launch_tile(c, "bwd_scat_tile", (kBytesBwdFused + kBytesBwdScat) * CELLS(n),
-                  bwd_tile_fn<true>(!d.rbc, tx), tile_grid(c, tx, 2 * n), bwd_tile_bytes(tx, true),
-                  t, it < d.nt - 1);
+                  bwd_tile_k<true>(!d.rbc, tx), tile_grid(c, tx, 2 * n), t, it < d.nt - 1);
       std::swap(fc, fn);
       std::swap(ac, an);
       if (b.it >= 0) std::swap(bc, bn);
@@ -1856,8 +1883,7 @@ int ac_L_tile(ds2d_ctx *c, int n) {
     t.set[1].e_in = e[(l - 1) & 1];
     t.set[1].rec_vz = c->rec[0];
     t.set[1].rec_vx = c->rec[1];
-    launch_tile(c, "ac_tile", 0, ac_tile_fn(!d.rbc, tx), tile_grid(c, tx, 2 * n), ac_tile_smem(tx),
-                t, l > 0);
+    launch_tile(c, "ac_tile", 0, ac_tile_k(!d.rbc, tx), tile_grid(c, tx, 2 * n), t, l > 0);
   }
   CK(cudaGetLastError());
   return DS2D_OK;
@@ -2045,8 +2071,7 @@ int ac_LT_tile(ds2d_ctx *c, int n) {
     t.nset = 1;
     t.set[0] = ac_tile_args(c, 0, it & 1, it);
     t.st = StripSaveArgs{d, c->d_shots, t.set[0].vx, t.set[0].vz, c->st_a, it - 1};
-    launch_tile(c, "ac_tile", 0, ac_tile_fn(!d.rbc, tx), tile_grid(c, tx, n * (1 + nst)),
-                ac_tile_smem(tx), t, it > 0);
+    launch_tile(c, "ac_tile", 0, ac_tile_k(!d.rbc, tx), tile_grid(c, tx, n * (1 + nst)), t, it > 0);
   }
   float *bk[2][3], *yk[2][5];
   for (int i = 0; i < 3; i++) {
@@ -2080,8 +2105,8 @@ int ac_LT_tile(ds2d_ctx *c, int n) {
     a.b = c->par.b; a.lam = c->par.lam; a.dampx = c->par.dampx; a.dampz = c->par.dampz;
     a.wavelet = c->wavelet; a.grad = c->img_slot; a.it = it; a.rmap = c->d_rmap;
     a.res_vz = c->rec[0]; a.res_vx = c->rec[1]; a.st = c->st_a;
-    launch_tile(c, "ac_rev_tile", kBytesAcRev * CELLS(n), ac_rev_tile_fn(!d.rbc, tx),
-                tile_grid(c, tx, n), ac_rev_tile_smem(tx), a, it < d.nt - 1);
+    launch_tile(c, "ac_rev_tile", kBytesAcRev * CELLS(n), ac_rev_tile_k(!d.rbc, tx),
+                tile_grid(c, tx, n), a, it < d.nt - 1);
   }
   CK(cudaGetLastError());
   return reduce_images(c, n, 1);

@@ -15,9 +15,10 @@
 // (TX + 8) x 40 cells for TX x 32) is paid from idle SMs; the state of such batches stays in L2.
 // State ping-pongs between two buffers as in the marching kernels.
 //
-// Measured (B200, whole calls, tile 8 against the marching kernels): forward of one 251x101 shot +
-// 20 PML, 2000 steps: 391 -> 8.2 ms (4.1 us a step); RTM of 2 64x32 shots, 200 steps: 22 -> 1.3 ms;
-// ELSRTM of 4 251x101 shots, 500 steps: 529 -> 30 ms; CG-LSRTM of 8 96x48 shots: 245 -> 13 ms.
+// Measured (B200, whole calls, against the marching kernels): forward of one 251x101 shot + 20 PML,
+// 2000 steps: 391 -> 9.6 ms; RTM of 2 64x32 shots, 200 steps: 22 -> 1.3 ms; ELSRTM of 4 251x101
+// shots, 500 steps: 529 -> 25 ms; CG-LSRTM of 8 96x48 shots: 245 -> 11 ms.  What bounds a full grid
+// is instruction issue (0.65 a cycle and scheduler), not bytes.
 //
 // Launches of consecutive steps use programmatic dependent launch: a CTA fetches everything that
 // no step writes (moduli, damping, image weights, trace indexes, residuals) before
@@ -30,17 +31,25 @@
 namespace ds2d {
 
 constexpr int kTileZ = 32;              // output columns of a tile
-constexpr int kTileT = 320;             // threads: 8 row groups x 40 stage-1 columns
 constexpr int kTileC1 = kTileZ + 8;     // stage-1 columns (tile + 4 on each side)
 constexpr int kTileC0 = kTileZ + 16;    // input columns (tile + 8)
-// Shared row pitch of the inputs: a multiple of 4 floats (16-byte copies) that puts the row groups
-// of neighbouring lanes 8 banks apart.
-__host__ __device__ constexpr int tile_p0(int tx) { return tx == 16 ? 56 : 52; }
-__host__ __device__ constexpr int tile_n0(int tx) { return (tx + 16) * tile_p0(tx); }
-__host__ __device__ constexpr int tile_n1(int tx) { return (tx + 8) * kTileC1; }
-__host__ __device__ constexpr size_t tile_smem(int tx, int inputs, int mids) {
-  return sizeof(float) * ((size_t)inputs * tile_n0(tx) + (size_t)mids * tile_n1(tx));
-}
+// Shape of a tile step: TX output rows, kG stage-1 row groups of R1 rows (40 kG threads), kG2 stage-2
+// row groups of R2 rows (one warp each).
+template <int kTX, int kG>
+struct TileCfg {
+  static constexpr int TX = kTX, G = kG, T = kTileC1 * kG, R1 = (kTX + 8) / kG;
+  static_assert(R1 * kG == kTX + 8, "row groups cover the tile plus 8 rows");
+  static constexpr int G2 = kTX <= T / 32 ? kTX : kTX / 2 <= T / 32 ? kTX / 2 : kTX / 4;
+  static constexpr int R2 = kTX / G2;
+  // Shared row pitch of the inputs: a multiple of 4 floats (16-byte copies) that puts the row
+  // groups of neighbouring lanes 8 banks apart.
+  static constexpr int P0 = R1 == 3 ? 56 : 52;
+  static constexpr int N0 = (kTX + 16) * P0, N1 = (kTX + 8) * kTileC1;
+  static constexpr int kLd = ((kTX + 16) * (kTileC0 / 4) + T - 1) / T;  // 16-byte copies per thread
+  static constexpr size_t smem(int inputs, int mids) {
+    return sizeof(float) * ((size_t)inputs * N0 + (size_t)mids * N1);
+  }
+};
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() {
@@ -53,17 +62,38 @@ __device__ __forceinline__ void cp_async16z(float *smem, const float *gmem, bool
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n) : "memory");
 }
 
+// A product that is rounded before it is added: the update's two increments and the split parts are
+// summed as rounded values, in every variant of a step and as in the PML ring kernels, so that a
+// cell's bits do not depend on which class its tile belongs to (nor 16-bit strips on the path).
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+
+// Tiles cover the updated cells [nop, n - nop) only.
+template <int TX>
+__device__ __forceinline__ int tile_x0() { return 4 + blockIdx.y * TX; }
+__device__ __forceinline__ int tile_z0() { return 4 + blockIdx.x * kTileZ; }
+
+// Class of a tile, a template parameter of the step functions so that the larger part of a grid runs
+// without a test per cell: kTileInner = its whole input window lies in the interior, at least nop
+// cells from the PML or random band (every cell is updated and imaged, none is a PML or strip
+// cell); kTilePml = a PML context's other tiles; kTileEdge = a random-boundary context's.
+constexpr int kTileEdge = 0, kTilePml = 1, kTileInner = 2;
+template <int TX>
+__device__ __forceinline__ bool tile_inner(const Dims &d, const ShotDev &sh) {
+  const int e = d.pml + d.nop, x0 = tile_x0<TX>(), z0 = tile_z0();
+  return x0 - 8 >= e && x0 + TX + 8 <= sh.nxp - e && z0 - 8 >= e && z0 + kTileZ + 8 <= d.nzp - e;
+}
+
 // Copies one field's input window (tile + 8) of the slot at `base` into dst.  Windows start on
 // 16-byte boundaries (tile columns are multiples of 32, rows `ld` multiples of 32); rows and
 // columns outside the padded grid are zeros.
-template <int TX>
+template <class C, bool kIn = false>
 __device__ __forceinline__ void tile_load(float *dst, const float *src, const Dims &d, int base,
                                           int x0, int z0) {
-  for (int i = threadIdx.x; i < (TX + 16) * (kTileC0 / 4); i += kTileT) {
+  for (int i = threadIdx.x; i < (C::TX + 16) * (kTileC0 / 4); i += C::T) {
     const int r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
     const int x = x0 - 8 + r, z = z0 - 8 + c;
-    const bool in = x >= 0 && x < d.nxp && z >= 0 && z < d.ld;
-    cp_async16z(dst + r * tile_p0(TX) + c, src + (in ? base + x * d.ld + z : 0), in);
+    const bool in = kIn || (x >= 0 && x < d.nxp && z >= 0 && z < d.ld);
+    cp_async16z(dst + r * C::P0 + c, src + (in ? base + x * d.ld + z : 0), in);
   }
 }
 
@@ -120,20 +150,22 @@ __device__ __forceinline__ TileDamp tile_damp(float dampx, float dampz, float dt
 
 // ---- forward step (modes of k_fwd_ring: 0 plain, 1 + Born source out, 2 overlay in and Born source
 // out, 3 overlay in) ------------------------------------------------------------------------------
-__host__ __device__ constexpr size_t fwd_tile_smem(int tx) { return tile_smem(tx, 3, 2); }
+template <class C>
+constexpr size_t fwd_tile_smem() { return C::smem(3, 2); }
 
-template <bool kPML, int TX, int kMode>
+template <int kCls, class C, int kMode>
 __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm) {
+  constexpr bool kPML = kCls == kTilePml, kIn = kCls == kTileInner;
   constexpr bool kOvIn = kMode >= 2, kBornOut = kMode == 1 || kMode == 2, kSrc = kMode < 2;
-  constexpr int R1 = (TX + 8) / 8, R2 = TX / 8, P0 = tile_p0(TX), N0 = tile_n0(TX);
-  constexpr int kLd = ((TX + 16) * (kTileC0 / 4) + kTileT - 1) / kTileT;  // copies per thread
+  constexpr int TX = C::TX, R1 = C::R1, R2 = C::R2, P0 = C::P0, N0 = C::N0;
+  constexpr int kLd = C::kLd;
   float *const i_xx = sm, *const i_zz = sm + N0, *const i_xz = sm + 2 * N0;
-  float *const v_x = sm + 3 * N0, *const v_z = v_x + tile_n1(TX);
+  float *const v_x = sm + 3 * N0, *const v_z = v_x + C::N1;
   const int tid = threadIdx.x;
   const ShotDev sh = a.shots[s];
   const Dims d = slot_dims(a.d, sh);
-  const int x0 = blockIdx.y * TX, z0 = blockIdx.x * kTileZ;
-  if (x0 >= d.nxp) return;  // beyond this slot's window, whole CTA
+  const int x0 = tile_x0<TX>(), z0 = tile_z0();
+  if (x0 >= d.nxp - d.nop) return;  // beyond this slot's window, whole CTA
   const int base = (int)(d.slot * s), ld = d.ld;
   const float dtdx = d.dt / d.dx, dtdz = d.dt / d.dz;
   const bool tp = kPML && tile_has_pml<TX>(d, x0, z0, 4);
@@ -141,11 +173,11 @@ __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm
   const int g1 = tid / kTileC1, c1 = tid - g1 * kTileC1, z1 = z0 - 4 + c1, xs1 = x0 - 4 + g1 * R1;
   const int g2 = tid >> 5, c2 = tid & 31, z2 = z0 + c2, xs2 = x0 + g2 * R2;
   const bool zu1 = z1 >= d.nop && z1 < d.nzp - d.nop;
-  const bool zu2 = tid < 256 && z2 >= d.nop && z2 < d.nzp - d.nop;
-  const bool zi2 = z2 >= d.pml && z2 < d.nzp - d.pml;
+  const bool zu2 = tid < 32 * C::G2 && (kIn || (z2 >= d.nop && z2 < d.nzp - d.nop));
+  const bool zi2 = kIn || (z2 >= d.pml && z2 < d.nzp - d.pml);
   const int k1 = base + xs1 * ld + z1, k2 = base + xs2 * ld + z2;
-  auto up1 = [&](int r) { return zu1 && xs1 + r >= d.nop && xs1 + r < d.nxp - d.nop; };
-  auto up2 = [&](int r) { return zu2 && xs2 + r >= d.nop && xs2 + r < d.nxp - d.nop; };
+  auto up1 = [&](int r) { return kIn || (zu1 && xs1 + r >= d.nop && xs1 + r < d.nxp - d.nop); };
+  auto up2 = [&](int r) { return zu2 && (kIn || (xs2 + r >= d.nop && xs2 + r < d.nxp - d.nop)); };
   auto pm1 = [&](int r) { return tp && pml_cell(d, xs1 + r, z1); };
   auto pm2 = [&](int r) { return tp && pml_cell(d, xs2 + r, z2); };
   auto own1 = [&](int r) {
@@ -176,7 +208,7 @@ __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm
       q2x[r] = __ldg(a.p.dampx + k2 + r * ld);
       q2z[r] = __ldg(a.p.dampz + k2 + r * ld);
     }
-    if (kBornOut && up2(r) && zi2 && xs2 + r >= d.pml && xs2 + r < d.nxp - d.pml) {
+    if (kBornOut && up2(r) && zi2 && (kIn || (xs2 + r >= d.pml && xs2 + r < d.nxp - d.pml))) {
       mp_[r] = __ldg(a.p.dmp + k2 + r * ld);
       ms_[r] = __ldg(a.p.dms + k2 + r * ld);
     }
@@ -184,17 +216,17 @@ __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm
   const float sval = kSrc ? __ldg(a.wavelet + a.it) : 0.f;
   pdl_wait();
   // ---- state -------------------------------------------------------------------------------------
-  tile_load<TX>(i_xx, a.a.txx, d, base, x0, z0);
-  tile_load<TX>(i_zz, a.a.tzz, d, base, x0, z0);
-  tile_load<TX>(i_xz, a.a.txz, d, base, x0, z0);
+  tile_load<C, kIn>(i_xx, a.a.txx, d, base, x0, z0);
+  tile_load<C, kIn>(i_zz, a.a.tzz, d, base, x0, z0);
+  tile_load<C, kIn>(i_xz, a.a.txz, d, base, x0, z0);
   cp_async_commit();
   float4 ov[kOvIn ? kLd : 1][3];
   if (kOvIn) {
 #pragma unroll
     for (int j = 0; j < kLd; j++) {
-      const int i = tid + j * kTileT, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
+      const int i = tid + j * C::T, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
       const int x = x0 - 8 + r, z = z0 - 8 + c;
-      const bool in = r < TX + 16 && x >= 0 && x < d.nxp && z >= 0 && z < ld;
+      const bool in = r < TX + 16 && (kIn || (x >= 0 && x < d.nxp && z >= 0 && z < ld));
       const int k = in ? base + x * ld + z : 0;
       const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
       ov[j][0] = in ? *reinterpret_cast<const float4 *>(a.ovi_txx + k) : zero;
@@ -233,7 +265,7 @@ __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm
   if (kOvIn) {  // Born source of the previous set: a thread adds it to the chunks it copied
 #pragma unroll
     for (int j = 0; j < kLd; j++) {
-      const int i = tid + j * kTileT, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
+      const int i = tid + j * C::T, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
       if (r >= TX + 16) continue;
 #pragma unroll
       for (int f = 0; f < 3; f++) {
@@ -247,7 +279,7 @@ __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm
   if (kSrc) {  // explosive source (transient): the thread that copied the cell adds it
     const int r = sh.isx - (x0 - 8), c = sh.isz - (z0 - 8);
     if (r >= 0 && r < TX + 16 && c >= 0 && c < kTileC0 &&
-        tid == (r * (kTileC0 / 4) + c / 4) % kTileT) {
+        tid == (r * (kTileC0 / 4) + c / 4) % C::T) {
       i_xx[r * P0 + c] += sval;
       i_zz[r * P0 + c] += sval;
     }
@@ -268,14 +300,14 @@ __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm
         const float ez = tile_dzp(i_zz + o + r * P0);
         const float bb = b_[r];
         const float cbx = bb * dtdx, cbz = bb * dtdz;
-        const float ux_x = cbx * ax[r], ux_z = cbz * bz, uz_x = cbx * fx[r], uz_z = cbz * ez;
+        const float ux_x = mul(cbx, ax[r]), ux_z = mul(cbz, bz), uz_x = mul(cbx, fx[r]), uz_z = mul(cbz, ez);
         const bool own = own1(r);
         if (kPML && pm1(r)) {
           const TileDamp q = tile_damp(q1x[r], q1z[r], d.dt);
-          const float vxx = fmaf(q.d1, s1[r][0], ux_x) * q.i2;
-          const float vxz = fmaf(q.d3, s1[r][1], ux_z) * q.i4;
-          const float vzx = fmaf(q.d1, s1[r][2], uz_x) * q.i2;
-          const float vzz = fmaf(q.d3, s1[r][3], uz_z) * q.i4;
+          const float vxx = mul(fmaf(q.d1, s1[r][0], ux_x), q.i2);
+          const float vxz = mul(fmaf(q.d3, s1[r][1], ux_z), q.i4);
+          const float vzx = mul(fmaf(q.d1, s1[r][2], uz_x), q.i2);
+          const float vzz = mul(fmaf(q.d3, s1[r][3], uz_z), q.i4);
           if (own) {
             a.b.vx_x[k] = vxx; a.b.vx_z[k] = vxz; a.b.vz_x[k] = vzx; a.b.vz_z[k] = vzz;
           }
@@ -314,17 +346,17 @@ __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm
       const float se = tile_dzp(v_x + o + r * kTileC1);
       const float lam = lam_[r], mu = mu_[r];
       const float l2m = lam + 2.0f * mu;
-      const float xx_x = l2m * dtdx * sa[r], xx_z = lam * dtdz * sb;
-      const float zz_x = lam * dtdx * sa[r], zz_z = l2m * dtdz * sb;
-      const float xz_x = dtdx * mu * sf[r], xz_z = dtdz * mu * se;
+      const float xx_x = mul(l2m * dtdx, sa[r]), xx_z = mul(lam * dtdz, sb);
+      const float zz_x = mul(lam * dtdx, sa[r]), zz_z = mul(l2m * dtdz, sb);
+      const float xz_x = mul(dtdx * mu, sf[r]), xz_z = mul(dtdz * mu, se);
       if (kPML && pm2(r)) {
         const TileDamp q = tile_damp(q2x[r], q2z[r], d.dt);
-        const float a1 = fmaf(q.d1, s2[r][0], xx_x) * q.i2;
-        const float a2 = fmaf(q.d3, s2[r][1], xx_z) * q.i4;
-        const float b1 = fmaf(q.d1, s2[r][2], zz_x) * q.i2;
-        const float b2 = fmaf(q.d3, s2[r][3], zz_z) * q.i4;
-        const float e1 = fmaf(q.d1, s2[r][4], xz_x) * q.i2;
-        const float e2 = fmaf(q.d3, s2[r][5], xz_z) * q.i4;
+        const float a1 = mul(fmaf(q.d1, s2[r][0], xx_x), q.i2);
+        const float a2 = mul(fmaf(q.d3, s2[r][1], xx_z), q.i4);
+        const float b1 = mul(fmaf(q.d1, s2[r][2], zz_x), q.i2);
+        const float b2 = mul(fmaf(q.d3, s2[r][3], zz_z), q.i4);
+        const float e1 = mul(fmaf(q.d1, s2[r][4], xz_x), q.i2);
+        const float e2 = mul(fmaf(q.d3, s2[r][5], xz_z), q.i4);
         a.b.txx_x[k] = a1; a.b.txx_z[k] = a2;
         a.b.tzz_x[k] = b1; a.b.tzz_z[k] = b2;
         a.b.txz_x[k] = e1; a.b.txz_z[k] = e2;
@@ -342,7 +374,7 @@ __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm
         a.b.tzz[k] = ozz + (zz_x + zz_z);
         a.b.txz[k] = oxz + (xz_x + xz_z);
       }
-      if (kBornOut && rs >= d.pml && rs < d.nxp - d.pml && zi2) {
+      if (kBornOut && zi2 && (kIn || (rs >= d.pml && rs < d.nxp - d.pml))) {
         const BornSrc e = born_source(lam, mu, mp_[r], ms_[r], sa[r], sb, se, sf[r], 1.0f / d.dx, 1.0f / d.dz);
         a.ovo_txx[k] = e.xx;
         a.ovo_tzz[k] = e.zz;
@@ -357,8 +389,8 @@ __device__ __forceinline__ void fwd_tile(const FwdFusedArgs &a, int s, float *sm
 __device__ __forceinline__ void tile_strips(const StripSaveArgs &a, int s) {
   const Dims d = slot_dims(a.d, a.shots[s]);
   const int lane = threadIdx.x & 31, nseg = (d.lb + 31) / 32;
-  const int w0 = (blockIdx.y * gridDim.x + blockIdx.x) * (kTileT / 32) + (threadIdx.x >> 5);
-  const int nw = gridDim.x * gridDim.y * (kTileT / 32);
+  const int w0 = (blockIdx.y * gridDim.x + blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5);
+  const int nw = gridDim.x * gridDim.y * (blockDim.x / 32);
   pdl_wait();
   pdl_launch();
   for (int w = w0; w < 2 * nseg; w += nw) {
@@ -383,8 +415,8 @@ struct FwdTileArgs {
   int n, nset, nst;
 };
 
-template <bool kPML, int TX, bool kBorn>
-__global__ void __launch_bounds__(kTileT, TX == 8 ? 3 : TX == 16 ? 2 : 1) k_fwd_tile(const __grid_constant__ FwdTileArgs a) {
+template <bool kPML, class C, bool kBorn>
+__global__ void __launch_bounds__(C::T, C::TX == 8 ? 3 : C::TX == 16 ? 2 : 1) k_fwd_tile(const __grid_constant__ FwdTileArgs a) {
   extern __shared__ __align__(16) float tsm[];
   const int m = blockIdx.z / a.n, s = blockIdx.z - m * a.n;
   if (m >= a.nset) {
@@ -393,10 +425,19 @@ __global__ void __launch_bounds__(kTileT, TX == 8 ? 3 : TX == 16 ? 2 : 1) k_fwd_
     return;
   }
   if (a.set[m].it < 0) return;
-  if (!kBorn) fwd_tile<kPML, TX, 0>(a.set[0], s, tsm);
-  else if (m == 0) fwd_tile<kPML, TX, 1>(a.set[0], s, tsm);
-  else if (m == 1) fwd_tile<kPML, TX, 2>(a.set[1], s, tsm);
-  else fwd_tile<kPML, TX, 3>(a.set[2], s, tsm);
+  const FwdFusedArgs &f = a.set[m];
+  constexpr int kRest = kPML ? kTilePml : kTileEdge;
+  if (tile_inner<C::TX>(f.d, f.shots[s])) {
+    if (!kBorn) fwd_tile<kTileInner, C, 0>(f, s, tsm);
+    else if (m == 0) fwd_tile<kTileInner, C, 1>(f, s, tsm);
+    else if (m == 1) fwd_tile<kTileInner, C, 2>(f, s, tsm);
+    else fwd_tile<kTileInner, C, 3>(f, s, tsm);
+  } else {
+    if (!kBorn) fwd_tile<kRest, C, 0>(f, s, tsm);
+    else if (m == 0) fwd_tile<kRest, C, 1>(f, s, tsm);
+    else if (m == 1) fwd_tile<kRest, C, 2>(f, s, tsm);
+    else fwd_tile<kRest, C, 3>(f, s, tsm);
+  }
 }
 
 // band_offset with the left / right bands first.
@@ -415,19 +456,19 @@ __device__ __forceinline__ int band_offset_lr(const Dims &d, int ix, int iz) {
 // Loads one velocity field of a reconstructed set: in tiles that reach the strip band, element by
 // element (strip value in the band, state elsewhere), otherwise by 16-byte copies.
 // kAc: the acoustic L^T keeps the left / right band's element where two bands meet (the corners).
-template <int TX, bool kAc = false>
+template <class C, bool kAc = false>
 __device__ __forceinline__ void tile_load_strip(float *dst, const float *src, const Dims &d,
                                                 int base, int s, int x0, int z0, const Strips &st,
                                                 int it, int comp, bool band) {
   if (!band) {
-    tile_load<TX>(dst, src, d, base, x0, z0);
+    tile_load<C>(dst, src, d, base, x0, z0);
     return;
   }
-  constexpr int kN = (TX + 16) * kTileC0, kL = (kN + kTileT - 1) / kTileT;
+  constexpr int kN = (C::TX + 16) * kTileC0, kL = (kN + C::T - 1) / C::T;
   float v[kL];
 #pragma unroll
   for (int j = 0; j < kL; j++) {
-    const int i = threadIdx.x + j * kTileT, r = i / kTileC0, c = i - r * kTileC0;
+    const int i = threadIdx.x + j * C::T, r = i / kTileC0, c = i - r * kTileC0;
     const int x = x0 - 8 + r, z = z0 - 8 + c;
     v[j] = 0.f;
     if (i < kN && x >= 0 && x < d.nxp && z >= 0 && z < d.nzp) {
@@ -437,8 +478,8 @@ __device__ __forceinline__ void tile_load_strip(float *dst, const float *src, co
   }
 #pragma unroll
   for (int j = 0; j < kL; j++) {
-    const int i = threadIdx.x + j * kTileT, r = i / kTileC0, c = i - r * kTileC0;
-    if (i < kN) dst[r * tile_p0(TX) + c] = v[j];
+    const int i = threadIdx.x + j * C::T, r = i / kTileC0, c = i - r * kTileC0;
+    if (i < kN) dst[r * C::P0 + c] = v[j];
   }
 }
 // Whether the tile's input window reaches the strip band (4 cells on either side of the interior's
@@ -449,18 +490,20 @@ __device__ __forceinline__ bool tile_has_band(const Dims &d, int x0, int z0) {
   return x0 - 8 < e || x0 + TX + 8 > d.nxp - e || z0 - 8 < e || z0 + kTileZ + 8 > d.nzp - e;
 }
 
-__host__ __device__ constexpr size_t bwd_tile_smem(int tx) { return tile_smem(tx, 4, 6); }
+template <class C>
+constexpr size_t bwd_tile_smem() { return C::smem(4, 6); }
 
-template <bool kPML, int TX>
+template <int kCls, class C>
 __device__ __forceinline__ void bwd_tile(const BwdFusedArgs &a, int s, float *sm) {
-  constexpr int R1 = (TX + 8) / 8, R2 = TX / 8, P0 = tile_p0(TX), N0 = tile_n0(TX), N1 = tile_n1(TX);
+  constexpr bool kPML = kCls == kTilePml, kIn = kCls == kTileInner;
+  constexpr int TX = C::TX, R1 = C::R1, R2 = C::R2, P0 = C::P0, N0 = C::N0, N1 = C::N1;
   float *const i_bx = sm, *const i_bz = sm + N0, *const i_ax = sm + 2 * N0, *const i_az = sm + 3 * N0;
   float *const m0 = sm + 4 * N0;  // btxx, btzz, btxz, PL, M, PzLx of the tile plus 4 cells
   const int tid = threadIdx.x;
   const ShotDev sh = a.shots[s];
   const Dims d = slot_dims(a.d, sh);
-  const int x0 = blockIdx.y * TX, z0 = blockIdx.x * kTileZ;
-  if (x0 >= d.nxp) return;
+  const int x0 = tile_x0<TX>(), z0 = tile_z0();
+  if (x0 >= d.nxp - d.nop) return;
   const int base = (int)(d.slot * s), ld = d.ld, pml = d.pml;
   const float dtdx = d.dt / d.dx, dtdz = d.dt / d.dz;
   const float rdx = 1.0f / d.dx, rdz = 1.0f / d.dz;
@@ -468,14 +511,14 @@ __device__ __forceinline__ void bwd_tile(const BwdFusedArgs &a, int s, float *sm
   const bool strips = kPML && a.strips_on, band = strips && tile_has_band<TX>(d, x0, z0);
   const int g1 = tid / kTileC1, c1 = tid - g1 * kTileC1, z1 = z0 - 4 + c1, xs1 = x0 - 4 + g1 * R1;
   const int g2 = tid >> 5, c2 = tid & 31, z2 = z0 + c2, xs2 = x0 + g2 * R2;
-  const bool zin1 = z1 >= 0 && z1 < d.nzp, zin2 = tid < 256 && z2 < d.nzp;
-  const bool zi1 = z1 >= pml && z1 < d.nzp - pml, zi2 = z2 >= pml && z2 < d.nzp - pml;
-  const bool zu1 = z1 >= d.nop && z1 < d.nzp - d.nop, zu2 = z2 >= d.nop && z2 < d.nzp - d.nop;
+  const bool zin1 = z1 >= 0 && z1 < d.nzp, zin2 = tid < 32 * C::G2 && (kIn || z2 < d.nzp);
+  const bool zi1 = kIn || (z1 >= pml && z1 < d.nzp - pml), zi2 = kIn || (z2 >= pml && z2 < d.nzp - pml);
+  const bool zu1 = kIn || (z1 >= d.nop && z1 < d.nzp - d.nop), zu2 = kIn || (z2 >= d.nop && z2 < d.nzp - d.nop);
   const int k1 = base + xs1 * ld + z1, k2 = base + xs2 * ld + z2;
-  auto in1 = [&](int r) { return zin1 && xs1 + r >= 0 && xs1 + r < d.nxp; };
-  auto in2 = [&](int r) { return zin2 && xs2 + r < d.nxp; };
-  auto xi = [&](int x) { return x >= pml && x < d.nxp - pml; };
-  auto xu = [&](int x) { return x >= d.nop && x < d.nxp - d.nop; };
+  auto in1 = [&](int r) { return kIn || (zin1 && xs1 + r >= 0 && xs1 + r < d.nxp); };
+  auto in2 = [&](int r) { return zin2 && (kIn || xs2 + r < d.nxp); };
+  auto xi = [&](int x) { return kIn || (x >= pml && x < d.nxp - pml); };
+  auto xu = [&](int x) { return kIn || (x >= d.nop && x < d.nxp - d.nop); };
   auto pm1 = [&](int r) { return tp && pml_cell(d, xs1 + r, z1); };
   auto pm2 = [&](int r) { return tp && pml_cell(d, xs2 + r, z2); };
   auto own1 = [&](int r) {
@@ -524,10 +567,10 @@ __device__ __forceinline__ void bwd_tile(const BwdFusedArgs &a, int s, float *sm
   }
   pdl_wait();
   // ---- state -------------------------------------------------------------------------------------
-  tile_load<TX>(i_ax, a.aa.vx, d, base, x0, z0);
-  tile_load<TX>(i_az, a.aa.vz, d, base, x0, z0);
-  tile_load_strip<TX>(i_bx, a.ra.vx, d, base, s, x0, z0, a.st, a.it, 0, band);
-  tile_load_strip<TX>(i_bz, a.ra.vz, d, base, s, x0, z0, a.st, a.it, 1, band);
+  tile_load<C, kIn>(i_ax, a.aa.vx, d, base, x0, z0);
+  tile_load<C, kIn>(i_az, a.aa.vz, d, base, x0, z0);
+  tile_load_strip<C>(i_bx, a.ra.vx, d, base, s, x0, z0, a.st, a.it, 0, band);
+  tile_load_strip<C>(i_bz, a.ra.vz, d, base, s, x0, z0, a.st, a.it, 1, band);
   cp_async_commit();
   float s1[R1][9];  // btxx btzz btxz atxx atzz atxz (or its two split parts), images pp, ps
 #pragma unroll
@@ -725,29 +768,31 @@ __device__ __forceinline__ void bwd_tile(const BwdFusedArgs &a, int s, float *sm
 // ---- reverse step of the first-order scattered set (arithmetic of k_bwd_scat_ring and k_born) -----
 // The Born source of the background's reconstructed velocities is formed here from those
 // velocities instead of being written and read back.
-__host__ __device__ constexpr size_t scat_tile_smem(int tx) { return tile_smem(tx, 4, 3); }
+template <class C>
+constexpr size_t scat_tile_smem() { return C::smem(4, 3); }
 
-template <bool kPML, int TX>
+template <int kCls, class C>
 __device__ __forceinline__ void scat_tile(const BwdScatArgs &a, const float *fvx, const float *fvz,
                                           int s, float *sm) {
-  constexpr int R1 = (TX + 8) / 8, R2 = TX / 8, P0 = tile_p0(TX), N0 = tile_n0(TX), N1 = tile_n1(TX);
+  constexpr bool kPML = kCls == kTilePml, kIn = kCls == kTileInner;
+  constexpr int TX = C::TX, R1 = C::R1, R2 = C::R2, P0 = C::P0, N0 = C::N0, N1 = C::N1;
   float *const i_bx = sm, *const i_bz = sm + N0, *const i_fx = sm + 2 * N0, *const i_fz = sm + 3 * N0;
   float *const m0 = sm + 4 * N0;  // btxx, btzz, btxz plus the Born source
   const int tid = threadIdx.x;
   const Dims d = slot_dims(a.d, a.shots[s]);
-  const int x0 = blockIdx.y * TX, z0 = blockIdx.x * kTileZ;
-  if (x0 >= d.nxp) return;
+  const int x0 = tile_x0<TX>(), z0 = tile_z0();
+  if (x0 >= d.nxp - d.nop) return;
   const int base = (int)(d.slot * s), ld = d.ld, pml = d.pml;
   const float dtdx = d.dt / d.dx, dtdz = d.dt / d.dz;
   const float rdx = 1.0f / d.dx, rdz = 1.0f / d.dz;
   const bool band = kPML && a.strips_on && tile_has_band<TX>(d, x0, z0);
   const int g1 = tid / kTileC1, c1 = tid - g1 * kTileC1, z1 = z0 - 4 + c1, xs1 = x0 - 4 + g1 * R1;
   const int g2 = tid >> 5, c2 = tid & 31, z2 = z0 + c2, xs2 = x0 + g2 * R2;
-  const bool zin1 = z1 >= 0 && z1 < d.nzp, zi1 = z1 >= pml && z1 < d.nzp - pml;
-  const bool zi2 = tid < 256 && z2 >= pml && z2 < d.nzp - pml;
+  const bool zin1 = z1 >= 0 && z1 < d.nzp, zi1 = kIn || (z1 >= pml && z1 < d.nzp - pml);
+  const bool zi2 = tid < 32 * C::G2 && (kIn || (z2 >= pml && z2 < d.nzp - pml));
   const int k1 = base + xs1 * ld + z1, k2 = base + xs2 * ld + z2;
-  auto in1 = [&](int r) { return zin1 && xs1 + r >= 0 && xs1 + r < d.nxp; };
-  auto xi = [&](int x) { return x >= pml && x < d.nxp - pml; };
+  auto in1 = [&](int r) { return kIn || (zin1 && xs1 + r >= 0 && xs1 + r < d.nxp); };
+  auto xi = [&](int x) { return kIn || (x >= pml && x < d.nxp - pml); };
   auto own1 = [&](int r) {
     const int x = xs1 + r;
     return x >= x0 && x < x0 + TX && c1 >= 4 && c1 < 4 + kTileZ;
@@ -769,10 +814,10 @@ __device__ __forceinline__ void scat_tile(const BwdScatArgs &a, const float *fvx
 #pragma unroll
   for (int r = 0; r < R2; r++) b_[r] = zi2 && xi(xs2 + r) ? __ldg(a.p.b + k2 + r * ld) : 0.f;
   pdl_wait();
-  tile_load<TX>(i_fx, fvx, d, base, x0, z0);
-  tile_load<TX>(i_fz, fvz, d, base, x0, z0);
-  tile_load_strip<TX>(i_bx, a.ra.vx, d, base, s, x0, z0, a.st, a.it, 0, band);
-  tile_load_strip<TX>(i_bz, a.ra.vz, d, base, s, x0, z0, a.st, a.it, 1, band);
+  tile_load<C, kIn>(i_fx, fvx, d, base, x0, z0);
+  tile_load<C, kIn>(i_fz, fvz, d, base, x0, z0);
+  tile_load_strip<C>(i_bx, a.ra.vx, d, base, s, x0, z0, a.st, a.it, 0, band);
+  tile_load_strip<C>(i_bz, a.ra.vz, d, base, s, x0, z0, a.st, a.it, 1, band);
   cp_async_commit();
   float s1[R1][8];  // btxx btzz btxz | atxx atzz atxz, images of own interior cells
 #pragma unroll
@@ -880,17 +925,20 @@ struct BwdTileArgs {
   const float *fvx, *fvz;
   int n;
 };
-// Register budget at 8 rows: 64 (3 CTAs an SM) without a PML and for the two-slice launch, where the
-// occupancy gains more than a few spilled values cost (16 shots of 1201x401: random 31.3 -> 28.3 ms,
-// ELSRTM 143 -> 138 ms); 96 for the PML step alone (41.5 against 44.5 ms).
-template <bool kPML, int TX, bool kScat>
-__global__ void __launch_bounds__(kTileT, TX == 8 ? (!kPML || kScat ? 3 : 2) : TX == 16 ? 2 : 1) k_bwd_tile(const __grid_constant__ BwdTileArgs a) {
+// Register budget: 64 (3 CTAs an SM of 8 rows, 2 of 16) except for the PML step alone at 8 rows: the
+// occupancy gains more than a few spilled values cost.
+template <bool kPML, class C, bool kScat>
+__global__ void __launch_bounds__(C::T, C::TX == 8 ? (!kPML || kScat ? 3 : 2) : C::TX == 16 ? 2 : 1) k_bwd_tile(const __grid_constant__ BwdTileArgs a) {
   extern __shared__ __align__(16) float tsm[];
   const int m = blockIdx.z / a.n, s = blockIdx.z - m * a.n;
+  constexpr int kRest = kPML ? kTilePml : kTileEdge;
   if (m == 0) {
-    if (a.b.it >= 0) bwd_tile<kPML, TX>(a.b, s, tsm);
+    if (a.b.it < 0) return;
+    if (tile_inner<C::TX>(a.b.d, a.b.shots[s])) bwd_tile<kTileInner, C>(a.b, s, tsm);
+    else bwd_tile<kRest, C>(a.b, s, tsm);
   } else if (kScat && a.sc.it >= 0) {
-    scat_tile<kPML, TX>(a.sc, a.fvx, a.fvz, s, tsm);
+    if (tile_inner<C::TX>(a.sc.d, a.sc.shots[s])) scat_tile<kTileInner, C>(a.sc, a.fvx, a.fvz, s, tsm);
+    else scat_tile<kRest, C>(a.sc, a.fvx, a.fvz, s, tsm);
   }
 }
 
@@ -919,29 +967,31 @@ struct AcTileArgs {
   const int *rmap;
   float *rec_vz, *rec_vx;  // scattered set: records
 };
-__host__ __device__ constexpr size_t ac_tile_smem(int tx) { return tile_smem(tx, 1, 2); }
+template <class C>
+constexpr size_t ac_tile_smem() { return C::smem(1, 2); }
 
-template <bool kPML, int TX, bool kScat>
+template <int kCls, class C, bool kScat, bool kCtxPml>
 __device__ __forceinline__ void ac_tile(const AcTileArgs &a, int s, float *sm) {
-  constexpr int R1 = (TX + 8) / 8, R2 = TX / 8, P0 = tile_p0(TX), N0 = tile_n0(TX);
-  constexpr int kLd = ((TX + 16) * (kTileC0 / 4) + kTileT - 1) / kTileT;
-  float *const i_s = sm, *const v_x = sm + N0, *const v_z = v_x + tile_n1(TX);
+  constexpr bool kPML = kCls == kTilePml, kIn = kCls == kTileInner;
+  constexpr int TX = C::TX, R1 = C::R1, R2 = C::R2, P0 = C::P0, N0 = C::N0;
+  constexpr int kLd = C::kLd;
+  float *const i_s = sm, *const v_x = sm + N0, *const v_z = v_x + C::N1;
   const int tid = threadIdx.x;
   const ShotDev sh = a.shots[s];
   const Dims d = slot_dims(a.d, sh);
-  const int x0 = blockIdx.y * TX, z0 = blockIdx.x * kTileZ;
-  if (x0 >= d.nxp) return;
+  const int x0 = tile_x0<TX>(), z0 = tile_z0();
+  if (x0 >= d.nxp - d.nop) return;
   const int base = (int)(d.slot * s), ld = d.ld;
   const float cx = d.dt / d.dx, cz = d.dt / d.dz;
   const bool tp = kPML && tile_has_pml<TX>(d, x0, z0, 4);
   const int g1 = tid / kTileC1, c1 = tid - g1 * kTileC1, z1 = z0 - 4 + c1, xs1 = x0 - 4 + g1 * R1;
   const int g2 = tid >> 5, c2 = tid & 31, z2 = z0 + c2, xs2 = x0 + g2 * R2;
   const bool zu1 = z1 >= d.nop && z1 < d.nzp - d.nop;
-  const bool zu2 = tid < 256 && z2 >= d.nop && z2 < d.nzp - d.nop;
-  const bool zi2 = z2 >= d.pml && z2 < d.nzp - d.pml;
+  const bool zu2 = tid < 32 * C::G2 && (kIn || (z2 >= d.nop && z2 < d.nzp - d.nop));
+  const bool zi2 = kIn || (z2 >= d.pml && z2 < d.nzp - d.pml);
   const int k1 = base + xs1 * ld + z1, k2 = base + xs2 * ld + z2;
-  auto up1 = [&](int r) { return zu1 && xs1 + r >= d.nop && xs1 + r < d.nxp - d.nop; };
-  auto up2 = [&](int r) { return zu2 && xs2 + r >= d.nop && xs2 + r < d.nxp - d.nop; };
+  auto up1 = [&](int r) { return kIn || (zu1 && xs1 + r >= d.nop && xs1 + r < d.nxp - d.nop); };
+  auto up2 = [&](int r) { return zu2 && (kIn || (xs2 + r >= d.nop && xs2 + r < d.nxp - d.nop)); };
   auto pm1 = [&](int r) { return tp && pml_cell(d, xs1 + r, z1); };
   auto pm2 = [&](int r) { return tp && pml_cell(d, xs2 + r, z2); };
   auto own1 = [&](int r) {
@@ -971,20 +1021,20 @@ __device__ __forceinline__ void ac_tile(const AcTileArgs &a, int s, float *sm) {
       q2z[r] = __ldg(a.dampz + k2 + r * ld);
     }
     m_[r] = 0.f;
-    if (!kScat && a.e_out && up2(r) && zi2 && xs2 + r >= d.pml && xs2 + r < d.nxp - d.pml)
+    if (!kScat && a.e_out && up2(r) && zi2 && (kIn || (xs2 + r >= d.pml && xs2 + r < d.nxp - d.pml)))
       m_[r] = __ldg(a.m + k2 + r * ld);
   }
   const float sval = kScat ? 0.f : __ldg(a.wavelet + a.it);
   pdl_wait();
-  tile_load<TX>(i_s, a.s, d, base, x0, z0);
+  tile_load<C, kIn>(i_s, a.s, d, base, x0, z0);
   cp_async_commit();
   float4 ov[kScat ? kLd : 1];
   if (kScat) {
 #pragma unroll
     for (int j = 0; j < kLd; j++) {
-      const int i = tid + j * kTileT, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
+      const int i = tid + j * C::T, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
       const int x = x0 - 8 + r, z = z0 - 8 + c;
-      const bool in = r < TX + 16 && x >= 0 && x < d.nxp && z >= 0 && z < ld;
+      const bool in = r < TX + 16 && (kIn || (x >= 0 && x < d.nxp && z >= 0 && z < ld));
       ov[j] = in ? *reinterpret_cast<const float4 *>(a.e_in + base + x * ld + z)
                  : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -1011,7 +1061,7 @@ __device__ __forceinline__ void ac_tile(const AcTileArgs &a, int s, float *sm) {
   if (kScat) {
 #pragma unroll
     for (int j = 0; j < kLd; j++) {
-      const int i = tid + j * kTileT, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
+      const int i = tid + j * C::T, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
       if (r >= TX + 16) continue;
       float4 *p = reinterpret_cast<float4 *>(i_s + r * P0 + c);
       float4 v = *p;
@@ -1021,7 +1071,7 @@ __device__ __forceinline__ void ac_tile(const AcTileArgs &a, int s, float *sm) {
   } else {
     const int r = sh.isx - (x0 - 8), c = sh.isz - (z0 - 8);
     if (r >= 0 && r < TX + 16 && c >= 0 && c < kTileC0 &&
-        tid == (r * (kTileC0 / 4) + c / 4) % kTileT)
+        tid == (r * (kTileC0 / 4) + c / 4) % C::T)
       i_s[r * P0 + c] += sval;
   }
   __syncthreads();
@@ -1074,10 +1124,10 @@ __device__ __forceinline__ void ac_tile(const AcTileArgs &a, int s, float *sm) {
         a.sz_n[k] = nz;
         a.s_n[k] = nx + nz;
       } else {
-        a.s_n[k] = fmaf(lam, ac_sum<kPML>(cx, dx[r], cz, dz), s2[r][0]);
+        a.s_n[k] = fmaf(lam, ac_sum<kCtxPml>(cx, dx[r], cz, dz), s2[r][0]);
       }
-      if (!kScat && a.e_out && zi2 && xs2 + r >= d.pml && xs2 + r < d.nxp - d.pml)
-        a.e_out[k] = -2.0f * lam * m_[r] * ac_sum<kPML>(1.0f / d.dx, dx[r], 1.0f / d.dz, dz);
+      if (!kScat && a.e_out && zi2 && (kIn || (xs2 + r >= d.pml && xs2 + r < d.nxp - d.pml)))
+        a.e_out[k] = -2.0f * lam * m_[r] * ac_sum<kCtxPml>(1.0f / d.dx, dx[r], 1.0f / d.dz, dz);
     }
   }
 }
@@ -1089,15 +1139,22 @@ struct AcFwdTileArgs {
   StripSaveArgs st;
   int n, nset;
 };
-template <bool kPML, int TX>
-__global__ void __launch_bounds__(kTileT, 2) k_ac_tile(const __grid_constant__ AcFwdTileArgs a) {
+template <bool kPML, class C>
+__global__ void __launch_bounds__(C::T, 2) k_ac_tile(const __grid_constant__ AcFwdTileArgs a) {
   extern __shared__ __align__(16) float tsm[];
   const int m = blockIdx.z / a.n, s = blockIdx.z - m * a.n;
   if (m >= a.nset) {
     if (a.st.it >= 0) tile_strips(a.st, s);
   } else if (a.set[m].it >= 0) {
-    if (m == 0) ac_tile<kPML, TX, false>(a.set[0], s, tsm);
-    else ac_tile<kPML, TX, true>(a.set[1], s, tsm);
+    constexpr int kRest = kPML ? kTilePml : kTileEdge;
+    const AcTileArgs &f = a.set[m];
+    if (tile_inner<C::TX>(f.d, f.shots[s])) {
+      if (m == 0) ac_tile<kTileInner, C, false, kPML>(f, s, tsm);
+      else ac_tile<kTileInner, C, true, kPML>(f, s, tsm);
+    } else {
+      if (m == 0) ac_tile<kRest, C, false, kPML>(f, s, tsm);
+      else ac_tile<kRest, C, true, kPML>(f, s, tsm);
+    }
   }
 }
 
@@ -1118,20 +1175,21 @@ struct AcRevTileArgs {
   const float *res_vz, *res_vx;
   Strips st;
 };
-__host__ __device__ constexpr size_t ac_rev_tile_smem(int tx) { return tile_smem(tx, 4, 4); }
+template <class C>
+constexpr size_t ac_rev_tile_smem() { return C::smem(4, 4); }
 
-template <bool kPML, int TX>
-__global__ void __launch_bounds__(kTileT, 2) k_ac_rev_tile(const __grid_constant__ AcRevTileArgs a) {
-  extern __shared__ __align__(16) float tsm[];
-  constexpr int R1 = (TX + 8) / 8, R2 = TX / 8, P0 = tile_p0(TX), N0 = tile_n0(TX), N1 = tile_n1(TX);
-  constexpr int kLd = ((TX + 16) * (kTileC0 / 4) + kTileT - 1) / kTileT;
+template <int kCls, class C, bool kCtxPml>
+__device__ __forceinline__ void ac_rev_tile(const AcRevTileArgs &a, float *tsm) {
+  constexpr bool kPML = kCls == kTilePml, kIn = kCls == kTileInner;
+  constexpr int TX = C::TX, R1 = C::R1, R2 = C::R2, P0 = C::P0, N0 = C::N0, N1 = C::N1;
+  constexpr int kLd = C::kLd;
   float *const i_vx = tsm, *const i_vz = tsm + N0, *const i_wx = tsm + 2 * N0;
   float *const m0 = tsm + 4 * N0;  // ux, uz, background stress + source, gradient factor
   const int tid = threadIdx.x, s = blockIdx.z;
   const ShotDev sh = a.shots[s];
   const Dims d = slot_dims(a.d, sh);
-  const int x0 = blockIdx.y * TX, z0 = blockIdx.x * kTileZ;
-  if (x0 >= d.nxp) return;
+  const int x0 = tile_x0<TX>(), z0 = tile_z0();
+  if (x0 >= d.nxp - d.nop) return;
   const int base = (int)(d.slot * s), ld = d.ld, pml = d.pml;
   const float cx = d.dt / d.dx, cz = d.dt / d.dz;
   const bool tp = kPML && tile_has_pml<TX>(d, x0, z0, 8);  // the adjoint's split stress is read
@@ -1139,17 +1197,17 @@ __global__ void __launch_bounds__(kTileT, 2) k_ac_rev_tile(const __grid_constant
   float *const i_wz = kPML && tp ? tsm + 3 * N0 : i_wx;  // x and z parts differ in the PML only
   const int g1 = tid / kTileC1, c1 = tid - g1 * kTileC1, z1 = z0 - 4 + c1, xs1 = x0 - 4 + g1 * R1;
   const int g2 = tid >> 5, c2 = tid & 31, z2 = z0 + c2, xs2 = x0 + g2 * R2;
-  const bool zu1 = z1 >= d.nop && z1 < d.nzp - d.nop, zi1 = z1 >= pml && z1 < d.nzp - pml;
-  const bool zu2 = tid < 256 && z2 >= d.nop && z2 < d.nzp - d.nop;
-  const bool zi2 = z2 >= pml && z2 < d.nzp - pml;
+  const bool zu1 = z1 >= d.nop && z1 < d.nzp - d.nop, zi1 = kIn || (z1 >= pml && z1 < d.nzp - pml);
+  const bool zu2 = tid < 32 * C::G2 && (kIn || (z2 >= d.nop && z2 < d.nzp - d.nop));
+  const bool zi2 = kIn || (z2 >= pml && z2 < d.nzp - pml);
   const int k1 = base + xs1 * ld + z1, k2 = base + xs2 * ld + z2;
-  auto xi = [&](int x) { return x >= pml && x < d.nxp - pml; };
-  auto in1 = [&](int r) { return z1 >= 0 && z1 < d.nzp && xs1 + r >= 0 && xs1 + r < d.nxp; };
-  auto up1 = [&](int r) { return zu1 && xs1 + r >= d.nop && xs1 + r < d.nxp - d.nop; };
-  auto up2 = [&](int r) { return zu2 && xs2 + r >= d.nop && xs2 + r < d.nxp - d.nop; };
+  auto xi = [&](int x) { return kIn || (x >= pml && x < d.nxp - pml); };
+  auto in1 = [&](int r) { return kIn || (z1 >= 0 && z1 < d.nzp && xs1 + r >= 0 && xs1 + r < d.nxp); };
+  auto up1 = [&](int r) { return kIn || (zu1 && xs1 + r >= d.nop && xs1 + r < d.nxp - d.nop); };
+  auto up2 = [&](int r) { return zu2 && (kIn || (xs2 + r >= d.nop && xs2 + r < d.nxp - d.nop)); };
   // cells where the background is rebuilt
-  auto rb1 = [&](int r) { return kPML ? zi1 && xi(xs1 + r) : up1(r); };
-  auto rb2 = [&](int r) { return kPML ? zu2 && zi2 && xi(xs2 + r) : up2(r); };
+  auto rb1 = [&](int r) { return kCtxPml ? zi1 && xi(xs1 + r) : up1(r); };
+  auto rb2 = [&](int r) { return kCtxPml ? zu2 && zi2 && xi(xs2 + r) : up2(r); };
   auto pm1 = [&](int r) { return tp && pml_cell(d, xs1 + r, z1); };
   auto pm2 = [&](int r) { return tp && pml_cell(d, xs2 + r, z2); };
   auto own1 = [&](int r) {
@@ -1189,23 +1247,23 @@ __global__ void __launch_bounds__(kTileT, 2) k_ac_rev_tile(const __grid_constant
   float4 lw[kLd];  // lam on the input chunks (outside the PML)
 #pragma unroll
   for (int j = 0; j < kLd; j++) {
-    const int i = tid + j * kTileT, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
+    const int i = tid + j * C::T, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
     const int x = x0 - 8 + r, z = z0 - 8 + c;
-    const bool in = r < TX + 16 && x >= 0 && x < d.nxp && z >= 0 && z < ld;
+    const bool in = r < TX + 16 && (kIn || (x >= 0 && x < d.nxp && z >= 0 && z < ld));
     lw[j] = in ? __ldg(reinterpret_cast<const float4 *>(a.lam + base + x * ld + z))
                : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const float sval = __ldg(a.wavelet + a.it);
   pdl_wait();
-  tile_load_strip<TX, true>(i_vx, a.vx, d, base, s, x0, z0, a.st, a.it, 0, band);
-  tile_load_strip<TX, true>(i_vz, a.vz, d, base, s, x0, z0, a.st, a.it, 1, band);
+  tile_load_strip<C, true>(i_vx, a.vx, d, base, s, x0, z0, a.st, a.it, 0, band);
+  tile_load_strip<C, true>(i_vz, a.vz, d, base, s, x0, z0, a.st, a.it, 1, band);
   cp_async_commit();
 #pragma unroll
   for (int j = 0; j < kLd; j++) {
-    const int i = tid + j * kTileT, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
+    const int i = tid + j * C::T, r = i / (kTileC0 / 4), c = (i - r * (kTileC0 / 4)) * 4;
     const int x = x0 - 8 + r, z = z0 - 8 + c;
     if (r >= TX + 16) continue;
-    const bool in = x >= 0 && x < d.nxp && z >= 0 && z < ld;
+    const bool in = kIn || (x >= 0 && x < d.nxp && z >= 0 && z < ld);
     const int k = in ? base + x * ld + z : base;
     const float4 y = in ? *reinterpret_cast<const float4 *>(a.ys + k) : make_float4(0.f, 0.f, 0.f, 0.f);
     float4 wx = make_float4(lw[j].x * y.x, lw[j].y * y.y, lw[j].z * y.z, lw[j].w * y.w), wz = wx;
@@ -1284,8 +1342,8 @@ __global__ void __launch_bounds__(kTileT, 2) k_ac_rev_tile(const __grid_constant
       }
       if (rb1(r)) {
         const float dz = tile_dzm(i_vz + o + r * P0);
-        sn = fmaf(-lam1[r], ac_sum<kPML>(cx, dx[r], cz, dz), sn);
-        f = -2.0f * lam1[r] * ac_sum<kPML>(1.0f / d.dx, dx[r], 1.0f / d.dz, dz);
+        sn = fmaf(-lam1[r], ac_sum<kCtxPml>(cx, dx[r], cz, dz), sn);
+        f = -2.0f * lam1[r] * ac_sum<kCtxPml>(1.0f / d.dx, dx[r], 1.0f / d.dz, dz);
         if (own1(r)) a.s_n[k] = sn;
       }
       if (z1 == sh.isz && xs1 + r == sh.isx) sn += sval;
@@ -1324,6 +1382,13 @@ __global__ void __launch_bounds__(kTileT, 2) k_ac_rev_tile(const __grid_constant
       }
     }
   }
+}
+
+template <bool kPML, class C>
+__global__ void __launch_bounds__(C::T, 2) k_ac_rev_tile(const __grid_constant__ AcRevTileArgs a) {
+  extern __shared__ __align__(16) float tsm[];
+  if (tile_inner<C::TX>(a.d, a.shots[blockIdx.z])) ac_rev_tile<kTileInner, C, kPML>(a, tsm);
+  else ac_rev_tile<kPML ? kTilePml : kTileEdge, C, kPML>(a, tsm);
 }
 
 }  // namespace ds2d
