@@ -1,7 +1,7 @@
 // Backward RTM step of k_bwd_ring (random boundary) with its operand rows fed by bulk copies.
 //
 // The one-column backward step executes most of its instructions on per-row work rather than on
-// the stencils: every thread issues its own 18 cp.async copies a row step (addresses, range
+// the stencils: every thread of k_bwd_ring issues its own 18 cp.async copies a row step (addresses, range
 // predicates, zero stores for rows outside the window) and waits on its own commit groups.  Here
 // one cp.async.bulk per field row copies it for the whole CTA (global -> shared, completion
 // counted on the ring slot's mbarrier), as in the pair kernels of ds2d_pair.cuh, and every
@@ -26,7 +26,11 @@
 namespace ds2d {
 
 constexpr int kBulkRing = 4;
-constexpr int kBwdBulkFields = 18;
+// bvx bvz avx avz | btxx btzz btxz atxx atzz atxz lam mu, images pp ps | b, illumination.  The
+// imaging weights are made from lam and mu (-2 rho vp^2 = -2 (lam + 2 mu), -2 rho vs^2 = -2 mu),
+// and no row of a uniform density's b is copied: 112 bytes per cell instead of 124
+// (RTM of 60 shots of 1201x401, 250 steps: 371.2 -> 366.8 ms; the issue slots bound it).
+constexpr int kBwdBulkFields = 16;
 __host__ __device__ constexpr size_t bwd_bulk_smem(int kT) {
   return sizeof(float) * (size_t)kBulkRing * kBwdBulkFields * kT + 8 * kBulkRing;
 }
@@ -95,13 +99,13 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
     const long long ibase = (long long)s * d.wnx_max * d.ild - (long long)pml * ld;
     const float *src[NF] = {a.ra.vx,  a.ra.vz,  a.aa.vx,  a.aa.vz,  a.ra.txx, a.ra.tzz,
                             a.ra.txz, a.aa.txx, a.aa.tzz, a.aa.txz, a.p.lam,  a.p.mu,
-                            a.p.kpp,  a.p.kps,  img_pp,   img_ps,   a.p.b,    img_il};
+                            img_pp,   img_ps,   a.p.bconst != 0.f ? nullptr : a.p.b, img_il};
 #pragma unroll
     for (int f = 0; f < NF; f++)
       if (my_f == f) {
-        const bool img = f == 14 || f == 15 || f == 17;
-        fd.src = src[f] + (img ? ibase : fbase);
-        fd.lag = f < 4 ? 0 : (f < 16 ? 4 : 8);
+        const bool img = f == 12 || f == 13 || f == 15;
+        fd.src = src[f] ? src[f] + (img ? ibase : fbase) : nullptr;
+        fd.lag = f < 4 ? 0 : (f < 14 ? 4 : 8);
         fd.lo = img ? pml : 0;
         fd.hi = img ? d.nxp - pml : d.nxp;
       }
@@ -258,11 +262,11 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
       PzLx = l2m * atzz + lam * atxx;
       if (own && x_int && z_int) {
         const int o = (img_row + (r1 - pml)) * d.ild + z;
-        const float kpp = S[12 * kT], kps = S[13 * kT];
+        const float kpp = -2.0f * l2m, kps = -2.0f * mu;  // -2 rho vp^2, -2 rho vs^2
         const float lamda_grad = (gx_vx + gz_vz) * (atxx + atzz);
         const float miu_grad = -2.0f * (gx_vx * atzz + gz_vz * atxx) + (gz_vx + gx_vz) * atxz;
-        img_pp[o] = S[14 * kT] + kpp * lamda_grad;
-        img_ps[o] = S[15 * kT] + kps * miu_grad;
+        img_pp[o] = S[12 * kT] + kpp * lamda_grad;
+        img_ps[o] = S[13 * kT] + kps * miu_grad;
       }
     }
     push(w_btxx, btxx);
@@ -283,7 +287,7 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
     if (c2 && zin && r2 >= x0 && r2 < x1) {
       const int k = base + r2 * ld + z;
       const bool x_int = r2 >= pml && r2 < d.nxp - pml;
-      const float bb = S[16 * kT];
+      const float bb = a.p.bconst != 0.f ? a.p.bconst : S[14 * kT];
       const float cbx = bb * dtdx, cbz = bb * dtdz;
       if (x_int && z_int) {
         const float ax = dxp_mid(w_btxx);
@@ -295,7 +299,7 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
         a.rb.vx[k] = vx;
         a.rb.vz[k] = vz;
         const int o = (img_row + (r2 - pml)) * d.ild + z;
-        img_il[o] = S[17 * kT] + (vx * vx + vz * vz);
+        img_il[o] = S[15 * kT] + (vx * vx + vz * vz);
       }
       if (r2 >= d.nop && r2 < d.nxp - d.nop && z_upd) {
         const float t_x = dxp_mid(w_PL);

@@ -579,6 +579,8 @@ int setup_batch(ds2d_ctx *c, int n, int shot_base, bool with_image) {
   a.L = std::log10((double)(1.0f / 0.001f));  // rr = 0.001 (FD2DGPU.cu:1299)
   a.seed = c->o.seed;
   a.shot_base = shot_base;
+  // every density b of the windows is then this value (k_setup's expression)
+  c->par.bconst = c->rho_all ? 0.f : (float)(1.0 / (double)2000.0f);
   dim3 grid((c->d.ld + 127) / 128, c->d.nxp, n);
   k_setup<<<grid, 128, 0, c->stream>>>(a);
   CK(cudaGetLastError());
@@ -639,6 +641,8 @@ constexpr double kBytesAcRev = 64;
 // Fused backward RTM step per padded cell: source and adjoint fields r/w (2 x 40), b, lam, mu
 // (12), imaging weights (8) and three image accumulators r/w (24).
 constexpr double kBytesBwdFused = 124;
+// k_bwd_bulk: no imaging weights read (made from lam and mu), b read only if a density is set.
+constexpr double kBytesBwdBulk = 112;
 #define CELLS(n) (c->batch_cells)
 #define WCELLS(n) (c->batch_wcells)
 #define LAUNCH(kernel, grid, block, args) LAUNCHP(#kernel, 0, kernel, grid, block, args)
@@ -1375,7 +1379,7 @@ int rtm_batch_body(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base) {
         const int bxr = pair_xr(c, bns, c->occ_bulk[bulk_idx(bc, c->opt_bwd_1b != 0)]);
         a.tz = btz; a.xr = bxr; a.err = c->d_err;
         dim3 bgrid(bns, (d.nxp + bxr - 1) / bxr, n);
-        LAUNCHS("bwd_fused", kBytesBwdFused * CELLS(n), bulk_fn(bc, c->opt_bwd_1b != 0), bgrid,
+        LAUNCHS("bwd_fused", (kBytesBwdBulk + (c->rho_all ? 4 : 0)) * CELLS(n), bulk_fn(bc, c->opt_bwd_1b != 0), bgrid,
                 bc, bwd_bulk_smem(bc), a);
       } else if (ws_on(c)) {
         const int kt = c->opt_bwd_ws;

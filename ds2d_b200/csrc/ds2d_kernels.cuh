@@ -70,6 +70,7 @@ struct Strain {
 
 struct Par {
   const float *b, *lam, *mu, *dampx, *dampz, *kpp, *kps, *dmp, *dms;
+  float bconst;  // 1 / rho of a uniform density (no density array was set), else 0
 };
 
 // Saved boundary strips of one wavefield set: [slot][it][component][lb] elements in `prec`

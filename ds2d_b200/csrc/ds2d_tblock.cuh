@@ -156,7 +156,8 @@ __global__ void __launch_bounds__(kT, kMinB) k_fwd_tb(FwdFusedArgs a) {
         const float *src = f == 0 ? a.a.txx : f == 1 ? a.a.tzz : f == 2 ? a.a.txz
                          : f == 3 ? a.a.vx : f == 4 ? a.a.vz
                          : f < 5 + kK ? a.p.b : ((f - 5 - kK) & 1) ? a.p.mu : a.p.lam;
-        fd.src = src + fbase;
+        // no copies of a uniform density's b (Par::bconst): 48 of 52 bytes per cell are left
+        fd.src = f >= 5 && f < 5 + kK && a.p.bconst != 0.f ? nullptr : src + fbase;
         fd.lag = f < 3 ? 0 : f < 5 ? 4 : f < 5 + kK ? 4 + 8 * (f - 5) : 8 + 8 * ((f - 5 - kK) >> 1);
       }
     if (t == 0) {
@@ -231,7 +232,7 @@ __global__ void __launch_bounds__(kT, kMinB) k_fwd_tb(FwdFusedArgs a) {
     float bb[kK], lam[kK], mu[kK];
 #pragma unroll
     for (int k = 0; k < kK; k++) {
-      bb[k] = S[(5 + k) * kT];
+      bb[k] = kBulk && a.p.bconst != 0.f ? a.p.bconst : S[(5 + k) * kT];
       lam[k] = S[(5 + kK + 2 * k) * kT];
       mu[k] = S[(6 + kK + 2 * k) * kT];
     }

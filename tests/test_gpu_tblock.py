@@ -111,3 +111,33 @@ def test_time_blocked_uneven_windows_vs_oracle(cuda_device):
         assert rel(rz[off:off + s.ntr], oz) < GATE, (i, rel(rz[off:off + s.ntr], oz))
         assert rel(rx[off:off + s.ntr], ox) < GATE, (i, rel(rx[off:off + s.ntr], ox))
         off += s.ntr
+
+
+@pytest.mark.parametrize("allnz,cta", [(300, 128), (300, 256), (440, 192)])
+def test_uniform_density_as_constant_or_array(cuda_device, allnz, cta):
+    """The bulk-copy kernels take a uniform density's 1/rho as a launch constant and read it from
+    its array otherwise: the same value, so the same records and images to rounding (1e-6), on
+    one context whose density is set, changed and dropped between calls (replayed launches must
+    not keep the other kind's); a varying density gives the ring kernels' records."""
+    c, vp, vs, w, shots, obs = _case(allnz, nt=103)
+    vary = np.random.default_rng(2).uniform(1800, 2400, vp.shape).astype(np.float32)
+    outs = []
+    with Elastic2D(c["allnx"], c["allnz"], c["nx"], c["pml"], c["nt"], c["dx"], c["dz"], c["dt"],
+                   boundary="random", seed=5, max_shots=len(shots),
+                   max_ntr=max(s.ntr for s in shots)) as e:
+        e.set_wavelet(w)
+        for k, v in {"tile": 0, "tb": 2, "pair": 2, "bwd_bulk": 1, "bwd_cta": cta}.items():
+            e.set_option(k, v)
+        for rho in (None, np.full_like(vp, 2000), vary, None):
+            e.set_models(vp, vs, rho)
+            rec = e.forward(shots)
+            e.rtm(shots, obs[0], obs[1])
+            outs.append((*rec, *e.read_images().values()))
+        for k, v in {"tb": 0, "pair": 0, "bwd_bulk": 0}.items():
+            e.set_option(k, v)
+        e.set_models(vp, vs, vary)
+        ring = e.forward(shots)
+    for i in (1, 3):
+        assert all(rel(a, b) <= 1e-6 for a, b in zip(outs[i], outs[0]))
+    assert rel(outs[2][0], outs[0][0]) > 1e-3
+    assert all(rel(a, b) <= TB_GATE for a, b in zip(outs[2], ring))
