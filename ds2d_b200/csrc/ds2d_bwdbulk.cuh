@@ -59,8 +59,9 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
   constexpr int kD = kBulkRing, NF = kBwdBulkFields;
   extern __shared__ __align__(16) float ring[];  // [kD][NF][kT], then the slot barriers
   unsigned long long *bars = (unsigned long long *)(ring + (size_t)kD * NF * kT);
-  // z-tap rows: bvx bvz avx avz (stage 1), btxz btzz M PzLx (stage 2); two buffers with kOne
-  __shared__ float s_zt[kOne ? 2 : 1][8][kT];
+  // z-tap rows: (bvx, avx) (bvz, avz) (stage 1), (btxz, M) (btzz, PzLx) (stage 2); two buffers
+  // with kOne
+  __shared__ pair_t s_zt[kOne ? 2 : 1][4][kT];
   __shared__ int s_tr[16], s_has[16];
   __shared__ float s_rz[16], s_rx[16], s_ownx[16], s_ownz[16];
   const int s = blockIdx.z, t = threadIdx.x;
@@ -130,14 +131,15 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
   for (int j = 0; j < kD - 1; j++)
     issue_slot_col<kT>(fd, ring + (size_t)j * NF * kT, my_f, &bars[j], rs0 + j, ld, c0, lane);
 
-  float w_bvx[9], w_bvz[9], w_avx[9], w_avz[9];
-  // adjoint-velocity operands, as k_bwd_ring: PL = (l+2m) atxx + l atzz, PzLx = (l+2m) atzz + l atxx
-  float w_btxx[9], w_btxz[9], w_btzz[5], w_PL[9], w_M[9], w_PzLx[5];
+  // windows of (source field, adjoint field): the two fields' derivatives are the same operators.
+  // Adjoint-velocity operands as k_bwd_ring: PL = (l+2m) atxx + l atzz, M = mu atxz,
+  // PzLx = (l+2m) atzz + l atxx
+  pair_t w_vx[9], w_vz[9];                // (bvx, avx), (bvz, avz)
+  pair_t w_xx[9], w_xz[9], w_zz[5];       // (btxx, PL), (btxz, M), (btzz, PzLx)
 #pragma unroll
-  for (int i = 0; i < 9; i++)
-    w_bvx[i] = w_bvz[i] = w_avx[i] = w_avz[i] = w_btxx[i] = w_btxz[i] = w_PL[i] = w_M[i] = 0.f;
+  for (int i = 0; i < 9; i++) w_vx[i] = w_vz[i] = w_xx[i] = w_xz[i] = 0;
 #pragma unroll
-  for (int i = 0; i < 5; i++) w_btzz[i] = w_PzLx[i] = 0.f;
+  for (int i = 0; i < 5; i++) w_zz[i] = 0;
 
   RingCursor<kD> cur;
   bool ok = true, aborted = false;
@@ -179,25 +181,18 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
           n_avx += s_rx[r & 15];
         }
       }
-      push(w_bvx, n_bvx);
-      push(w_bvz, n_bvz);
-      push(w_avx, n_avx);
-      push(w_avz, n_avz);
+      push(w_vx, pk(n_bvx, n_avx));
+      push(w_vz, pk(n_bvz, n_avz));
     }
     const int r1 = r - 4;
-    float *const zb = s_zt[kOne ? (r & 1) : 0][0];
-    float *const s_bvx = zb, *const s_bvz = zb + kT, *const s_avx = zb + 2 * kT;
-    float *const s_avz = zb + 3 * kT, *const s_btxz = zb + 4 * kT, *const s_btzz = zb + 5 * kT;
-    float *const s_m = zb + 6 * kT, *const s_pzlx = zb + 7 * kT;
-    s_bvx[t] = w_bvx[4];
-    s_bvz[t] = w_bvz[4];
-    s_avx[t] = w_avx[4];
-    s_avz[t] = w_avz[4];
+    pair_t *const zb = s_zt[kOne ? (r & 1) : 0][0];
+    pair_t *const s_vx = zb + t, *const s_vz = s_vx + kT, *const s_xz = s_vx + 2 * kT;
+    pair_t *const s_zz = s_vx + 3 * kT;  // this thread's entries; neighbours at +-1 .. 4
+    s_vx[0] = w_vx[4];
+    s_vz[0] = w_vz[4];
     if (kOne) {  // stage-2 rows of row r - 8 (before this step's stage-1 push: index 5 / 1)
-      s_btxz[t] = w_btxz[5];
-      s_btzz[t] = w_btzz[1];
-      s_m[t] = w_M[5];
-      s_pzlx[t] = w_PzLx[1];
+      s_xz[0] = w_xz[5];
+      s_zz[0] = w_zz[1];
     }
     if (__syncthreads_or(!ok)) {
       aborted = true;
@@ -220,20 +215,26 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
       const bool x_int = r1 >= pml && r1 < d.nxp - pml;
       float gx_vx = 0.f, gz_vz = 0.f, gz_vx = 0.f, gx_vz = 0.f;
       const float lam = S[10 * kT], mu = S[11 * kT];
-      if (x_int && z_int) {
-        const float sa = dxm_mid(w_bvx);
-        const float sf = dxp_mid(w_bvz);
-        const float sb = stencil4([&](int i) { return s_bvz[t + i - 1] - s_bvz[t - i]; });
-        const float se = stencil4([&](int i) { return s_bvx[t + i] - s_bvx[t - i + 1]; });
+      const bool in_b = x_int && z_int;
+      const bool in_a = r1 >= d.nop && r1 < d.nxp - d.nop && z_upd;
+      float2 sa = {}, sf = {}, sb = {}, se = {};
+      if (in_a || in_b) {
+        // the own tap comes from the window, not from shared memory
+        sa = upk(dxm_mid(w_vx));
+        sf = upk(dxp_mid(w_vz));
+        sb = upk(stencil4x2([&](int i) { return sub2(i == 1 ? w_vz[4] : s_vz[i - 1], s_vz[-i]); }));
+        se = upk(stencil4x2([&](int i) { return sub2(s_vx[i], i == 1 ? w_vx[4] : s_vx[1 - i]); }));
+      }
+      if (in_b) {
         const float l2m = lam + 2.0f * mu;
         const float dir = -1.0f;
-        btxx = btxx + (dir * l2m * dtdx * sa + dir * lam * dtdz * sb);
-        btzz = btzz + (dir * lam * dtdx * sa + dir * l2m * dtdz * sb);
-        btxz = btxz + (dir * mu * dtdx * sf + dir * mu * dtdz * se);
-        gx_vx = sa * rdx;  // strains; reciprocal multiply
-        gz_vz = sb * rdz;
-        gz_vx = se * rdz;
-        gx_vz = sf * rdx;
+        btxx = btxx + (dir * l2m * dtdx * sa.x + dir * lam * dtdz * sb.x);
+        btzz = btzz + (dir * lam * dtdx * sa.x + dir * l2m * dtdz * sb.x);
+        btxz = btxz + (dir * mu * dtdx * sf.x + dir * mu * dtdz * se.x);
+        gx_vx = sa.x * rdx;  // strains; reciprocal multiply
+        gz_vz = sb.x * rdz;
+        gz_vx = se.x * rdz;
+        gx_vz = sf.x * rdx;
         if (own) {
           a.rb.txx[k] = btxx;
           a.rb.tzz[k] = btzz;
@@ -241,12 +242,8 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
         }
       }
       float atxx = 0.f, atzz = 0.f, atxz = 0.f;
-      if (r1 >= d.nop && r1 < d.nxp - d.nop && z_upd) {
-        const float sa = dxm_mid(w_avx);
-        const float sf = dxp_mid(w_avz);
-        const float sb = stencil4([&](int i) { return s_avz[t + i - 1] - s_avz[t - i]; });
-        const float se = stencil4([&](int i) { return s_avx[t + i] - s_avx[t - i + 1]; });
-        const float xx = -dtdx * sa, zz = -dtdz * sb, xz_x = -dtdx * sf, xz_z = -dtdz * se;
+      if (in_a) {
+        const float xx = -dtdx * sa.y, zz = -dtdz * sb.y, xz_x = -dtdx * sf.y, xz_z = -dtdz * se.y;
         atxx = S[7 * kT] + xx;
         atzz = S[8 * kT] + zz;
         atxz = S[9 * kT] + (xz_x + xz_z);
@@ -269,19 +266,14 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
         img_ps[o] = S[13 * kT] + kps * miu_grad;
       }
     }
-    push(w_btxx, btxx);
-    push(w_btxz, btxz);
-    push(w_btzz, btzz);
-    push(w_PL, PL);
-    push(w_M, M);
-    push(w_PzLx, PzLx);
+    push(w_xx, pk(btxx, PL));
+    push(w_xz, pk(btxz, M));
+    push(w_zz, pk(btzz, PzLx));
     // ---- stage 2: velocities of row r2 = r - 8 ---------------------------------------------
     const int r2 = r - 8;
     if (!kOne) {
-      s_btxz[t] = w_btxz[4];
-      s_btzz[t] = w_btzz[0];
-      s_m[t] = w_M[4];
-      s_pzlx[t] = w_PzLx[0];
+      s_xz[0] = w_xz[4];
+      s_zz[0] = w_zz[0];
       __syncthreads();
     }
     if (c2 && zin && r2 >= x0 && r2 < x1) {
@@ -289,26 +281,27 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
       const bool x_int = r2 >= pml && r2 < d.nxp - pml;
       const float bb = a.p.bconst != 0.f ? a.p.bconst : S[14 * kT];
       const float cbx = bb * dtdx, cbz = bb * dtdz;
-      if (x_int && z_int) {
-        const float ax = dxp_mid(w_btxx);
-        const float fx = dxm_mid(w_btxz);
-        const float bz = stencil4([&](int i) { return s_btxz[t + i - 1] - s_btxz[t - i]; });
-        const float ez = stencil4([&](int i) { return s_btzz[t + i] - s_btzz[t - i + 1]; });
-        const float vx = w_bvx[0] + (-cbx * ax + -cbz * bz);
-        const float vz = w_bvz[0] + (-cbx * fx + -cbz * ez);
+      const bool in_b = x_int && z_int;
+      const bool in_a = r2 >= d.nop && r2 < d.nxp - d.nop && z_upd;
+      float2 xx = {}, xz = {}, zx = {}, zz = {};
+      if (in_a || in_b) {
+        xx = upk(dxp_mid(w_xx));
+        xz = upk(dxm_mid(w_xz));
+        zx = upk(stencil4x2([&](int i) { return sub2(i == 1 ? w_xz[4] : s_xz[i - 1], s_xz[-i]); }));
+        zz = upk(stencil4x2([&](int i) { return sub2(s_zz[i], i == 1 ? w_zz[0] : s_zz[1 - i]); }));
+      }
+      if (in_b) {
+        const float vx = upk(w_vx[0]).x + (-cbx * xx.x + -cbz * zx.x);
+        const float vz = upk(w_vz[0]).x + (-cbx * xz.x + -cbz * zz.x);
         a.rb.vx[k] = vx;
         a.rb.vz[k] = vz;
         const int o = (img_row + (r2 - pml)) * d.ild + z;
         img_il[o] = S[15 * kT] + (vx * vx + vz * vz);
       }
-      if (r2 >= d.nop && r2 < d.nxp - d.nop && z_upd) {
-        const float t_x = dxp_mid(w_PL);
-        const float s_xz = dxm_mid(w_M);
-        const float t_xz = stencil4([&](int i) { return s_m[t + i - 1] - s_m[t - i]; });
-        const float s_z = stencil4([&](int i) { return s_pzlx[t + i] - s_pzlx[t - i + 1]; });
-        const float ux_x = -cbx * t_x, ux_z = -cbz * t_xz;
-        const float uz_x = -cbx * s_xz, uz_z = -cbz * s_z;
-        float ovx = w_avx[0], ovz = w_avz[0];
+      if (in_a) {
+        const float ux_x = -cbx * xx.y, ux_z = -cbz * zx.y;
+        const float uz_x = -cbx * xz.y, uz_z = -cbz * zz.y;
+        float ovx = upk(w_vx[0]).y, ovz = upk(w_vz[0]).y;
         if (rec_col) {  // receiver column: the state without the residual
           ovx = s_ownx[r2 & 15];
           ovz = s_ownz[r2 & 15];

@@ -56,8 +56,8 @@ struct FwdFusedArgs {
   int *err;  // device error word of the pair kernels' bounded waits (null: none)
 };
 
-template <int N>
-__device__ __forceinline__ void push(float (&w)[N], float v) {
+template <class T, int N>
+__device__ __forceinline__ void push(T (&w)[N], T v) {
 #pragma unroll
   for (int i = 0; i < N - 1; i++) w[i] = w[i + 1];
   w[N - 1] = v;
@@ -70,6 +70,12 @@ __device__ __forceinline__ float dxp_mid(const float (&w)[9]) {
 }
 __device__ __forceinline__ float dxm_mid(const float (&w)[9]) {
   return stencil4([&](int i) { return w[3 + i] - w[4 - i]; });
+}
+__device__ __forceinline__ pair_t dxp_mid(const pair_t (&w)[9]) {
+  return stencil4x2([&](int i) { return sub2(w[4 + i], w[5 - i]); });
+}
+__device__ __forceinline__ pair_t dxm_mid(const pair_t (&w)[9]) {
+  return stencil4x2([&](int i) { return sub2(w[3 + i], w[4 - i]); });
 }
 
 template <bool kPML>

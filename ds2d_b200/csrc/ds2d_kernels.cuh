@@ -95,6 +95,44 @@ __device__ __forceinline__ float stencil4(F f) {
   return t;
 }
 
+// Two FP32 values in one 64-bit register, for the packed arithmetic: each half is rounded as the
+// scalar operation rounds it, and one instruction does both.
+using pair_t = unsigned long long;
+__device__ __forceinline__ pair_t pk(float x, float y) {
+  pair_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 upk(pair_t a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ pair_t sub2(pair_t a, pair_t b) {
+  pair_t r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ pair_t mul2(pair_t a, pair_t b) {
+  pair_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c) {
+  pair_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// stencil4 of two fields, f(i) = the packed differences of tap i.
+template <class F>
+__device__ __forceinline__ pair_t stencil4x2(F f) {
+  pair_t t = mul2(pk(kC1, kC1), f(1));
+  t = fma2(pk(kC2, kC2), f(2), t);
+  t = fma2(pk(kC3, kC3), f(3), t);
+  t = fma2(pk(kC4, kC4), f(4), t);
+  return t;
+}
+
 __device__ __forceinline__ bool pml_cell(const Dims &d, int ix, int iz) {
   return !d.rbc && (ix < d.pml || ix > d.nxp - d.pml || iz < d.pml || iz > d.nzp - d.pml);
 }
