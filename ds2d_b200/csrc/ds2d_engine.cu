@@ -1863,7 +1863,8 @@ AcTileArgs ac_tile_args(ds2d_ctx *c, int set, int cur, int it) {
 }
 
 // L m on the tile kernels: one launch per step, the scattered set one step behind the background.
-int ac_L_tile(ds2d_ctx *c, int n) {
+// keep: with a PML, each launch also saves the strips of the background it reads.
+int ac_L_tile(ds2d_ctx *c, int n, bool keep) {
   const Dims &d = c->d;
   const size_t bytes = sizeof(float) * (size_t)d.slot * n, nrec = (size_t)n * d.max_ntr * d.nt;
   for (int i = 0; i < 6; i++) {
@@ -1875,7 +1876,7 @@ int ac_L_tile(ds2d_ctx *c, int n) {
   float *const e[2] = {c->ac[9], c->ac_e2};
   for (float *p : e) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
   for (int i = 0; i < 2; i++) CK(cudaMemsetAsync(c->rec[i], 0, nrec * 4, c->stream));
-  const int tx = tile_rows(c, true);
+  const int tx = tile_rows(c, true), nst = keep && !d.rbc ? 1 : 0;
   for (int l = 0; l <= d.nt; l++) {
     AcFwdTileArgs t{};
     t.n = n;
@@ -1887,19 +1888,30 @@ int ac_L_tile(ds2d_ctx *c, int n) {
     t.set[1].e_in = e[(l - 1) & 1];
     t.set[1].rec_vz = c->rec[0];
     t.set[1].rec_vx = c->rec[1];
-    launch_tile(c, "ac_tile", 0, ac_tile_k(!d.rbc, tx), tile_grid(c, tx, 2 * n), t, l > 0);
+    if (nst) t.st = StripSaveArgs{d, c->d_shots, t.set[0].vx, t.set[0].vz, c->st_a, l - 1};
+    launch_tile(c, "ac_tile", 0, ac_tile_k(!d.rbc, tx), tile_grid(c, tx, (2 + nst) * n), t, l > 0);
   }
   CK(cudaGetLastError());
   return DS2D_OK;
 }
 
+// Whether L m leaves the background as L^T r needs it: its final state in the buffers of side
+// nt mod 2 and, with a PML, its strips of every step in st_a.  An L^T that follows L on the same
+// batch within one call then starts from them instead of replaying the background, a quarter to a
+// third of L^T L: 16 shots of 2001x601, random boundary, 102.4 -> 82.9 ms; 8 of 1001x301 with
+// a PML, 67.9 -> 57.6 ms.  (The half-step kernels and the checkpointed L^T replay.)
+bool ac_keeps(const ds2d_ctx *c) {
+  if (!c->d.rbc && c->opt_ac_ckpt > 0 && c->opt_ac_ckpt < c->d.nt) return false;
+  return tile_on(c, true) || (c->d.rbc && c->opt_fused && c->ring_ok && c->ac2[0]);
+}
+
 // L m for the uploaded batch: scattered vz / vx into rec[0] / rec[1] (m = the window p_dmp).
-int ac_L_batch(ds2d_ctx *c, int n) {
+int ac_L_batch(ds2d_ctx *c, int n, bool keep) {
   const Dims &d = c->d;
   size_t bytes = sizeof(float) * (size_t)d.slot * n;
   if (!d.rbc)
     for (float *p : c->ac_split) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
-  if (tile_on(c, true)) return ac_L_tile(c, n);
+  if (tile_on(c, true)) return ac_L_tile(c, n, keep);
   if (d.rbc && c->opt_fused && c->ring_ok && c->ac2[0]) {
     // fused: per step one background launch (Born source out) and one scattered launch
     for (int i = 0; i < 10; i++)
@@ -2060,16 +2072,16 @@ int ac_LT_batch_pml_ckpt(ds2d_ctx *c, int n, int K) {
   return reduce_images(c, n, 1);
 }
 
-// L^T r on the tile kernels: forward replay of the background (with a PML each launch saves the
-// strips of the state it reads), then one launch per reverse step.
-int ac_LT_tile(ds2d_ctx *c, int n) {
+// L^T r on the tile kernels: forward replay of the background unless L left it (`kept`; with a PML
+// each launch saves the strips of the state it reads), then one launch per reverse step.
+int ac_LT_tile(ds2d_ctx *c, int n, bool kept) {
   const Dims &d = c->d;
   const size_t bytes = sizeof(float) * (size_t)d.slot * n;
   const int tx = tile_rows(c, true), nst = d.rbc ? 0 : 1;
-  for (float *p : c->ac2) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
+  for (int i = kept ? 3 : 0; i < 6; i++) CK(cudaMemsetAsync(c->ac2[i], 0, bytes, c->stream));
   for (float *p : c->ac_split2)
     if (p) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
-  for (int it = 0; it < d.nt; it++) {
+  for (int it = 0; it < d.nt && !kept; it++) {
     AcFwdTileArgs t{};
     t.n = n;
     t.nset = 1;
@@ -2090,8 +2102,10 @@ int ac_LT_tile(ds2d_ctx *c, int n) {
     yk[1][3 + i] = c->ac_split2[4 + i];
   }
   if (!d.rbc) {
-    StripSaveArgs sv{d, c->d_shots, bk[0][0], bk[0][1], c->st_a, d.nt - 1};
-    LAUNCH(k_strip_save, dim3((d.lb + 255) / 256, 2, n), 256, sv);
+    if (!kept) {
+      StripSaveArgs sv{d, c->d_shots, bk[0][0], bk[0][1], c->st_a, d.nt - 1};
+      LAUNCH(k_strip_save, dim3((d.lb + 255) / 256, 2, n), 256, sv);
+    }
     // cells outside the interior are not rebuilt: both buffers keep them as the forward pass left
     // them
     for (int i = 0; i < 3; i++)
@@ -2116,12 +2130,12 @@ int ac_LT_tile(ds2d_ctx *c, int n) {
   return reduce_images(c, n, 1);
 }
 
-int ac_LT_batch_pml(ds2d_ctx *c, int n) {
+int ac_LT_batch_pml(ds2d_ctx *c, int n, bool kept) {
   const Dims &d = c->d;
   size_t bytes = sizeof(float) * (size_t)d.slot * n;
   for (float *p : c->ac_split) CK(cudaMemsetAsync(p, 0, bytes, c->stream));
   if (c->opt_ac_ckpt > 0 && c->opt_ac_ckpt < d.nt) return ac_LT_batch_pml_ckpt(c, n, c->opt_ac_ckpt);
-  if (tile_on(c, true)) return ac_LT_tile(c, n);
+  if (tile_on(c, true)) return ac_LT_tile(c, n, kept);
   dim3 grid = cell_grid(d, n), blk(32, 8);
   for (int it = 0; it < d.nt; it++) {
     AcArgs b = ac_args(c, 0, it, 1.f);
@@ -2137,25 +2151,27 @@ int ac_LT_batch_pml(ds2d_ctx *c, int n) {
 }
 
 // L^T r for the uploaded batch (r in rec[0] / rec[1]); the windowed gradients are added into
-// the model-size image 0.
-int ac_LT_batch(ds2d_ctx *c, int n) {
+// the model-size image 0.  kept: L of this batch left the background (ac_keeps).
+int ac_LT_batch(ds2d_ctx *c, int n, bool kept) {
   const Dims &d = c->d;
   size_t bytes = sizeof(float) * (size_t)d.slot * n;
   for (int i = 0; i < 9; i++)
-    if (i < 3 || i >= 6) CK(cudaMemsetAsync(c->ac[i], 0, bytes, c->stream));
+    if ((i < 3 && !kept) || i >= 6) CK(cudaMemsetAsync(c->ac[i], 0, bytes, c->stream));
   size_t plane = (size_t)c->B * d.wnx * d.ild;
   CK(cudaMemsetAsync(c->img_slot, 0, plane * sizeof(float), c->stream));
   dim3 grid = cell_grid(d, n), blk(32, 8);
-  if (!d.rbc) return ac_LT_batch_pml(c, n);
-  if (tile_on(c, true)) return ac_LT_tile(c, n);
+  if (!d.rbc) return ac_LT_batch_pml(c, n, kept);
+  if (tile_on(c, true)) return ac_LT_tile(c, n, kept);
   const bool fused = c->opt_fused && c->ring_ok && c->ac2[0];
   if (fused) {
     // fused forward replay of the background, final state left in ac[0..2]
-    for (int i = 0; i < 3; i++) CK(cudaMemsetAsync(c->ac2[i], 0, bytes, c->stream));
     int rc, cur = 0;
-    for (int it = 0; it < d.nt; it++, cur ^= 1)
-      if ((rc = ac_ring_step(c, n, 0, cur, it, false, false))) return rc;
-    if (cur == 1)
+    if (!kept) {
+      for (int i = 0; i < 3; i++) CK(cudaMemsetAsync(c->ac2[i], 0, bytes, c->stream));
+      for (int it = 0; it < d.nt; it++, cur ^= 1)
+        if ((rc = ac_ring_step(c, n, 0, cur, it, false, false))) return rc;
+    }
+    if (d.nt & 1)
       for (int i = 0; i < 3; i++)
         CK(cudaMemcpyAsync(c->ac[i], c->ac2[i], bytes, cudaMemcpyDeviceToDevice, c->stream));
     // fused reversal: one k_ac_rev_ring launch per step; the background ping-pongs between
@@ -2235,40 +2251,49 @@ int ac_LT_batch(ds2d_ctx *c, int n) {
   return reduce_images(c, n, 1);
 }
 
+// L m (m in pp_all, data into rec[0..1]) or L^T r (r in rec[0..1], gradient added to image 0) of
+// the batch of m shots from shot f.  shared: L keeps the background for the L^T that follows on
+// the same batch in the same call, and that L^T starts from it (setup, too, is L's).
+int ac_batch(ds2d_ctx *c, const ds2d_shot *shots, int f, int m, bool adjoint, bool shared) {
+  int rc;
+  if ((rc = upload_batch(c, shots + f, m))) return rc;
+  shared = shared && ac_keeps(c);
+  if (adjoint && (rc = ensure_ckpt(c))) return rc;
+  rc = run_graph(c, graph_key(c, (adjoint ? 6 : 5) + (shared ? 2 : 0), m, f), [&]() {
+    if (adjoint && shared) return ac_LT_batch(c, m, true);
+    const int r = setup_batch(c, m, f, !adjoint);
+    return r ? r : adjoint ? ac_LT_batch(c, m, false) : ac_L_batch(c, m, shared);
+  });
+  if (rc) return rc;
+  c->last_updates += 2.0 * c->batch_cells * c->d.nt;
+  return DS2D_OK;
+}
+
 // Applies L (m_dev -> data vector [n][max_ntr][nt] x {z, x}) or L^T (data -> grad_dev) over all
-// shots in batches.  m_dev / grad_dev are model-size device arrays.
+// shots in batches.  m_dev / grad_dev are model-size device arrays.  shared: the call runs L, then
+// L^T on the same shots; it takes effect when they are one batch.
 int ac_apply(ds2d_ctx *c, const ds2d_shot *shots, int n, bool adjoint, const float *m_dev,
-             float *dz, float *dx, float *grad_dev) {
+             float *dz, float *dx, float *grad_dev, bool shared) {
   const Dims &d = c->d;
   int rc;
   size_t nall = (size_t)d.allnx * d.allnz;
   if (!adjoint) CK(cudaMemcpyAsync(c->pp_all, m_dev, nall * 4, cudaMemcpyDeviceToDevice, c->stream));
   else CK(cudaMemsetAsync(c->images, 0, nall * 4, c->stream));
   const size_t per = (size_t)d.max_ntr * d.nt;
+  shared = shared && n <= c->B;
   for (int f = 0; f < n; f += c->B) {
     const int m = std::min(c->B, n - f);
-    if ((rc = upload_batch(c, shots + f, m))) return rc;
-    if (!adjoint) {
-      rc = run_graph(c, graph_key(c, 5, m, f), [&]() {
-        const int r = setup_batch(c, m, f, true);
-        return r ? r : ac_L_batch(c, m);
-      });
-      if (rc) return rc;
-      CK(cudaMemcpyAsync(dz + f * per, c->rec[0], m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
-      CK(cudaMemcpyAsync(dx + f * per, c->rec[1], m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
-    } else {
+    if (adjoint) {
       CK(cudaMemcpyAsync(c->rec[0], dz + f * per, m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
       CK(cudaMemcpyAsync(c->rec[1], dx + f * per, m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
-      if ((rc = ensure_ckpt(c))) return rc;
-      rc = run_graph(c, graph_key(c, 6, m, f), [&]() {
-        const int r = setup_batch(c, m, f, false);
-        return r ? r : ac_LT_batch(c, m);
-      });
-      if (rc) return rc;
+    }
+    if ((rc = ac_batch(c, shots, f, m, adjoint, shared))) return rc;
+    if (!adjoint) {
+      CK(cudaMemcpyAsync(dz + f * per, c->rec[0], m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
+      CK(cudaMemcpyAsync(dx + f * per, c->rec[1], m * per * 4, cudaMemcpyDeviceToDevice, c->stream));
     }
     // upload_batch of the next batch overwrites d_shots / rmap: finish this batch first.
     CK(cudaStreamSynchronize(c->stream));
-    c->last_updates += 2.0 * c->batch_cells * d.nt;
   }
   if (adjoint) CK(cudaMemcpyAsync(grad_dev, c->images, nall * 4, cudaMemcpyDeviceToDevice, c->stream));
   return DS2D_OK;
@@ -2741,7 +2766,7 @@ int ds2d_ac_born(ds2d_ctx *c, const ds2d_shot *shots, int n, const float *m, flo
   if ((rc = work_vec(c, 0, nall, &mv)) || (rc = work_vec(c, 7, nd, &dz)) || (rc = work_vec(c, 8, nd, &dx)))
     return rc;
   CK(cudaMemcpyAsync(mv, m, nall * 4, cudaMemcpyDefault, c->stream));
-  if ((rc = ac_apply(c, shots, n, false, mv, dz, dx, nullptr))) return rc;
+  if ((rc = ac_apply(c, shots, n, false, mv, dz, dx, nullptr, false))) return rc;
   if ((rc = data_io(c, shots, n, dz, rec_vz, false)) || (rc = data_io(c, shots, n, dx, rec_vx, false)))
     return rc;
   CK(cudaStreamSynchronize(c->stream));
@@ -2765,7 +2790,7 @@ int ds2d_ac_born_adj(ds2d_ctx *c, const ds2d_shot *shots, int n, const float *re
   if ((rc = data_io(c, shots, n, dz, (float *)rec_vz, true)) ||
       (rc = data_io(c, shots, n, dx, (float *)rec_vx, true)))
     return rc;
-  if ((rc = ac_apply(c, shots, n, true, nullptr, dz, dx, gv))) return rc;
+  if ((rc = ac_apply(c, shots, n, true, nullptr, dz, dx, gv, false))) return rc;
   CK(cudaMemcpyAsync(grad, gv, nall * 4, cudaMemcpyDefault, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return check_pair_err(c);
@@ -2799,14 +2824,14 @@ int ds2d_lsrtm(ds2d_ctx *c, const ds2d_shot *shots, int n, const float *obs_vz,
   if ((rc = dot64(c, rz, rz, nd, &tz)) || (rc = dot64(c, rx, rx, nd, &tx))) return rc;
   dd = tz + tx;
   if (!(dd > 0)) return fail(c, DS2D_E_NUMERIC, "observed data are zero or not finite");
-  if ((rc = ac_apply(c, shots, n, true, nullptr, rz, rx, sv))) return rc;
+  if ((rc = ac_apply(c, shots, n, true, nullptr, rz, rx, sv, false))) return rc;
   CK(cudaMemcpyAsync(p, sv, nall * 4, cudaMemcpyDeviceToDevice, c->stream));
   double gamma;
   if ((rc = dot64(c, sv, sv, nall, &gamma))) return rc;
   const int nb = 4 * 148;
   int k = 0;
   for (; k < niter; k++) {
-    if ((rc = ac_apply(c, shots, n, false, p, qz, qx, nullptr))) return rc;
+    if ((rc = ac_apply(c, shots, n, false, p, qz, qx, nullptr, true))) return rc;
     if ((rc = dot64(c, qz, qz, nd, &tz)) || (rc = dot64(c, qx, qx, nd, &tx))) return rc;
     const double delta = tz + tx;
     if (!(delta > 0) || !std::isfinite(gamma)) return fail(c, DS2D_E_NUMERIC, "CG breakdown at %d", k);
@@ -2818,11 +2843,11 @@ int ds2d_lsrtm(ds2d_ctx *c, const ds2d_shot *shots, int n, const float *obs_vz,
     if ((rc = dot64(c, rz, rz, nd, &tz)) || (rc = dot64(c, rx, rx, nd, &tx))) return rc;
     const double rel = std::sqrt((tz + tx) / dd);
     if (resid) resid[k] = rel;
-    if (rel <= target) {
+    if (rel <= target || k + 1 == niter) {  // no direction follows the last update
       k++;
       break;
     }
-    if ((rc = ac_apply(c, shots, n, true, nullptr, rz, rx, sv))) return rc;
+    if ((rc = ac_apply(c, shots, n, true, nullptr, rz, rx, sv, true))) return rc;
     double gnew;
     if ((rc = dot64(c, sv, sv, nall, &gnew))) return rc;
     const double beta = gnew / gamma;
@@ -2843,15 +2868,17 @@ int ds2d_ac_normal(ds2d_ctx *c, const ds2d_shot *shots, int n, const float *m, f
   if ((rc = ensure_acoustic(c)) || (rc = check_shots(c, shots, n))) return rc;
   c->last_launches = 0;
   c->last_updates = 0;
-  const size_t nall = (size_t)c->d.allnx * c->d.allnz, nd = (size_t)n * c->d.max_ntr * c->d.nt;
-  float *mv, *gv, *dz, *dx;
-  if ((rc = work_vec(c, 0, nall, &mv)) || (rc = work_vec(c, 1, nall, &gv)) ||
-      (rc = work_vec(c, 7, nd, &dz)) || (rc = work_vec(c, 8, nd, &dx)))
-    return rc;
-  CK(cudaMemcpyAsync(mv, m, nall * 4, cudaMemcpyDefault, c->stream));
-  if ((rc = ac_apply(c, shots, n, false, mv, dz, dx, nullptr))) return rc;
-  if ((rc = ac_apply(c, shots, n, true, nullptr, dz, dx, gv))) return rc;
-  CK(cudaMemcpyAsync(img, gv, nall * 4, cudaMemcpyDefault, c->stream));
+  const Dims &d = c->d;
+  const size_t nall = (size_t)d.allnx * d.allnz;
+  CK(cudaMemcpyAsync(c->pp_all, m, nall * 4, cudaMemcpyDefault, c->stream));
+  CK(cudaMemsetAsync(c->images, 0, nall * 4, c->stream));
+  // batch by batch, L's records left in place as the data of L^T
+  for (int f = 0; f < n; f += c->B)
+    for (const bool adjoint : {false, true}) {
+      if ((rc = ac_batch(c, shots, f, std::min(c->B, n - f), adjoint, true))) return rc;
+      CK(cudaStreamSynchronize(c->stream));  // the next upload overwrites d_shots / rmap
+    }
+  CK(cudaMemcpyAsync(img, c->images, nall * 4, cudaMemcpyDefault, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return check_pair_err(c);
 }
@@ -2946,13 +2973,13 @@ int ds2d_lsrtm_pcg(ds2d_ctx *c, ds2d_unet *net, const ds2d_shot *shots, int n, c
   if ((rc = dot64(c, rz, rz, nd, &tz)) || (rc = dot64(c, rx, rx, nd, &tx))) return rc;
   dd = tz + tx;
   if (!(dd > 0)) return fail(c, DS2D_E_NUMERIC, "observed data are zero or not finite");
-  if ((rc = ac_apply(c, shots, n, true, nullptr, rz, rx, g))) return rc;
+  if ((rc = ac_apply(c, shots, n, true, nullptr, rz, rx, g, false))) return rc;
   const int nb = 4 * 148;
   int k = 0, nwin = 0, head = 0;  // window: nwin entries, next slot `head`
   double prev_rel = 1.0;
   for (; k < niter; k++) {
     if ((rc = precondition(c, net, g, z))) return rc;
-    if ((rc = ac_apply(c, shots, n, false, z, wz, wx, nullptr))) return rc;
+    if ((rc = ac_apply(c, shots, n, false, z, wz, wx, nullptr, true))) return rc;
     for (int i = 0; i < nwin; i++) {
       const int j = (head - 1 - i + M) % M;
       double bz, bx;
@@ -2996,7 +3023,7 @@ int ds2d_lsrtm_pcg(ds2d_ctx *c, ds2d_unet *net, const ds2d_shot *shots, int n, c
       nwin = 0;
     }
     prev_rel = rel;
-    if ((rc = ac_apply(c, shots, n, true, nullptr, rz, rx, g))) return rc;
+    if ((rc = ac_apply(c, shots, n, true, nullptr, rz, rx, g, true))) return rc;
   }
   if (iters_done) *iters_done = k;
   CK(cudaMemcpyAsync(m_out, m, nall * 4, cudaMemcpyDefault, c->stream));

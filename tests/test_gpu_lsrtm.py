@@ -390,3 +390,39 @@ def test_ac_born_pml_vs_reference_golden(cuda_device):
             floor = rel(b32[j], b64[j])
             err = rel(got[i * ntr:(i + 1) * ntr], fx[key][i])
             assert err < gate(floor), (key, i, err, f"FP32 floor {floor:.3e}")
+
+
+@pytest.mark.parametrize("boundary,tile", [("random", 0), ("random", -1), ("pml", 0), ("pml", 8)])
+@pytest.mark.parametrize("nt", [121, 122])
+def test_normal_is_born_then_adjoint(cuda_device, boundary, tile, nt):
+    """L^T L in one call starts L^T from the background that L left; two calls replay it.  The
+    replay runs the same kernels on the same numbers, so the images agree bit for bit: one batch
+    and two, an even and an odd number of steps (the state ends in either buffer), a state left by
+    another model, the checkpointed L^T (which replays), and CGLS, which meets L and L^T in turn,
+    against the same iteration made of separate calls (FP32 vectors, so 1e-5)."""
+    import torch
+    c, vp, vs, w, shots, m = acoustic_case(nt, 3)
+    dev = torch.tensor(m).cuda()
+    for cap, ckpt in ((3, 0), (2, 0), (3, 40)):
+        with Elastic2D(c["allnx"], c["allnz"], c["nx"], c["pml"], nt, c["dx"], c["dz"], c["dt"],
+                       boundary=boundary, seed=21, max_shots=cap, max_ntr=c["nx"]) as e:
+            e.set_option("tile", tile)
+            e.set_option("ac_ckpt", ckpt)
+            e.set_wavelet(w)
+            for scale in (1.0, 1.1, 1.0):
+                e.set_models(vp * np.float32(scale), vs)
+                img = torch.full(m.shape, 7.0, device="cuda")
+                e.ac_normal_device(shots, dev.data_ptr(), img.data_ptr())
+                d = e.ac_born(shots, m)
+                assert np.array_equal(img.cpu().numpy(), e.ac_born_adj(shots, *d))
+            hist = e.lsrtm(shots, *d, 3)[1]
+            r, x = [v.astype(np.float64) for v in d], np.zeros(m.shape)
+            s = p = e.ac_born_adj(shots, *d).astype(np.float64)
+            for k in range(3):
+                q = e.ac_born(shots, p.astype(np.float32))
+                a = (s * s).sum() / sum((v.astype(np.float64) ** 2).sum() for v in q)
+                r = [u - a * v for u, v in zip(r, q)]
+                n2 = sum((u ** 2).sum() for u in r) / sum((v.astype(np.float64) ** 2).sum() for v in d)
+                assert abs(hist[k] - n2 ** 0.5) <= 1e-5 * n2 ** 0.5, (cap, ckpt, k)
+                sn = e.ac_born_adj(shots, *[u.astype(np.float32) for u in r]).astype(np.float64)
+                p, s = sn + (sn * sn).sum() / (s * s).sum() * p, sn
