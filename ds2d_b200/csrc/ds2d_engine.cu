@@ -23,6 +23,7 @@
 #include "ds2d_filter.cuh"
 #include "ds2d_fused.cuh"
 #include "ds2d_pair.cuh"
+#include "ds2d_acduo.cuh"
 #include "ds2d_step.cuh"
 #include "ds2d_tblock.cuh"
 #include "ds2d_bwdws.cuh"
@@ -303,6 +304,8 @@ struct ds2d_ctx {
   // resident CTAs per SM: forward 256 / 64, backward 256 / 160 / 64, split parts 1 / 2
   int occ_pair[7] = {0, 0, 0, 0, 0, 0, 0};
   int occ_ac_pair[3] = {0, 0, 0};  // k_ac_pair, 256 / 192 / 128 threads
+  int opt_ac_duo = 1;              // option "ac_duo": L's two sets in one launch (k_ac_duo)
+  int occ_ac_duo[3] = {0, 0, 0};   // k_ac_duo, 128 / 192 / 256 threads
   int occ_ac_rev[2] = {0, 0};      // k_ac_rev_pair, 192 / 128 threads
   std::vector<int> h_nxp;    // padded window rows of each slot of the current batch
   int opt_pcg_switch = 970;  // ds2d_lsrtm_pcg: per-mille residual ratio that ends the network phase
@@ -638,6 +641,8 @@ constexpr double kBytesBwdScat = 100;
 // Fused acoustic reverse step (k_ac_rev_ring): adjoint state and background, 3 fields each read
 // and written, b and lam read, the gradient updated on the interior.
 constexpr double kBytesAcRev = 64;
+// k_ac_duo: two sets of 3 fields read and written, lam, m, the Born source read and written.
+constexpr double kBytesAcDuo = 64;
 // Fused backward RTM step per padded cell: source and adjoint fields r/w (2 x 40), b, lam, mu
 // (12), imaging weights (8) and three image accumulators r/w (24).
 constexpr double kBytesBwdFused = 124;
@@ -930,6 +935,30 @@ int ac_pair_cta(const ds2d_ctx *c) {
 bool ac_pair_on(const ds2d_ctx *c) {
   return c->opt_ac_pair && pair_ok(c) && c->occ_ac_pair[ac_pair_idx(ac_pair_cta(c))] > 0;
 }
+// Both sets of L in one launch (k_ac_duo): 128 / 192 / 256 threads at 768 per SM (80 registers);
+// the width with the fewest threads per grid row, the wider on a tie.  Measured against a launch
+// per set (L^T L, random boundary): 21.9 M cells 74.5 / 82.8 ms, 8.9 M 21.2 / 22.9, 4.5 M 12.4 /
+// 15.2, 2.6 M 11.0 / 13.3, so it is taken wherever the column pairs were.
+using AcDuoFn = void (*)(AcDuoArgs);
+AcDuoFn ac_duo_fn(int i) {
+  return i == 0 ? k_ac_duo<128, 6> : i == 1 ? k_ac_duo<192, 4> : k_ac_duo<256, 3>;
+}
+struct DuoShape {
+  int i, ns, tz, xr;  // width index, z-strips, columns and rows per CTA
+};
+bool ac_duo_shape(const ds2d_ctx *c, DuoShape *s) {
+  if (!c->opt_ac_duo || !ac_pair_on(c)) return false;
+  int best = 1 << 30;
+  for (int i = 0; i < 3; i++) {
+    int ns, tz;
+    if (c->occ_ac_duo[i] <= 0 || !tb_split(c->d, kBulkCtas[i], 1, &ns, &tz)) continue;
+    if (ns * kBulkCtas[i] <= best) {
+      best = ns * kBulkCtas[i];
+      *s = DuoShape{i, ns, tz, pair_xr(c, ns, c->occ_ac_duo[i])};
+    }
+  }
+  return best < 1 << 30;
+}
 // Reverse step (k_ac_rev_pair): 192 / 128 threads at 2 / 3 CTAs per SM, strips with a
 // 12-column halo (each CTA computes tz <= 2 kT - 24 columns); the width with the fewest threads
 // per grid row, the wider on a tie.
@@ -1039,8 +1068,9 @@ bool tile_ok(const ds2d_ctx *c) {
 //    steps).  The marching kernels pay the PML's predicates row by row: always the tiles.
 //  - random boundary, elastic: 0.66 M 3.2 / 8.1, 2.22 M 7.2 / 7.9, 8.9 M 24.6 / 17.5: the
 //    bulk-copy marching kernels win once they fill the chip, between 2.2 and 8.9 M cells.
-//  - random boundary, acoustic: 0.66 M 2.9 / 14.2, 2.63 M 10.6 / 16.3, 21.9 M 25.8 / 21.3: 6 M.
-constexpr double kTileElastic = 3e6, kTileAcoustic = 6e6;
+//  - random boundary, acoustic (L^T L, k_ac_duo and k_ac_rev_pair / tiles of 32 rows): 2.6 M 11.0
+//    / 8.5, 2.8 M 10.5 / 8.7, 4.5 M 12.4 / 13.6, 8.9 M 21.2 / 26.5: 3.5 M.
+constexpr double kTileElastic = 3e6, kTileAcoustic = 3.5e6;
 bool tile_on(const ds2d_ctx *c, bool acoustic) {
   if (!tile_ok(c) || c->opt_tile == 0) return false;
   if (c->opt_tile > 0) return true;
@@ -1808,8 +1838,9 @@ AcArgs ac_args(ds2d_ctx *c, int set, int it, float dir) {
 }
 
 // One fused acoustic forward step (k_ac_ring) of the buffer pair `set` (0 background, 1
-// scattered) from ping-pong side `cur` to 1 - cur.
-int ac_ring_step(ds2d_ctx *c, int n, int set, int cur, int it, bool born_out, bool record) {
+// scattered) from ping-pong side `cur` to 1 - cur; e: the Born source, written (0, or null) or
+// read (1).
+int ac_ring_step(ds2d_ctx *c, int n, int set, int cur, int it, float *e) {
   const Dims &d = c->d;
   const int nstrips = (d.nzp + kFTZ - 1) / kFTZ;
   const int tz = (d.nzp + nstrips - 1) / nstrips;
@@ -1824,10 +1855,10 @@ int ac_ring_step(ds2d_ctx *c, int n, int set, int cur, int it, bool born_out, bo
   a.b = c->par.b; a.lam = c->par.lam; a.m = c->par.dmp;
   a.wavelet = c->wavelet; a.it = it; a.tz = tz; a.xr = xr; a.rmap = c->d_rmap;
   if (set == 0) {
-    a.e_out = born_out ? c->ac[9] : nullptr;
+    a.e_out = e;
   } else {
-    a.e_in = c->ac[9];
-    if (record) { a.rec_vz = c->rec[0]; a.rec_vx = c->rec[1]; }
+    a.e_in = e;
+    a.rec_vz = c->rec[0]; a.rec_vx = c->rec[1];
   }
   if (ac_pair_on(c)) {
     const int pc = ac_pair_cta(c);
@@ -1921,9 +1952,35 @@ int ac_L_batch(ds2d_ctx *c, int n, bool keep) {
     CK(cudaMemsetAsync(c->rec[0], 0, nrec * 4, c->stream));
     CK(cudaMemsetAsync(c->rec[1], 0, nrec * 4, c->stream));
     int rc;
+    DuoShape sh;
+    if (ac_duo_shape(c, &sh)) {  // background step it with scattered step it - 1
+      float *const e[2] = {c->ac[9], c->ac[6]};  // (ac[6]: L^T's)
+      CK(cudaMemsetAsync(e[1], 0, bytes, c->stream));
+      if ((rc = ac_ring_step(c, n, 0, 0, 0, e[0]))) return rc;
+      const int cta = kBulkCtas[sh.i];
+      for (int it = 1; it < d.nt; it++) {
+        float *const *side[2] = {c->ac, c->ac2};
+        AcDuoArgs a{};
+        a.d = d; a.shots = c->d_shots;
+        for (int k = 0; k < 2; k++) {
+          float *const *in = side[(it - k) & 1] + 3 * k, *const *out = side[(it - k + 1) & 1] + 3 * k;
+          a.vx[k] = in[0]; a.vz[k] = in[1]; a.s[k] = in[2];
+          a.vx_n[k] = out[0]; a.vz_n[k] = out[1]; a.s_n[k] = out[2];
+        }
+        a.b = c->par.b; a.lam = c->par.lam; a.m = c->par.dmp; a.bconst = c->par.bconst;
+        a.e_in = e[(it - 1) & 1]; a.e_out = e[it & 1];
+        a.wavelet = c->wavelet; a.it = it; a.tz = sh.tz; a.xr = sh.xr; a.rmap = c->d_rmap;
+        a.rec_vz = c->rec[0]; a.rec_vx = c->rec[1]; a.err = c->d_err;
+        LAUNCHS("ac_duo", kBytesAcDuo * CELLS(n), ac_duo_fn(sh.i),
+                dim3(sh.ns, (d.nxp + sh.xr - 1) / sh.xr, n), cta, ac_duo_smem(cta), a);
+      }
+      if ((rc = ac_ring_step(c, n, 1, (d.nt - 1) & 1, d.nt - 1, e[(d.nt - 1) & 1]))) return rc;
+      CK(cudaGetLastError());
+      return DS2D_OK;
+    }
     for (int it = 0, cur = 0; it < d.nt; it++, cur ^= 1) {
-      if ((rc = ac_ring_step(c, n, 0, cur, it, true, false))) return rc;
-      if ((rc = ac_ring_step(c, n, 1, cur, it, false, true))) return rc;
+      if ((rc = ac_ring_step(c, n, 0, cur, it, c->ac[9]))) return rc;
+      if ((rc = ac_ring_step(c, n, 1, cur, it, c->ac[9]))) return rc;
     }
     CK(cudaGetLastError());
     return DS2D_OK;
@@ -2169,7 +2226,7 @@ int ac_LT_batch(ds2d_ctx *c, int n, bool kept) {
     if (!kept) {
       for (int i = 0; i < 3; i++) CK(cudaMemsetAsync(c->ac2[i], 0, bytes, c->stream));
       for (int it = 0; it < d.nt; it++, cur ^= 1)
-        if ((rc = ac_ring_step(c, n, 0, cur, it, false, false))) return rc;
+        if ((rc = ac_ring_step(c, n, 0, cur, it, nullptr))) return rc;
     }
     if (d.nt & 1)
       for (int i = 0; i < 3; i++)
@@ -2475,6 +2532,14 @@ int ds2d_create(const ds2d_grid *grid, const ds2d_opts *opts, ds2d_ctx **out) {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->occ_bulk[bulk_idx(cta, one)],
                                                           bulk_fn(cta, one), cta,
                                                           bwd_bulk_smem(cta));
+    }
+    for (int i = 0; i < 3 && e == cudaSuccess; i++) {
+      const int cta = kBulkCtas[i];
+      e = cudaFuncSetAttribute(ac_duo_fn(i), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)ac_duo_smem(cta));
+      if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->occ_ac_duo[i], ac_duo_fn(i), cta,
+                                                          ac_duo_smem(cta));
     }
     for (int i = 0; i < 3 && e == cudaSuccess; i++) {
       const int kt = kWsRoles[i];
@@ -3091,6 +3156,9 @@ int ds2d_set_option(ds2d_ctx *c, const char *key, long long value) {
   } else if (k == "ac_pair") {
     if (value != 0 && value != 1) return fail(c, DS2D_E_ARG, "ac_pair must be 0 or 1");
     c->opt_ac_pair = (int)value;
+  } else if (k == "ac_duo") {
+    if (value != 0 && value != 1) return fail(c, DS2D_E_ARG, "ac_duo must be 0 or 1");
+    c->opt_ac_duo = (int)value;
   } else if (k == "ac_pair_cta") {
     if (value != 0 && value != 128 && value != 192 && value != 256)
       return fail(c, DS2D_E_ARG, "ac_pair_cta must be 0 (automatic), 128, 192 or 256");

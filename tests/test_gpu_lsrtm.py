@@ -3,6 +3,7 @@ import numpy as np
 import pytest
 
 from ds2d_b200 import Elastic2D, synth
+from ds2d_b200.api import ShotGeom
 from oracle import pyoracle as po
 from tests.helpers import gate, rel
 
@@ -426,3 +427,35 @@ def test_normal_is_born_then_adjoint(cuda_device, boundary, tile, nt):
                 assert abs(hist[k] - n2 ** 0.5) <= 1e-5 * n2 ** 0.5, (cap, ckpt, k)
                 sn = e.ac_born_adj(shots, *[u.astype(np.float32) for u in r]).astype(np.float64)
                 p, s = sn + (sn * sn).sum() / (s * s).sum() * p, sn
+
+
+@pytest.mark.parametrize("allnz,nt", [(36, 41), (100, 2), (101, 1), (150, 40), (231, 41), (430, 40),
+                                      (500, 9)])
+@pytest.mark.parametrize("rho", [False, True])
+def test_ac_duo_matches_two_launches(cuda_device, allnz, nt, rho):
+    """L with both sets in one launch (k_ac_duo) against one launch per set: bit for bit, on one
+    z-strip of 128, 192 and 256 threads and on two and three strips, narrow and full windows, with
+    a uniform density (a constant) and an array, for one step, an odd and an even number; the
+    source and the receivers lie at a strip's edge for the deepest grids."""
+    pml, allnx, nx = 12, 90, 70
+    rng = np.random.default_rng(allnz)
+    vp = rng.uniform(1800, 4500, (allnx, allnz)).astype(np.float32)
+    den = rng.uniform(1800, 2400, vp.shape).astype(np.float32) if rho else None
+    m = rng.normal(0, 0.05, vp.shape).astype(np.float32)
+    w = synth.ricker(nt, 15.0, 0.0008) + np.float32(1)
+    shots = []
+    for k, width in enumerate((nx, 20, 47)):
+        igz = pml + (0 if allnz < 300 else allnz // 2 - 4 + k)
+        shots.append(ShotGeom(win_left=5 * k, isx=pml + 4 + k, isz=igz + 1, igz=igz,
+                                igx=np.arange(pml, pml + width, 1 + k, dtype=np.int32), nx=width))
+    outs = []
+    for duo in (0, 1):
+        with Elastic2D(allnx, allnz, nx, pml, nt, 10.0, 10.0, 0.0008, boundary="random", seed=3,
+                       max_shots=3, max_ntr=nx) as e:
+            e.set_option("ac_duo", duo)
+            e.set_models(vp, 0 * vp, den)
+            e.set_wavelet(w)
+            d = [np.array(v) for v in e.ac_born(shots, m)]
+            outs.append([*d, *e.ac_born(shots, m), e.ac_born_adj(shots, *d)])
+    assert all(np.abs(v).max() > 0 for v in outs[0]) or nt < 10
+    assert all(np.array_equal(a, b) for a, b in zip(*outs))
