@@ -20,7 +20,7 @@
 // first, then one FMA), so the records agree bit for bit: scattered fields carry a one-ulp change
 // of the background to 1e-4.
 #pragma once
-#include "ds2d_bwdbulk.cuh"
+#include "ds2d_pair.cuh"
 
 namespace ds2d {
 
@@ -94,8 +94,10 @@ __global__ void __launch_bounds__(kT, kMinB) k_ac_duo(AcDuoArgs a) {
   }
   __syncthreads();
   const int rs0 = x0 - 8;
-  for (int j = 0; j < kD - 1; j++)
-    issue_slot_col<kT>(fd, ring + (size_t)j * NF * kT, my_f, &bars[j], rs0 + j, ld, c0, lane);
+  RowCopies rc;
+  rc.init<kT>(fd, ring, my_f, rs0, ld, c0);
+  const unsigned bar0 = smem_u32(bars);
+  for (int j = 0; j < kD - 1; j++) rc.issue(j * NF * kT * 4, bar0 + 8 * j, ld, lane);
 
   pair_t w_S[8], w_vx[9], w_vz[5];
 #pragma unroll
@@ -127,8 +129,7 @@ __global__ void __launch_bounds__(kT, kMinB) k_ac_duo(AcDuoArgs a) {
     }
     {  // every thread is done with the previous slot
       const int ps = cur.slot == 0 ? kD - 1 : cur.slot - 1;
-      issue_slot_col<kT>(fd, ring + (size_t)ps * NF * kT, my_f, &bars[ps], r + kD - 1, ld, c0,
-                         lane);
+      rc.issue(ps * NF * kT * 4, bar0 + 8 * ps, ld, lane);
     }
     // ---- stage V: velocities of row rv = r - 4 ----------------------------------------------
     const int rv = r - 4;

@@ -28,30 +28,16 @@ namespace ds2d {
 constexpr int kBulkRing = 4;
 // bvx bvz avx avz | btxx btzz btxz atxx atzz atxz lam mu, images pp ps | b, illumination.  The
 // imaging weights are made from lam and mu (-2 rho vp^2 = -2 (lam + 2 mu), -2 rho vs^2 = -2 mu),
-// and no row of a uniform density's b is copied: 112 bytes per cell instead of 124
-// (RTM of 60 shots of 1201x401, 250 steps: 371.2 -> 366.8 ms; the issue slots bound it).
+// and no row of a uniform density's b is copied: 112 bytes per cell instead of 124.
+//
+// What bounds it: its issue slots and fixed latencies (16 warps per SM at 128 registers; 60 % of
+// the slots used, DRAM 47 %).  The source and the adjoint field take the same derivatives, so one
+// 64-bit window entry, z-tap and packed stencil serves both.  RTM of 60 shots of 1201x401, 250
+// steps, forward and backward: 371 ms with scalar fields and all 18 rows, 367 with 15 rows, 357
+// packed, 349 with RowCopies.
 constexpr int kBwdBulkFields = 16;
 __host__ __device__ constexpr size_t bwd_bulk_smem(int kT) {
   return sizeof(float) * (size_t)kBulkRing * kBwdBulkFields * kT + 8 * kBulkRing;
-}
-
-// Copies of one ring slot for one-column CTAs, by one warp: its lane owning ring field f (row
-// q - lag of its array if that row lies in [lo, hi)) copies it; the CTA's columns
-// [c0, c0 + kT) map to ring floats 0 .. kT, clipped to [0, ld).  Lane 0 arrives on the slot's
-// barrier with the bytes of the warp's copies before any is issued.
-template <int kT>
-__device__ __forceinline__ void issue_slot_col(const RingField &fd, float *slot_base, int f,
-                                               unsigned long long *bar, int q, int ld, int c0,
-                                               int lane) {
-  const int glo = max(0, c0), ghi = min(ld, c0 + kT);
-  const unsigned bytes = (unsigned)(ghi - glo) * 4u;
-  const int row = q - fd.lag;
-  const bool mine = fd.src != nullptr && row >= fd.lo && row < fd.hi;
-  const unsigned n = __popc(__ballot_sync(0xffffffffu, mine));
-  if (lane == 0) mbar_arrive_tx(bar, n * bytes);
-  __syncwarp();
-  if (mine)
-    bulk_g2s(slot_base + f * kT + (glo - c0), fd.src + (long long)row * ld + glo, bytes, bar);
 }
 
 template <int kT, int kMinB, bool kOne>
@@ -128,8 +114,10 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
   }
   __syncthreads();
   const int rs0 = x0 - 8;
-  for (int j = 0; j < kD - 1; j++)
-    issue_slot_col<kT>(fd, ring + (size_t)j * NF * kT, my_f, &bars[j], rs0 + j, ld, c0, lane);
+  RowCopies rc;
+  rc.init<kT>(fd, ring, my_f, rs0, ld, c0);
+  const unsigned bar0 = smem_u32(bars);
+  for (int j = 0; j < kD - 1; j++) rc.issue(j * NF * kT * 4, bar0 + 8 * j, ld, lane);
 
   // windows of (source field, adjoint field): the two fields' derivatives are the same operators.
   // Adjoint-velocity operands as k_bwd_ring: PL = (l+2m) atxx + l atzz, M = mu atxz,
@@ -201,8 +189,7 @@ __global__ void __launch_bounds__(kT, kMinB) k_bwd_bulk(BwdFusedArgs a) {
     // every thread is done with the previous slot: refill it kD - 1 steps ahead
     {
       const int ps = cur.slot == 0 ? kD - 1 : cur.slot - 1;
-      issue_slot_col<kT>(fd, ring + (size_t)ps * NF * kT, my_f, &bars[ps], r + kD - 1, ld, c0,
-                         lane);
+      rc.issue(ps * NF * kT * 4, bar0 + 8 * ps, ld, lane);
     }
     // ---- stage 1: stresses of row r1 = r - 4 -----------------------------------------------
     float btxx = 0.f, btzz = 0.f, btxz = 0.f, PL = 0.f, M = 0.f, PzLx = 0.f;
