@@ -320,6 +320,7 @@ struct ds2d_ctx {
   float *ac2[6] = {};        // second (ping-pong) buffers of bvx bvz bs | dvx dvz ds (fused steps)
   float *ac_split2[6] = {};  // tile steps: second buffers of the split stress
   float *ac_e2 = nullptr;    // tile steps: second Born source (the sets run one step apart)
+  bool tile_nomem = false;   // no memory for the buffers that only the tile steps need
   double *dot_part = nullptr, *dot_out = nullptr;  // FP64 inner-product scratch
   // Work vectors of the LSRTM solver (model- and data-space), grown on demand.
   struct Vec {
@@ -1072,7 +1073,7 @@ bool tile_ok(const ds2d_ctx *c) {
 //    / 8.5, 2.8 M 10.5 / 8.7, 4.5 M 12.4 / 13.6, 8.9 M 21.2 / 26.5: 3.5 M.
 constexpr double kTileElastic = 3e6, kTileAcoustic = 3.5e6;
 bool tile_on(const ds2d_ctx *c, bool acoustic) {
-  if (!tile_ok(c) || c->opt_tile == 0) return false;
+  if (!tile_ok(c) || c->opt_tile == 0 || c->tile_nomem) return false;
   if (c->opt_tile > 0) return true;
   if (c->shape_set) return false;
   return !c->d.rbc || (double)c->B * c->d.slot <= (acoustic ? kTileAcoustic : kTileElastic);
@@ -1756,6 +1757,24 @@ int elsrtm_body(ds2d_ctx *c, int n, int shot_base, int iter) {
   return reduce_images(c, n, 7);
 }
 
+// Gives back the buffers that only the tile steps need and keeps the context on the other kernels
+// (ELSRTM and the acoustic operators then run in the memory that they need there).  False when the
+// context holds none.
+bool drop_tile_buffers(ds2d_ctx *c) {
+  bool any = false;
+  auto drop = [&](float *&p) {
+    any = any || p;
+    release(c, p);
+    p = nullptr;
+  };
+  for (auto &o : c->ov_t)
+    for (float *&p : o) drop(p);
+  for (float *&p : c->ac_split2) drop(p);
+  drop(c->ac_e2);
+  c->tile_nomem = c->tile_nomem || any;
+  return any;
+}
+
 int elsrtm_batch(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base, int iter,
                  double *mis_host) {
   const Dims &d = c->d;
@@ -1768,10 +1787,16 @@ int elsrtm_batch(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base, int 
     for (float *&p : c->ov_s2)
       if (!p && (rc = alloc_slots(c, &p))) return rc;
   }
-  if (tile_on(c, false))
+  if (tile_on(c, false)) {
+    rc = DS2D_OK;
     for (auto &o : c->ov_t)
       for (float *&p : o)
-        if (!p && (rc = alloc_slots(c, &p))) return rc;
+        if (!rc && !p) rc = alloc_slots(c, &p);
+    if (rc) {
+      drop_tile_buffers(c);
+      c->tile_nomem = true;
+    }
+  }
   rc = run_graph(c, graph_key(c, iter == 0 ? 3 : 4, n, shot_base),
                  [&]() { return elsrtm_body(c, n, shot_base, iter); });
   if (rc) return rc;
@@ -1809,11 +1834,6 @@ int ensure_acoustic(ds2d_ctx *c) {
   if (c->opt_fused && c->ring_ok)
     for (float *&p : c->ac2)
       if (!p && (rc = alloc_slots(c, &p))) return rc;
-  if (tile_on(c, true)) {
-    if (!c->ac_e2 && (rc = alloc_slots(c, &c->ac_e2))) return rc;
-    for (float *&p : c->ac_split2)
-      if (!c->d.rbc && !p && (rc = alloc_slots(c, &p))) return rc;
-  }
   if (!c->img_slot) {  // per-shot gradient planes (same 7-plane size as the RTM images)
     size_t n = (size_t)7 * c->B * c->d.wnx * c->d.ild;
     if ((rc = alloc(c, (void **)&c->img_slot, n * sizeof(float)))) return rc;
@@ -1821,6 +1841,16 @@ int ensure_acoustic(ds2d_ctx *c) {
   if (!c->dot_part) {
     if ((rc = alloc(c, (void **)&c->dot_part, sizeof(double) * kDotBlocks))) return rc;
     if ((rc = alloc(c, (void **)&c->dot_out, sizeof(double)))) return rc;
+  }
+  if (tile_on(c, true)) {  // last: what the tile steps need on top
+    rc = DS2D_OK;
+    if (!c->ac_e2) rc = alloc_slots(c, &c->ac_e2);
+    for (float *&p : c->ac_split2)
+      if (!rc && !c->d.rbc && !p) rc = alloc_slots(c, &p);
+    if (rc) {
+      drop_tile_buffers(c);
+      c->tile_nomem = true;
+    }
   }
   return DS2D_OK;
 }
@@ -2364,6 +2394,10 @@ int work_vec(ds2d_ctx *c, int i, size_t n, float **out) {
     v.p = nullptr;
     v.n = 0;
     cudaError_t e = cudaMalloc(&v.p, n * sizeof(float));
+    if (e != cudaSuccess && drop_tile_buffers(c)) {
+      cudaGetLastError();
+      e = cudaMalloc(&v.p, n * sizeof(float));
+    }
     if (e != cudaSuccess) {
       cudaGetLastError();
       v.p = nullptr;
