@@ -1049,15 +1049,18 @@ __global__ void __launch_bounds__(128) k_conv3x3_wgrad_tma(WgradArgs a,
 }
 
 // Bias gradients db[co] += sum_p dz[p][co] (dz [P][cout]) of all layers in one launch (grid.y = layer:
-// their output gradients all stay in memory): each thread sums one 8-channel group over a strided
-// set of pixels; lanes of a warp that hold the same group add up by shuffles, then warps in shared
+// their output gradients all stay in memory; up to `blocks` CTAs each, so that a thread's chain of
+// FP32 sums stays short): each thread sums one 8-channel group over a strided set of pixels; lanes of
+// a warp that hold the same group add up by shuffles, then warps in shared
 // memory and CTAs in global memory.
 struct BiasLayer {
   const bf16 *dz;
   float *db;
   long long npx;
   int cout;
+  unsigned blocks;
 };
+constexpr unsigned kBiasBlocks = 148 * 4;
 struct BiasArgs {
   BiasLayer l[kConvLayers];
 };
@@ -1065,13 +1068,14 @@ __global__ void __launch_bounds__(256) k_bias_grad(const __grid_constant__ BiasA
   __shared__ float s_db[512];  // cout <= 512 (base channels <= 64)
   const BiasLayer &L = a.l[blockIdx.y];
   const int cout = L.cout;
+  if (blockIdx.x >= L.blocks) return;  // whole CTA
   for (int i = threadIdx.x; i < cout; i += 256) s_db[i] = 0.f;
   __syncthreads();
   const int g = cout / 8, per = 256 / g;  // threads per channel group; g is a power of two, 4 .. 64
   const int cg = threadIdx.x % g, lp = threadIdx.x / g;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
-  for (long long p = (long long)blockIdx.x * per + lp; p < L.npx; p += (long long)gridDim.x * per) {
+  for (long long p = (long long)blockIdx.x * per + lp; p < L.npx; p += (long long)L.blocks * per) {
     const uint4 v = *reinterpret_cast<const uint4 *>(L.dz + p * cout + cg * 8);
     const uint32_t wv[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -1579,11 +1583,12 @@ int wgrad(ds2d_unet *u, const ds2d_unet::Layer &L, const bf16 *dz, int zcs, cons
       return unet_fail(u, DS2D_E_CUDA, "wgrad: cuTensorMapEncodeTiled failed");
     const long long tchunks = (long long)n * h * ((wd + kWgP - 1) / kWgP);
     const long long ttiles = (long long)((L.cout + kWgM - 1) / kWgM) * (L.cin_pad / kn) * 3;
-    // Splits of the pixel range: as many CTAs as are resident at once (TMEM and shared memory hold
-    // one per SM with 96 or 128 input channels, two below).  More only add epilogues, each of
-    // which adds its whole 128 x 3 kN tile to the gradient in L2.
-    const long long resident = 148 * (kn >= 96 ? 1 : 2);
-    long long ts = resident / ttiles;
+    // Splits of the pixel range: four CTAs per SM, more than are resident at once, for the sake of
+    // the sums.  The tensor cores truncate as they add to the FP32 accumulator, so a sum's error
+    // grows with the MMAs it chains; the parts are added in L2 with rounding.  8 x 128x256 pixels,
+    // same-sign terms: 84 MMAs a chain (this count) 8e-7 relative, one resident wave (168 to 336)
+    // 5e-6 to 1.7e-5.
+    long long ts = (4 * 148 + ttiles - 1) / ttiles;
     ts = ts > tchunks ? tchunks : (ts < 1 ? 1 : ts);
     a.chunks_per_cta = (int)((tchunks + ts - 1) / ts);
     ts = (tchunks + a.chunks_per_cta - 1) / a.chunks_per_cta;
@@ -1754,7 +1759,7 @@ int backward(ds2d_unet *u, int n, int h, int w) {
   UCK(cudaMemsetAsync(u->grads, 0, sizeof(float) * u->nparam, u->stream));
   const auto &Lo = u->layers.back();
   {
-    const unsigned ob = nblk(npx) < 148u * 3 ? nblk(npx) : 148u * 3;  // grid-stride over pixels
+    const unsigned ob = nblk(npx) < 148u * 8 ? nblk(npx) : 148u * 8;  // grid-stride over pixels
     if (c[0] == 32)
       k_out_bwd<32><<<ob, 256, 0, u->stream>>>(u->act[U::D1B].p, u->dy, u->params + Lo.w_off,
                                                u->grad[U::D1B].p, u->grads + Lo.w_off,
@@ -1832,9 +1837,11 @@ int backward(ds2d_unet *u, int n, int h, int w) {
     BiasArgs b{};
     for (int i = 0; i < kConvLayers; i++) {
       const auto &L = u->layers[i];
-      b.l[i] = BiasLayer{u->grad[slot[i]].p, u->grads + L.b_off, npx >> (2 * level[i]), L.cout};
+      const long long px = npx >> (2 * level[i]);
+      b.l[i] = BiasLayer{u->grad[slot[i]].p, u->grads + L.b_off, px, L.cout,
+                         std::min(nblk(px * (L.cout / 8)), kBiasBlocks)};
     }
-    k_bias_grad<<<dim3(148, kConvLayers), 256, 0, u->stream>>>(b);
+    k_bias_grad<<<dim3(kBiasBlocks, kConvLayers), 256, 0, u->stream>>>(b);
   }
   UCK(cudaGetLastError());
   return DS2D_OK;

@@ -268,3 +268,48 @@ def test_unet_tiles_equal_staged(cuda_device, base, n, h, w):
     for k in g0:
         ref = np.linalg.norm(g1[k].astype(np.float64))
         assert np.linalg.norm(g0[k].astype(np.float64) - g1[k]) <= 1e-5 * ref, k
+
+
+@pytest.mark.parametrize("n,h,w", [(8, 128, 256), (2, 128, 64)])
+def test_unet_weight_gradient_sums(cuda_device, n, h, w):
+    """The last decoder level's weight gradients (96 -> 32 and 32 -> 32 channels, the longest sums of
+    a training step) where every BF16 operand is known exactly, against FP64: zero weights make
+    the activations the biases, an identity carries the output gradient -2 t / pixels (+ or - 1 per
+    channel) one layer further down, and equal biases in pairs make the output exactly 0.
+
+    The tensor cores truncate each addition to the FP32 accumulator: of same-sign terms it loses
+    2^-24 of the sum in the mean (half an ulp), and at this size a CTA may chain 84 of them (21
+    chunks of four).  The parts are added with rounding, which is smaller."""
+    import torch
+    from ds2d_b200.unet import UNet, layer_shapes, unflatten
+    rng = np.random.default_rng(3)
+
+    def bf16(a):
+        return torch.from_numpy(a.astype(np.float32)).bfloat16().float().numpy()
+
+    bias, vec = {}, []
+    for name, ws, bs in layer_shapes(32):
+        wgt, b = np.zeros(ws, np.float32), bf16(rng.uniform(0.5, 2.0, bs))
+        if name == "d1a":
+            b = np.repeat(b[::2], 2)
+        elif name == "d1b":
+            wgt[1, 1], b = np.eye(32), 0 * b
+        elif name == "out":
+            wgt.reshape(-1)[:], b = np.tile([1.0, -1.0], 16), 0 * b
+        bias[name] = b.astype(np.float64)
+        vec += [wgt.ravel(), b.ravel()]
+    t = bf16(rng.uniform(1.0, 2.0, (n, h, w)))
+    dy = -2.0 * t.astype(np.float64) / (n * h * w)
+    taps = np.array([[dy[:, max(0, 1 - ky):h + 1 - ky, max(0, 1 - kx):w + 1 - kx].sum()
+                      for kx in range(3)] for ky in range(3)])
+    sign = np.tile([1.0, -1.0], 16)
+    with UNet(max_n=n, max_h=h, max_w=w) as net:
+        net.set_params(np.concatenate(vec).astype(np.float32))
+        x, dt = torch.zeros((n, h, w), device="cuda"), torch.from_numpy(t).cuda()
+        _, g = net.loss_grad(x.data_ptr(), dt.data_ptr(), n, h, w, want_grads=True)
+    g = unflatten(g)
+    inputs = {"d1b": bias["d1a"], "d1a": np.concatenate([bias["d2b"], bias["e1b"]])}
+    for name, a in inputs.items():
+        want = taps[:, :, None, None] * sign[:, None] * a
+        assert rel(g[name + ".w"], want) < 84 * 2.0 ** -24, (name, rel(g[name + ".w"], want))
+    assert rel(g["d1b.b"], sign * dy.sum()) < 84 * 2.0 ** -24
