@@ -3540,21 +3540,23 @@ int bandpass_fft(int nx, int nz, int z1, int z2, float *const imgs[2], cudaStrea
   float *filt = reinterpret_cast<float *>(next);
   unsigned *fmax = reinterpret_cast<unsigned *>(filt + ncell);
   a.nx = nx; a.nz = nz; a.filt = filt; a.fmax = fmax;
-  const size_t sm[2] = {fft_smem(logm[0]), fft_smem(logm[1])}, most = std::max(sm[0], sm[1]);
-  if ((e = cudaFuncSetAttribute(k_fft_spec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most)) ||
-      (e = cudaFuncSetAttribute(k_fft_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most)) ||
-      (e = cudaFuncSetAttribute(k_fft_x, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most)) ||
-      (e = cudaFuncSetAttribute(k_fft_z_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most)))
-    return err("cudaFuncSetAttribute", e);
+  const size_t sm[2] = {fft_smem(logm[0]), fft_smem(logm[1])};
+  // The attribute belongs to the kernel, not to the call: always the size of the longest transform,
+  // so that a call on a small image never lowers it between another thread's call here and its
+  // launches.
+  for (auto k : {(const void *)k_fft_spec, (const void *)k_fft_z, (const void *)k_fft_x, (const void *)k_fft_z_inv})
+    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fft_smem(kFftMaxLogM))))
+      return err("cudaFuncSetAttribute", e);
   const FftPlan pz{nz, logm[0], t.t[0].tw, t.t[0].chirp, t.t[0].spec};
   const FftPlan px{nx, logm[1], t.t[1].tw, t.t[1].chirp, t.t[1].spec};
   const unsigned tb = (unsigned)((std::max(std::max(n[0], n[1]), (1 << std::max(logm[0], logm[1])) / 4) + kFftT - 1) / kFftT);
   if ((e = cudaMemsetAsync(fmax, 0, sizeof(unsigned), st))) return err("cudaMemsetAsync", e);
   k_fft_tables<<<dim3(tb, 2), kFftT, 0, st>>>(t);
-  k_fft_spec<<<2, kFftT, most, st>>>(t);
+  k_fft_spec<<<2, kFftT, std::max(sm[0], sm[1]), st>>>(t);
   k_bandpass_filter<<<(unsigned)((ncell + 255) / 256), 256, 0, st>>>(nx, nz, z1, z2, filt, fmax);
   k_fft_z<<<dim3(nx, nimg), kFftT, sm[0], st>>>(a, pz);
   k_fft_x<<<dim3(nz, nimg), kFftT, sm[1], st>>>(a, px);
+  if ((e = cudaGetLastError())) return err("launch", e);  // before the images are overwritten
   k_fft_z_inv<<<dim3(nx, nimg), kFftT, sm[0], st>>>(a, pz);
   if ((e = cudaGetLastError()) || (e = cudaStreamSynchronize(st))) return err("launch", e);
   return DS2D_OK;

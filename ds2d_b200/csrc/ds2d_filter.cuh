@@ -92,7 +92,8 @@ __global__ void __launch_bounds__(kDftTile *kDftTile) k_dft_gemm(DftArgs p) {
 }
 
 // ---- Bluestein transforms ----------------------------------------------------------------------
-constexpr int kFftMaxN = 4096;  // M = 8192 points: 144 KB of shared memory
+constexpr int kFftMaxN = 4096;   // M = 2^13 points: 144 KB of shared memory
+constexpr int kFftMaxLogM = 13;
 constexpr int kFftT = 256;
 
 struct FftPlan {

@@ -63,3 +63,34 @@ def test_bandpass_lengths(cuda_device, nx, nz, z1, z2):
     fpp, fps = bandpass_filter(pp, ps, z1, z2)
     assert rel(fpp, po.bandpass(pp, z1, z2)) < TOL
     assert rel(fps, po.bandpass(ps, z1, z2)) < TOL
+
+
+def test_bandpass_sizes_in_two_threads(cuda_device):
+    """Calls on a large and a small image in two threads (ctypes releases the interpreter lock):
+    both keep the results that they have alone."""
+    import threading
+    rng = np.random.default_rng(17)
+    cases = [(1201, 401, 10, 60, 60), (60, 40, 3, 12, 600)]
+    images = [rng.standard_normal((2, nx, nz)).astype(np.float32) for nx, nz, *_ in cases]
+    alone = [bandpass_filter(*im, z1, z2) for im, (_, _, z1, z2, _) in zip(images, cases)]
+    go, failed = threading.Barrier(2), []
+
+    def work(k):
+        _, _, z1, z2, calls = cases[k]
+        go.wait()
+        for _ in range(calls):
+            try:
+                got = bandpass_filter(*images[k], z1, z2)
+            except Exception as e:  # noqa: BLE001 - reported by the assertion below
+                failed.append((k, str(e)))
+                return
+            if not all(np.array_equal(a, b) for a, b in zip(got, alone[k])):
+                failed.append((k, "another result"))
+                return
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
