@@ -14,6 +14,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -311,9 +312,10 @@ struct ds2d_ctx {
   int opt_pcg_switch = 970;  // ds2d_lsrtm_pcg: per-mille residual ratio that ends the network phase
   int opt_pcg_m = 8;         // ds2d_lsrtm_pcg: directions kept for explicit conjugation
   // Tile kernels (ds2d_tile.cuh): option "tile" (-1 automatic, 0 off, 8 / 16 / 32 rows per CTA);
-  // an explicit launch-shape option selects the marching kernels it shapes.
+  // an explicit launch-shape option selects the marching kernels it shapes: those of the elastic
+  // steps, of the acoustic steps (note_shape).
   int opt_tile = -1;
-  bool shape_set = false;
+  bool shape_elastic = false, shape_acoustic = false;
   // Acoustic Born pair (LSRTM): background, scattered and adjoint states, Born overlay.
   float *ac[10] = {};        // bvx bvz bs | dvx dvz ds | yx yz ys | e
   float *ac_split[6] = {};   // with a PML: split stress s_x, s_z of background | scattered | adjoint
@@ -1075,7 +1077,7 @@ constexpr double kTileElastic = 3e6, kTileAcoustic = 3.5e6;
 bool tile_on(const ds2d_ctx *c, bool acoustic) {
   if (!tile_ok(c) || c->opt_tile == 0 || c->tile_nomem) return false;
   if (c->opt_tile > 0) return true;
-  if (c->shape_set) return false;
+  if (acoustic ? c->shape_acoustic : c->shape_elastic) return false;
   return !c->d.rbc || (double)c->B * c->d.slot <= (acoustic ? kTileAcoustic : kTileElastic);
 }
 // Rows per CTA.  Fewer rows are more CTAs, for batches that do not fill the chip (0.05 M cells
@@ -3140,18 +3142,13 @@ int ds2d_dot_f64(ds2d_ctx *c, const float *a, const float *b, long long n, doubl
   return dot64(c, a, b, n, result);
 }
 
-int ds2d_set_option(ds2d_ctx *c, const char *key, long long value) {
-  if (!c || !key) return DS2D_E_ARG;
-  std::string k(key);
-  // A graph holds the options of its capture ("graph" itself and the solver's options shape none).
-  if (k != "graph" && k.compare(0, 4, "pcg_") != 0) clear_graphs(c);
-  if (k != "graph" && k.compare(0, 4, "pcg_") != 0 && k != "adjoint_born" && k != "ac_ckpt" &&
-      k != "tile")
-    c->shape_set = true;
+// Stores one option; an unknown key or a rejected value changes nothing.
+static int store_option(ds2d_ctx *c, const std::string &k, long long value) {
   if (k == "tile") {
     if (value != -1 && value != 0 && value != 8 && value != 16 && value != 32)
       return fail(c, DS2D_E_ARG, "tile must be -1 (automatic), 0 (off), 8, 16 or 32 rows per CTA");
     c->opt_tile = (int)value;
+    if (value < 0) c->shape_elastic = c->shape_acoustic = false;  // automatic again
   } else if (k == "fused") {
     c->opt_fused = value != 0;
   } else if (k == "adjoint_born") {
@@ -3236,8 +3233,33 @@ int ds2d_set_option(ds2d_ctx *c, const char *key, long long value) {
     if (value < 8 || value > 4096) return fail(c, DS2D_E_ARG, "xr must be in [8, 4096]");
     c->opt_xr = (int)value;
   } else {
-    return fail(c, DS2D_E_ARG, "unknown option '%s'", key);
+    return fail(c, DS2D_E_ARG, "unknown option '%s'", k.c_str());
   }
+  return DS2D_OK;
+}
+
+// What an accepted option shapes: marching kernels of the elastic steps, of the acoustic ones.  With
+// a PML only the one-column ring kernels of the elastic steps take a shape.
+static void note_shape(ds2d_ctx *c, const std::string &k) {
+  auto in = [&](std::initializer_list<const char *> keys) {
+    return std::find(keys.begin(), keys.end(), k) != keys.end();
+  };
+  const bool both = in({"fused", "xr"}), ring = in({"ring", "occ", "cta", "bwd_1b"});
+  const bool acoustic = in({"ac_pair", "ac_pair_cta", "ac_duo"});
+  const bool bulk = in({"pair", "pair_cta", "pair_split", "pair_fcta", "pair_xr", "tb", "tb_cta",
+                        "tb_bulk", "bwd_bulk", "bwd_cta", "bwd_ws"});
+  if (both || ring || (bulk && c->d.rbc)) c->shape_elastic = true;
+  if (c->d.rbc && (both || acoustic || k == "pair_xr")) c->shape_acoustic = true;
+}
+
+int ds2d_set_option(ds2d_ctx *c, const char *key, long long value) {
+  if (!c || !key) return DS2D_E_ARG;
+  const std::string k(key);
+  const int rc = store_option(c, k, value);
+  if (rc) return rc;
+  // A graph holds the options of its capture ("graph" itself and the solver's options shape none).
+  if (k != "graph" && k.compare(0, 4, "pcg_") != 0) clear_graphs(c);
+  note_shape(c, k);
   return DS2D_OK;
 }
 

@@ -220,8 +220,9 @@ int ds2d_bandpass_filter_device(int nx, int nz, int x1, int x2, int z1, int z2, 
  * forward step only: the default), "pair_fcta" (forward CTA width 64 / 256, 0 = 256), "pair_cta" (backward
  * 64 / 160 / 256, 0 = 64), "pair_split" (0 / 1: backward in one or two launches), "pair_xr" (rows
  * per CTA, 0 = the count that fills the SMs' waves best), "ac_pair" (0 / 1: acoustic forward
- * steps of the Born pair on k_ac_pair) and "ac_pair_cta" (128 / 192 / 256, 0 = the width with the
- * fewest threads per grid row).  "ac_ckpt" (K, 0 = off; PML acoustic L^T): keep a snapshot of
+ * steps of the Born pair on k_ac_pair), "ac_pair_cta" (128 / 192 / 256, 0 = the width with the
+ * fewest threads per grid row) and "ac_duo" (1 = both sets of the Born modelling in one launch: the
+ * default; 0 = one launch per set).  "ac_ckpt" (K, 0 = off; PML acoustic L^T): keep a snapshot of
  * the whole background state every K steps, in the strip precision with one FP32 scale per field,
  * shot and snapshot, and replay each K-step segment from its snapshot with strips before
  * reversing it: snapshots plus K steps of strips instead of nt steps of strips, for one more
@@ -234,8 +235,10 @@ int ds2d_bandpass_filter_device(int nx, int nz, int x1, int x2, int z1, int z2, 
  * the default; 0 = two), "bwd_ws" (0 off, or 96 / 128 / 192 threads per role of the
  * warp-specialised step).  "tile": the tile kernels, one launch per time step with every row of a
  * tile in parallel, for batches that do not fill the chip and for every PML step: -1 = automatic
- * (the default: by boundary and padded cells of the context's slots, unless one of the launch-shape
- * options above is set), 0 = off, 8 / 16 / 32 = on with that many rows per CTA. */
+ * (the default: by boundary and padded cells of the context's slots; a launch-shape option above
+ * that is accepted later selects the marching kernels that it shapes, of the elastic or of the acoustic
+ * steps, until "tile" is set to -1 again), 0 = off, 8 / 16 / 32 = on with that many rows per CTA.  An
+ * unknown key or a rejected value (DS2D_E_ARG) changes nothing. */
 int ds2d_set_option(ds2d_ctx *ctx, const char *key, long long value);
 
 /* Profiling (no counterpart in the reference, which has only a commented-out host timer,

@@ -124,3 +124,37 @@ def test_changed_density_is_not_replayed(cuda_device):
         f.set_models(vp, vs)
         for a, b in zip(e.forward(shots), f.forward(shots)):
             np.testing.assert_array_equal(a, b)
+
+
+def test_options_leave_the_kernel_choice_alone(cuda_device):
+    """Which kernels a call runs (the names of the profile) after options that are refused, that
+    shape another path, that shape this path, and after "tile" = -1."""
+    from ds2d_b200._lib import DS2DError
+    c, vp, vs, rho, w, _ = _case(60, 48, 48, 8, 12)
+    shots = _shots(c, uneven=False)
+    m = np.full(vp.shape, 0.01, np.float32)
+
+    def tiles(e, acoustic):
+        e.profile(True)
+        e.ac_born(shots, m) if acoustic else e.forward(shots)
+        names = set(e.profile_report())
+        e.profile(False)
+        return ("ac_tile" if acoustic else "fwd_tile") in names
+
+    for boundary in ("pml", "random"):
+        with _ctx(c, shots, boundary=boundary) as e:
+            e.set_models(vp, vs, rho)
+            e.set_wavelet(w)
+            for key, value in (("no_such_option", 1), ("xr", 3), ("ac_duo", 7), ("tile", 5)):
+                with pytest.raises(DS2DError):
+                    e.set_option(key, value)
+            assert tiles(e, False) and tiles(e, True), boundary
+            e.set_option("ac_duo", 1)
+            assert tiles(e, False) and tiles(e, True) == (boundary == "pml"), boundary
+            e.set_option("tile", -1)
+            e.set_option("bwd_cta", 128)  # random-boundary RTM steps
+            assert tiles(e, False) == (boundary == "pml") and tiles(e, True), boundary
+            e.set_option("xr", 64)
+            assert not tiles(e, False) and tiles(e, True) == (boundary == "pml"), boundary
+            e.set_option("tile", -1)
+            assert tiles(e, False) and tiles(e, True), boundary
