@@ -338,6 +338,7 @@ struct ds2d_ctx {
   double batch_cells = 0, batch_wcells = 0;  // padded / interior cells of the current batch
   // CUDA graphs of whole batches (time loops included), keyed by everything baked into them.
   int opt_graph = 1;
+  bool graph_failed = false;  // no graph could be made on this stream: direct launches
   struct GraphEntry {
     std::array<long long, 5> key;
     cudaGraphExec_t exec;
@@ -1303,7 +1304,7 @@ GraphKey graph_key(const ds2d_ctx *c, int kind, int n, int shot_base) {
 }
 template <class F>
 int run_graph(ds2d_ctx *c, const GraphKey &key, F &&body) {
-  if (!c->opt_graph || c->prof.on || c->stream == nullptr) return body();
+  if (!c->opt_graph || c->graph_failed || c->prof.on || c->stream == nullptr) return body();
   for (const auto &g : c->graphs)
     if (key == g.key) {
       CK(cudaGraphLaunch(g.exec, c->stream));
@@ -1311,24 +1312,30 @@ int run_graph(ds2d_ctx *c, const GraphKey &key, F &&body) {
       return DS2D_OK;
     }
   const long long before = c->last_launches;
-  CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  const int rc = body();
-  cudaGraph_t graph = nullptr;
-  const cudaError_t e = cudaStreamEndCapture(c->stream, &graph);
-  if (rc) {
-    if (graph) cudaGraphDestroy(graph);
-    return rc;
-  }
-  CK(e);
   ds2d_ctx::GraphEntry g{};
   g.key = key;
-  const cudaError_t ie = cudaGraphInstantiate(&g.exec, graph, 0);
-  cudaGraphDestroy(graph);
-  CK(ie);
-  g.launches = c->last_launches - before;
-  c->graphs.push_back(g);
-  CK(cudaGraphLaunch(g.exec, c->stream));
-  return DS2D_OK;
+  cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    const int rc = body();
+    cudaGraph_t graph = nullptr;
+    e = cudaStreamEndCapture(c->stream, &graph);
+    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&g.exec, graph, 0);
+    if (graph) cudaGraphDestroy(graph);
+    if (rc) return rc;
+    g.launches = c->last_launches - before;
+    if (e == cudaSuccess) e = cudaGraphLaunch(g.exec, c->stream);
+    if (e == cudaSuccess) {
+      c->graphs.push_back(g);
+      return DS2D_OK;
+    }
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+  }
+  // A stream that cannot be captured (cudaStreamLegacy) or no memory for another graph: the same
+  // work in direct launches, from now on.
+  cudaGetLastError();
+  c->graph_failed = true;
+  c->last_launches = before;
+  return body();
 }
 
 int rtm_batch(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base) {
@@ -2673,6 +2680,7 @@ const char *ds2d_last_error(const ds2d_ctx *c) { return c ? c->err.c_str() : g_c
 int ds2d_set_stream(ds2d_ctx *c, void *stream) {
   if (!c) return DS2D_E_ARG;
   c->stream = stream ? (cudaStream_t)stream : c->own;
+  c->graph_failed = false;
   return DS2D_OK;
 }
 
@@ -3155,6 +3163,7 @@ static int store_option(ds2d_ctx *c, const std::string &k, long long value) {
     c->opt_adjoint_born = value != 0;
   } else if (k == "graph") {
     c->opt_graph = value != 0;
+    c->graph_failed = false;
   } else if (k == "ring") {
     if (value == 1) value = kDefaultRing;
     if (value != 0 && value != 2 && value != 4 && value != 8)

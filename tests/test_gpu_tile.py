@@ -158,3 +158,25 @@ def test_options_leave_the_kernel_choice_alone(cuda_device):
             assert not tiles(e, False) and tiles(e, True) == (boundary == "pml"), boundary
             e.set_option("tile", -1)
             assert tiles(e, False) and tiles(e, True), boundary
+
+
+def test_stream_that_cannot_be_captured(cuda_device):
+    """cudaStreamLegacy (handle 1) refuses graph capture: the calls launch directly, with the same
+    results as on the context's own stream."""
+    c, vp, vs, rho, w, rng = _case(60, 48, 48, 8, 40)
+    shots = _shots(c, uneven=False)
+    ntr = sum(s.ntr for s in shots)
+    obs = [rng.normal(size=(ntr, c["nt"])).astype(np.float32) for _ in range(2)]
+    m = 0.05 * rng.normal(size=vp.shape).astype(np.float32)
+    out = []
+    for handle in (0, 1):
+        with _ctx(c, shots, boundary="pml") as e:
+            e.set_stream(handle)
+            e.set_models(vp, vs, rho)
+            e.set_wavelet(w)
+            e.set_image(m, m)
+            mis = e.elsrtm(shots, *obs, 1)
+            out.append([mis, *e.read_images().values(), *e.ac_born(shots, m),
+                        e.ac_born_adj(shots, *obs), *e.forward(shots)])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
