@@ -339,6 +339,7 @@ struct ds2d_ctx {
   // CUDA graphs of whole batches (time loops included), keyed by everything baked into them.
   int opt_graph = 1;
   bool graph_failed = false;  // no graph could be made on this stream: direct launches
+  long long graph_held = 0;   // launches in the graphs of kinds from kGraphBounded on
   struct GraphEntry {
     std::array<long long, 5> key;
     cudaGraphExec_t exec;
@@ -434,6 +435,7 @@ int alloc_strips(ds2d_ctx *c, Strips &st, int steps) {
 void clear_graphs(ds2d_ctx *c) {
   for (auto &g : c->graphs) cudaGraphExecDestroy(g.exec);
   c->graphs.clear();
+  c->graph_held = 0;
 }
 
 // Frees one arena allocation before the context's end (buffers whose size follows an option).
@@ -1298,7 +1300,14 @@ int rtm_batch_body(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base);
 // graphs are off, when profiling, or on the legacy default stream (which cannot be captured).
 // A key names the call, its batch, the stream and the density array that k_setup reads; the other
 // options and buffers are those of the capture (a changed option or freed buffer drops the graphs).
+// Kinds: 1 forward modelling, 2 RTM, 3 / 4 ELSRTM (first / later iteration), 5 / 6 acoustic L / L^T,
+// 7 / 8 the same with the background kept between them.
 using GraphKey = std::array<long long, 5>;
+// A launch costs up to 4 KB of device and 12 KB of host memory in its graph, and ELSRTM and the
+// acoustic operators make two or more of them a time step: a survey of 240 single-shot batches of
+// 6000 steps would hold 12 GB on the device.  Theirs are kept up to this many launches (0.5 GB), the
+// batches beyond are launched directly.
+constexpr long long kGraphBounded = 3, kGraphLaunches = 1 << 17;
 GraphKey graph_key(const ds2d_ctx *c, int kind, int n, int shot_base) {
   return {kind, n, shot_base, (long long)(size_t)c->stream, (long long)(size_t)c->rho_all};
 }
@@ -1311,6 +1320,8 @@ int run_graph(ds2d_ctx *c, const GraphKey &key, F &&body) {
       c->last_launches += g.launches;
       return DS2D_OK;
     }
+  const bool bounded = key[0] >= kGraphBounded;
+  if (bounded && c->graph_held >= kGraphLaunches) return body();
   const long long before = c->last_launches;
   ds2d_ctx::GraphEntry g{};
   g.key = key;
@@ -1326,6 +1337,7 @@ int run_graph(ds2d_ctx *c, const GraphKey &key, F &&body) {
     if (e == cudaSuccess) e = cudaGraphLaunch(g.exec, c->stream);
     if (e == cudaSuccess) {
       c->graphs.push_back(g);
+      if (bounded) c->graph_held += g.launches;
       return DS2D_OK;
     }
     if (g.exec) cudaGraphExecDestroy(g.exec);

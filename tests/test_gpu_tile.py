@@ -180,3 +180,27 @@ def test_stream_that_cannot_be_captured(cuda_device):
                         e.ac_born_adj(shots, *obs), *e.forward(shots)])
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+def test_graph_memory_of_many_batches_is_bounded(cuda_device):
+    """The normal operator over 110 single-shot batches of 2000 steps: 440 thousand launches, whose
+    graphs at 4 KB a launch would hold 1.8 GB; at most 0.5 GB and the last graph are kept.  The
+    image is that of direct launches."""
+    import torch
+    c, vp, vs, rho, w, _ = _case(60, 48, 48, 8, 2000)
+    shots = [s for s in _shots(c, uneven=False)[:2] for _ in range(55)]
+    m = torch.full(vp.shape, 0.01, device="cuda")
+    out = []
+    for graph in (1, 0):
+        with Elastic2D(c["allnx"], c["allnz"], c["nx"], c["pml"], c["nt"], c["dx"], c["dz"], c["dt"],
+                       boundary="pml", max_shots=1, max_ntr=c["nx"]) as e:
+            e.set_option("graph", graph)
+            e.set_models(vp, vs, rho)
+            e.set_wavelet(w)
+            img = torch.zeros_like(m)
+            e.ac_normal_device(shots[:1], m.data_ptr(), img.data_ptr())  # allocates the state
+            free = torch.cuda.mem_get_info()[0]
+            e.ac_normal_device(shots, m.data_ptr(), img.data_ptr())
+            assert free - torch.cuda.mem_get_info()[0] < 1 << 30
+            out.append(img.cpu().numpy())
+    np.testing.assert_array_equal(*out)
