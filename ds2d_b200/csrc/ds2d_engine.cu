@@ -1673,6 +1673,14 @@ int elsrtm_backward_fused(ds2d_ctx *c, int n, bool strips) {
   return DS2D_OK;
 }
 
+// Whether ELSRTM's forward / backward pass runs fused.  The fused kernels compute the Born source
+// from the new velocities inside their stress stage; that needs every interior cell inside the
+// updated band (pml >= nop).  The fused backward pass has no scattered-adjoint term.
+bool elsrtm_fused(const ds2d_ctx *c, bool backward) {
+  return c->opt_fused && c->opt_ring == 4 && c->ring_ok && c->d.pml >= c->d.nop &&
+         !(backward && c->opt_adjoint_born);
+}
+
 int elsrtm_body(ds2d_ctx *c, int n, int shot_base, int iter) {
   const Dims &d = c->d;
   int rc;
@@ -1689,9 +1697,7 @@ int elsrtm_body(ds2d_ctx *c, int n, int shot_base, int iter) {
   const bool strips = !d.rbc;
   dim3 grid = cell_grid(d, n), blk(kBX, kBY);
   // Forward pass, FD2DGPU.cu:4396-4478: background, first- and second-order scattered sets.
-  // The ring kernels compute the Born source from the new velocities inside their stress stage;
-  // that needs every interior cell inside the updated band (pml >= nop).
-  const bool fused_fwd = c->opt_fused && c->opt_ring == 4 && c->ring_ok && d.pml >= d.nop;
+  const bool fused_fwd = elsrtm_fused(c, false), fused_bwd = elsrtm_fused(c, true);
   if (fused_fwd && (rc = elsrtm_forward_fused(c, n, strips))) return rc;
   for (int it = 0; it < d.nt && !fused_fwd; it++) {
     VelArgs v = vel_args(c, c->fw, it);
@@ -1729,8 +1735,7 @@ int elsrtm_body(ds2d_ctx *c, int n, int shot_base, int iter) {
   c->last_launches++;
   CK(cudaGetLastError());
   dim3 igrid((d.wnz + kBX - 1) / kBX, (d.wnx + kBY - 1) / kBY, n);
-  // Backward pass, FD2DGPU.cu:4685-4807 (the fused path has no scattered-adjoint term).
-  const bool fused_bwd = fused_fwd && !c->opt_adjoint_born;
+  // Backward pass, FD2DGPU.cu:4685-4807.
   if (fused_bwd && (rc = elsrtm_backward_fused(c, n, strips))) return rc;
   for (int it = d.nt - 1; it >= 0 && !fused_bwd; --it) {
     StrArgs sr = str_args(c, c->fw, it);
@@ -1800,15 +1805,15 @@ int elsrtm_batch(ds2d_ctx *c, const ds2d_shot *shots, int n, int shot_base, int 
                  double *mis_host) {
   const Dims &d = c->d;
   int rc;
-  // allocations must precede the graph capture
-  if (c->opt_fused) {
+  // allocations must precede the graph capture: what the passes below use, and no more
+  if (elsrtm_fused(c, false)) {
     for (Wave *w : {&c->fw2, &c->b1_2, &c->b2_2})
       if (!w->vx && (rc = alloc_wave(c, *w, false))) return rc;
-    if (!c->abk2.vx && (rc = alloc_wave(c, c->abk2, true))) return rc;
     for (float *&p : c->ov_s2)
       if (!p && (rc = alloc_slots(c, &p))) return rc;
   }
-  if (tile_on(c, false)) {
+  if (elsrtm_fused(c, true) && !c->abk2.vx && (rc = alloc_wave(c, c->abk2, true))) return rc;
+  if (elsrtm_fused(c, false) && tile_on(c, false)) {
     rc = DS2D_OK;
     for (auto &o : c->ov_t)
       for (float *&p : o)

@@ -204,3 +204,30 @@ def test_graph_memory_of_many_batches_is_bounded(cuda_device):
             assert free - torch.cuda.mem_get_info()[0] < 1 << 30
             out.append(img.cpu().numpy())
     np.testing.assert_array_equal(*out)
+
+
+def test_elsrtm_half_steps_allocate_no_fused_state(cuda_device):
+    """ELSRTM on half steps (ring 0) does not hold the fused passes' second buffers: three forward
+    sets of 15 arrays, an adjoint set of 11 and a Born source of 3 (59 arrays of every slot); with
+    "adjoint_born", whose backward pass is made of half steps, not the adjoint set."""
+    import torch
+    c, vp, vs, rho, w, rng = _case(500, 284, 500, 8, 3)
+    shots = _shots(c, uneven=False)
+    ntr = sum(s.ntr for s in shots)
+    obs = [rng.normal(size=(ntr, c["nt"])).astype(np.float32) for _ in range(2)]
+    img = 0.05 * rng.normal(size=vp.shape).astype(np.float32)
+    array = 4 * len(shots) * (500 + 16) * 320
+    used = {}
+    for name, opts in (("fused", {}), ("half", {"ring": 0}), ("born", {"adjoint_born": 1})):
+        with _ctx(c, shots, boundary="pml") as e:
+            e.set_option("graph", 0)
+            for k, v in opts.items():
+                e.set_option(k, v)
+            e.set_models(vp, vs, rho)
+            e.set_wavelet(w)
+            e.set_image(img, img)
+            free = torch.cuda.mem_get_info()[0]
+            e.elsrtm(shots, *obs, 1)
+            used[name] = free - torch.cuda.mem_get_info()[0]
+    assert used["half"] <= used["fused"] - 57 * array, used
+    assert used["born"] <= used["fused"] - 10 * array, used
