@@ -1063,8 +1063,11 @@ cudaError_t tile_attributes() {
   return e;
 }
 
-bool tile_ok(const ds2d_ctx *c) {
-  return c->opt_fused && c->ring_ok && c->d.nop == 4 && c->d.ild == c->d.ld;
+// A launch takes up to five grid slices of the batch's shots elastic (ELSRTM: three sets and two
+// strip slices) and three acoustic (two sets, one strip slice); a grid has 65535 slices.
+bool tile_ok(const ds2d_ctx *c, bool acoustic) {
+  return c->opt_fused && c->ring_ok && c->d.nop == 4 && c->d.ild == c->d.ld &&
+         c->B <= 65535 / (acoustic ? 3 : 5);
 }
 // Where a context's steps run on the tile kernels.  The rule looks at the context's batch (padded
 // cells of all its slots), so every batch of a context, a last short one too, takes the same
@@ -1078,7 +1081,7 @@ bool tile_ok(const ds2d_ctx *c) {
 //    / 8.5, 2.8 M 10.5 / 8.7, 4.5 M 12.4 / 13.6, 8.9 M 21.2 / 26.5: 3.5 M.
 constexpr double kTileElastic = 3e6, kTileAcoustic = 3.5e6;
 bool tile_on(const ds2d_ctx *c, bool acoustic) {
-  if (!tile_ok(c) || c->opt_tile == 0 || c->tile_nomem) return false;
+  if (!tile_ok(c, acoustic) || c->opt_tile == 0 || c->tile_nomem) return false;
   if (c->opt_tile > 0) return true;
   if (acoustic ? c->shape_acoustic : c->shape_elastic) return false;
   return !c->d.rbc || (double)c->B * c->d.slot <= (acoustic ? kTileAcoustic : kTileElastic);
@@ -1118,7 +1121,7 @@ void launch_tile(ds2d_ctx *c, const char *name, double bytes, const TileKernel<v
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = chain && ev < 0 ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k.fn, a);
+  cudaLaunchKernelEx(&cfg, k.fn, a);  // a refused launch is the last error, which the callers read
   c->last_launches++;
   if (ev >= 0) {
     cudaEventRecord(c->prof.pool[ev + 1], c->stream);

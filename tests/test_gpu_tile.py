@@ -231,3 +231,29 @@ def test_elsrtm_half_steps_allocate_no_fused_state(cuda_device):
             used[name] = free - torch.cuda.mem_get_info()[0]
     assert used["half"] <= used["fused"] - 57 * array, used
     assert used["born"] <= used["fused"] - 10 * array, used
+
+
+@pytest.mark.parametrize("shots_n", [13107, 13108])
+def test_elsrtm_of_the_largest_batches(cuda_device, shots_n):
+    """ELSRTM with a PML and the most shots that the tile launches' grid takes (five slices a shot,
+    65535 in all), and one more, against the same shots in batches of 700."""
+    c, vp, vs, _, w, rng = _case(16, 16, 16, 8, 24)
+    igx = np.arange(8, 24, 5, dtype=np.int32)
+    shots = [ShotGeom(0, 9 + k % 14, 10, 11, igx, 16) for k in range(shots_n)]
+    obs = [rng.normal(size=(shots_n * len(igx), c["nt"])).astype(np.float32) for _ in range(2)]
+    img = 0.05 * rng.normal(size=vp.shape).astype(np.float32)
+    out = []
+    for cap in (shots_n, 700):
+        with Elastic2D(16, 16, 16, 8, c["nt"], c["dx"], c["dz"], c["dt"], boundary="pml",
+                       max_shots=cap, max_ntr=len(igx)) as e:
+            e.set_models(vp, vs)
+            e.set_wavelet(w)
+            e.set_image(img, img)
+            mis = e.elsrtm(shots, *obs, 1)
+            out.append((mis, e.read_images()))
+    assert abs(out[0][0] - out[1][0]) < GATE * shots_n
+    for k, v in out[1][1].items():
+        if not np.any(v):  # the scattered adjoint's images
+            assert not np.any(out[0][1][k]) and k not in ("pp_grad", "ps_grad", "b_pp", "b_ps")
+            continue
+        assert rel(out[0][1][k], v) < (BORN_GATE if k in ("b_pp", "b_ps") else GATE), k
