@@ -77,6 +77,34 @@ def test_autotuner_candidates_name_every_knob():
     assert {c["bwd_cta"] for c in space} >= {128, 192, 256}
 
 
+def test_autotuner_holds_the_library_default():
+    """The untouched default is a candidate of both spaces, so tuning never ends slower than not
+    tuning, and so are all row counts of the tile kernels; applying it sets "tile" last, after
+    the launch shapes that would otherwise select the marching kernels."""
+    from ds2d_b200 import autotune
+
+    class Recorder:
+        def __init__(self):
+            self.calls = []
+
+        def set_option(self, key, value):
+            self.calls.append((key, value))
+
+    for boundary in ("random", "pml"):
+        space = autotune.default_space(boundary)
+        assert {c["tile"] for c in space} == {-1, 0, 8, 16, 32}
+        default = [c for c in space if c["tile"] == -1]
+        assert len(default) == 1
+        for cfg in (default[0], dict(sorted(default[0].items()))):
+            ctx = Recorder()
+            autotune.apply(ctx, cfg)
+            assert ctx.calls[-1] == ("tile", -1) and dict(ctx.calls) == default[0]
+        times = {autotune.key(c): 1.0 for c in space}
+        assert autotune.choose(space, times) == default[0]
+        times[autotune.key(space[-1])] = 0.98
+        assert autotune.choose(space, times) == space[-1]
+
+
 def test_tensor_peak_reads_the_measured_burst_figure():
     """The U-Net line's roofline denominator: the measured BF16 burst figure when the peaks file
     is there, the earlier pool measurement otherwise; a plausible B200 dense figure either way."""
