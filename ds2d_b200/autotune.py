@@ -120,7 +120,7 @@ def choose(space, timings):
     """The fastest setting; the library's default where no other is 1 % faster (two runs of one
     setting differ by about 0.5 %), since it alone leaves the context's other calls their choice."""
     best = min(space, key=lambda c: timings[key(c)])
-    default = next((c for c in space if c.get("tile") == -1), best)
+    default = LIBRARY_DEFAULT if LIBRARY_DEFAULT in space else best
     return default if timings[key(default)] <= 1.01 * timings[key(best)] else best
 
 
