@@ -313,3 +313,25 @@ def test_unet_weight_gradient_sums(cuda_device, n, h, w):
         want = taps[:, :, None, None] * sign[:, None] * a
         assert rel(g[name + ".w"], want) < 84 * 2.0 ** -24, (name, rel(g[name + ".w"], want))
     assert rel(g["d1b.b"], sign * dy.sum()) < 84 * 2.0 ** -24
+
+
+def test_unet_results_into_any_memory(cuda_device):
+    """Parameters and gradients read into pageable, pinned and device memory."""
+    import ctypes
+    import torch
+    from ds2d_b200.unet import UNet, he_normal
+    x = torch.ones((1, 8, 8), device="cuda")
+    fp = ctypes.POINTER(ctypes.c_float)
+    with UNet(max_n=1, max_h=8, max_w=8) as net:
+        params = he_normal(5)
+        net.set_params(params)
+        _, want = net.loss_grad(x.data_ptr(), x.data_ptr(), 1, 8, 8, want_grads=True)
+        for dst in (torch.zeros(net.n), torch.zeros(net.n).pin_memory(), torch.zeros(net.n, device="cuda")):
+            torch.cuda.synchronize()
+            ptr = ctypes.cast(dst.data_ptr(), fp)
+            net._check(net.lib.ds2d_unet_get_params(net.h, ptr, net.n))
+            np.testing.assert_array_equal(dst.cpu().numpy(), params)
+            net._check(net.lib.ds2d_unet_loss_grad(net.h, ctypes.c_void_p(x.data_ptr()),
+                                                   ctypes.c_void_p(x.data_ptr()), 1, 8, 8, None, ptr))
+            # sums of FP32 parts in no fixed order
+            assert rel(dst.cpu().numpy(), want) < 1e-5
