@@ -12,6 +12,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
+#include <cstdint>
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
@@ -3614,7 +3615,16 @@ int bandpass_fft(int nx, int nz, int z1, int z2, float *const imgs[2], cudaStrea
 }
 
 int bandpass_images(int nx, int nz, int z1, int z2, float *const imgs[2], cudaStream_t st) {
-  if (nx <= kFftMaxN && nz <= kFftMaxN) return bandpass_fft(nx, nz, z1, z2, imgs, st);
+  if (nx <= kFftMaxN && nz <= kFftMaxN) {
+    // both images in one launch, unless they share memory: then the second is filtered as the first
+    // left it
+    const std::uintptr_t a = (std::uintptr_t)imgs[0], b = (std::uintptr_t)imgs[1];
+    if (!a || !b || (a > b ? a - b : b - a) >= sizeof(float) * (size_t)nx * nz)
+      return bandpass_fft(nx, nz, z1, z2, imgs, st);
+    float *const one[2] = {imgs[0], nullptr}, *const two[2] = {imgs[1], nullptr};
+    const int rc = bandpass_fft(nx, nz, z1, z2, one, st);
+    return rc ? rc : bandpass_fft(nx, nz, z1, z2, two, st);
+  }
   auto err = [&](const char *what, cudaError_t e) {
     g_create_err = std::string("ds2d_bandpass_filter: ") + what + ": " + cudaGetErrorString(e);
     return DS2D_E_CUDA;

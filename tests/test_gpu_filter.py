@@ -94,3 +94,19 @@ def test_bandpass_sizes_in_two_threads(cuda_device):
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("shift", [0, 5])
+def test_bandpass_device_images_that_share_memory(cuda_device, shift):
+    """One buffer as both images, and two overlapping ones: filtered one after the other, the
+    second as the first left it."""
+    import torch
+    nx, nz = 24, 10
+    base = np.random.default_rng(4).standard_normal(nx * nz + shift * nz).astype(np.float32)
+    want = base.copy()
+    for at in (0, shift * nz):
+        want[at:at + nx * nz] = po.bandpass(want[at:at + nx * nz].reshape(nx, nz), 2, 5).ravel()
+    d = torch.from_numpy(base).cuda()
+    torch.cuda.synchronize()
+    bandpass_filter_device(d.data_ptr(), d.data_ptr() + 4 * shift * nz, nx, nz, 2, 5)
+    assert rel(d.cpu().numpy(), want) < TOL
