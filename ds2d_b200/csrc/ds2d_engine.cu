@@ -3177,6 +3177,7 @@ static int store_option(ds2d_ctx *c, const std::string &k, long long value) {
     if (value != -1 && value != 0 && value != 8 && value != 16 && value != 32)
       return fail(c, DS2D_E_ARG, "tile must be -1 (automatic), 0 (off), 8, 16 or 32 rows per CTA");
     c->opt_tile = (int)value;
+    c->tile_nomem = false;  // there may be memory again
     if (value < 0) c->shape_elastic = c->shape_acoustic = false;  // automatic again
   } else if (k == "fused") {
     c->opt_fused = value != 0;

@@ -237,7 +237,8 @@ int ds2d_bandpass_filter_device(int nx, int nz, int x1, int x2, int z1, int z2, 
  * tile in parallel, for batches that do not fill the chip and for every PML step: -1 = automatic
  * (the default: by boundary and padded cells of the context's slots; a launch-shape option above
  * that is accepted later selects the marching kernels that it shapes, of the elastic or of the acoustic
- * steps, until "tile" is set to -1 again), 0 = off, 8 / 16 / 32 = on with that many rows per CTA.  An
+ * steps, until "tile" is set to -1 again), 0 = off, 8 / 16 / 32 = on with that many rows per CTA.  A
+ * context without memory for their extra buffers stays on the other kernels until "tile" is set.  An
  * unknown key or a rejected value (DS2D_E_ARG) changes nothing. */
 int ds2d_set_option(ds2d_ctx *ctx, const char *key, long long value);
 

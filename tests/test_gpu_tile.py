@@ -257,3 +257,56 @@ def test_elsrtm_of_the_largest_batches(cuda_device, shots_n):
             assert not np.any(out[0][1][k]) and k not in ("pp_grad", "ps_grad", "b_pp", "b_ps")
             continue
         assert rel(out[0][1][k], v) < (BORN_GATE if k in ("b_pp", "b_ps") else GATE), k
+
+
+@pytest.mark.parametrize("acoustic", [True, False])
+def test_tiles_without_memory_for_their_buffers(cuda_device, acoustic):
+    """With room for three of the extra arrays that the tile steps need (seven acoustic, six for
+    ELSRTM), a context stays on the other kernels and gives those three back; once there is memory
+    again, setting "tile" brings the tiles back."""
+    import torch
+    c, vp, vs, rho, w, rng = _case(592, 496, 592, 8, 12)
+    shots = _shots(c, uneven=False) * 8
+    ntr = sum(s.ntr for s in shots)
+    obs = [rng.normal(size=(ntr, c["nt"])).astype(np.float32) for _ in range(2)]
+    m = 0.05 * rng.normal(size=vp.shape).astype(np.float32)
+    array = 4 * len(shots) * (592 + 16) * 512
+
+    def run(e):
+        e.profile(True)
+        if acoustic:
+            out = [*e.ac_born(shots, m), e.ac_born_adj(shots, *obs)]
+        else:
+            out = [e.elsrtm(shots, *obs, 1), *e.read_images().values()]
+        tiles = any("tile" in name for name in e.profile_report())
+        e.profile(False)
+        return out, tiles
+
+    with _ctx(c, shots, boundary="pml") as e:
+        e.set_models(vp, vs, rho)
+        e.set_wavelet(w)
+        e.set_image(m, m)
+        e.set_option("tile", 0)
+        want, tiles = run(e)
+        assert not tiles
+        torch.cuda.empty_cache()
+        held = [torch.empty(torch.cuda.mem_get_info()[0] - 8 * array, dtype=torch.uint8, device="cuda")]
+        with pytest.raises(torch.OutOfMemoryError):
+            while True:  # the rest, in blocks of one array
+                held.append(torch.empty(array, dtype=torch.uint8, device="cuda"))
+        del held[-3:]
+        torch.cuda.empty_cache()
+        left = torch.cuda.mem_get_info()[0]
+        e.set_option("tile", -1)
+        got, tiles = run(e)
+        assert not tiles and torch.cuda.mem_get_info()[0] >= left - (16 << 20)
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a, b)
+        del held
+        torch.cuda.empty_cache()
+        assert not run(e)[1]
+        e.set_option("tile", -1)
+        got, tiles = run(e)
+        assert tiles
+        for a, b in zip(got, want):
+            assert rel(a, b) < BORN_GATE or not np.any(b)
