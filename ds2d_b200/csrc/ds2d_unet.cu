@@ -1660,10 +1660,10 @@ int check_wait_flag(ds2d_unet *u) {
 
 // Gradients into the caller's array.  Pinned, managed and device memory takes one copy.  Pageable
 // memory is filled through two pinned chunks, one filling while the host empties the other, so the
-// page faults of a fresh array overlap the copy: 7.7 MB into a fresh array 2.04 ms against 3.37,
-// into one written before 0.50 against 0.48 (chunks of 256 KB 2.06 and 0.56, of 1 MB 2.15 and 0.49,
-// and pinning those costs ds2d_unet_create 1 ms more).
-constexpr size_t kStageChunk = 512 << 10;
+// page faults of a fresh array overlap the copy: 7.7 MB into a fresh array 2.06 ms against 3.37,
+// into one written before 0.56 against 0.48 (chunks of 512 KB 2.04 and 0.50, but ds2d_unet_create takes
+// 2 ms longer to pin them).
+constexpr size_t kStageChunk = 256 << 10;
 int to_host(ds2d_unet *u, void *dst, const void *src, size_t bytes) {
   cudaPointerAttributes at{};
   if (cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type != cudaMemoryTypeUnregistered) {
