@@ -67,7 +67,6 @@ struct ConvArgs {
   const bf16 *wt;   // [9][cout][cin]
   const float *bias;  // [cout] or null
   bf16 *out;        // [N][H][W][ocs], channels [oco, oco + cout)
-  float *out_f32;   // optional FP32 copy, same indexing as out
   const bf16 *mask; // optional: out *= (mask > 0), mask [N][H][W][ocs] at the same channels
   int n, h, w, cin, cout, ocs, oco, relu;
 };
@@ -146,10 +145,6 @@ __global__ void __launch_bounds__(64 * (kCo / 32)) k_conv3x3(ConvArgs a) {
         if (!(__bfloat162float(m.y) > 0.f)) v1 = 0.f;
       }
       *reinterpret_cast<__nv_bfloat162 *>(a.out + o) = __floats2bfloat162_rn(v0, v1);
-      if (a.out_f32) {
-        a.out_f32[o] = v0;
-        a.out_f32[o + 1] = v1;
-      }
     }
   }
 }
@@ -185,11 +180,9 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint
   return d;                // base offset 0, legacy LBO mode, layout type 0 (no swizzle)
 }
 
-// K-major with rows of kCK channels (32- or 64-byte swizzle): groups of 8 rows `sbo` bytes apart.
-template <int kCK>
-__device__ __forceinline__ uint64_t umma_desc_sw(uint32_t saddr, uint32_t sbo) {
-  static_assert(kCK == 16 || kCK == 32, "rows of 32 or 64 bytes");
-  return umma_desc(saddr, 16, sbo) | (uint64_t)(kCK == 16 ? 6 : 4) << 61;
+// K-major with rows of 16 channels (32-byte swizzle): groups of 8 rows `sbo` bytes apart.
+__device__ __forceinline__ uint64_t umma_desc_sw32(uint32_t saddr, uint32_t sbo) {
+  return umma_desc(saddr, 16, sbo) | (uint64_t)6 << 61;
 }
 
 // MN-major blocks of kC channels (32 or 16) with one row of kC channels per K index: blocks `lbo`
@@ -331,10 +324,6 @@ __global__ void __launch_bounds__(128) k_conv3x3_tc(ConvArgs a, int *err) {
 #pragma unroll
         for (int j = 0; j < 4; j++) p[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
         *reinterpret_cast<uint4 *>(a.out + o) = *reinterpret_cast<uint4 *>(p);
-        if (a.out_f32) {
-#pragma unroll
-          for (int j = 0; j < 8; j++) a.out_f32[o + j] = v[j];
-        }
       }
     }
   }
@@ -361,9 +350,9 @@ constexpr int tc_smem_bytes() {
 // ---------------------------------------------------------------------------------------------
 // The same convolution fed by the tensor-memory accelerator (option "tcgen05_tma").  A CTA owns kJ
 // M-tiles of 8 pixels x 16 rows side by side (8 kJ x 16 output pixels) and kN output channels.  Per
-// stage of kCK input channels one thread issues ONE tiled bulk-tensor load of the (8 kJ + 2) x 18
-// halo box, whose rows are the kCK channels of a pixel (32 or 64 bytes, whole sectors) in the
-// 32- or 64-byte swizzle that the A descriptor names, and one bulk copy of the stage's weights
+// 16-channel chunk, into one of kS stages, one thread issues ONE tiled bulk-tensor load of the
+// (8 kJ + 2) x 18 halo box, whose rows are the 16 channels of a pixel (32 bytes, a whole sector) in
+// the 32-byte swizzle that the A descriptor names, and one bulk copy of the chunk's weights
 // (contiguous: blocked by output tile).  An M-tile's 16 groups of 8 pixels are the 16 image rows of
 // the box, so the descriptor's group stride is the box's row pitch and every tap (and M-tile) is an
 // offset of its start address: (ky (8 kJ + 2) + kx + 8 j) pixels.  The swizzle acts on the address
@@ -372,25 +361,24 @@ constexpr int tc_smem_bytes() {
 // is bounded.
 //
 // Why this tile: widths are multiples of 8 but rarely of 128, and the deeper levels are 152, 76 or 32
-// pixels wide, so M-tiles along one image row did 1.05-4 times the work; the halo is 1.2 pixels per
-// output pixel for kJ = 4 against 1.52 for four rows of 130; and a box row of 8 channels (16 bytes,
+// pixels wide, so M-tiles along one image row did 1.05-4 times the work; the halo is 1.27 pixels
+// per output pixel for kJ = 2 and 1.41 for kJ = 1, against 1.52 for four rows of 130; and a box row of 8 channels (16 bytes,
 // half a sector) was one L2 request each, which set the pace.
 // ---------------------------------------------------------------------------------------------
 constexpr int kTileH = 16;  // output rows of a CTA's tile
 template <int kJ>
 __host__ __device__ constexpr int cv_pitch() { return 8 * kJ + 2; }  // halo pixels per box row
-template <int kJ, int kCK>
-__host__ __device__ constexpr int cv_a_bytes() { return cv_pitch<kJ>() * (kTileH + 2) * kCK * 2; }
-template <int kN, int kCK>
-__host__ __device__ constexpr int cv_b_bytes() { return 9 * 2 * kN * 16 * (kCK / 16); }
-template <int kN, int kJ, int kCK>
+template <int kJ>
+__host__ __device__ constexpr int cv_a_bytes() { return cv_pitch<kJ>() * (kTileH + 2) * 32; }
+template <int kN>
+__host__ __device__ constexpr int cv_b_bytes() { return 9 * 2 * kN * 16; }
+template <int kN, int kJ>
 __host__ __device__ constexpr int cv_stage_bytes() {
-  return (cv_a_bytes<kJ, kCK>() + 1023) / 1024 * 1024 + (cv_b_bytes<kN, kCK>() + 1023) / 1024 * 1024;
+  return (cv_a_bytes<kJ>() + 1023) / 1024 * 1024 + (cv_b_bytes<kN>() + 1023) / 1024 * 1024;
 }
-constexpr int kCvMaxStages = 3;
-template <int kN, int kJ, int kCK>
-constexpr int cv_smem_bytes(int stages) {
-  return 1024 + stages * cv_stage_bytes<kN, kJ, kCK>() + 8 * (2 * kCvMaxStages + 1);
+template <int kN, int kJ, int kS>
+constexpr int cv_smem_bytes() {
+  return 1024 + kS * cv_stage_bytes<kN, kJ>() + 8 * (2 * kS + 1);
 }
 
 __device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity) {
@@ -420,16 +408,16 @@ __device__ __forceinline__ void tmem_ld32(uint32_t (&r)[32], uint32_t taddr) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
-template <int kN, int kJ, int kCK>
+template <int kN, int kJ, int kS>
 __global__ void __launch_bounds__(128) k_conv3x3_tma(ConvArgs a, const __grid_constant__ CUtensorMap tmA,
-                                                     const bf16 *wblk, int stages, int *err) {
+                                                     const bf16 *wblk, int *err) {
   extern __shared__ unsigned char cv_raw[];
   unsigned char *sm = cv_raw + ((1024 - (smem_u32(cv_raw) & 1023)) & 1023);
-  constexpr int kStage = cv_stage_bytes<kN, kJ, kCK>();
-  constexpr int kA = (cv_a_bytes<kJ, kCK>() + 1023) / 1024 * 1024, kP = cv_pitch<kJ>();
-  uint64_t *full = reinterpret_cast<uint64_t *>(sm + stages * kStage);
-  uint64_t *empty = full + kCvMaxStages;
-  uint64_t *done = empty + kCvMaxStages;
+  constexpr int kStage = cv_stage_bytes<kN, kJ>();
+  constexpr int kA = (cv_a_bytes<kJ>() + 1023) / 1024 * 1024, kP = cv_pitch<kJ>();
+  uint64_t *full = reinterpret_cast<uint64_t *>(sm + kS * kStage);
+  uint64_t *empty = full + kS;
+  uint64_t *done = empty + kS;
   __shared__ uint32_t tmem_base;
   __shared__ int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -444,7 +432,7 @@ __global__ void __launch_bounds__(128) k_conv3x3_tma(ConvArgs a, const __grid_co
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
   if (tid == 0) {
-    for (int k = 0; k < 2 * kCvMaxStages + 1; k++)
+    for (int k = 0; k < 2 * kS + 1; k++)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(full + k)));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     s_fail = 0;
@@ -454,37 +442,37 @@ __global__ void __launch_bounds__(128) k_conv3x3_tma(ConvArgs a, const __grid_co
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
   const uint32_t tmem = tmem_base;
   constexpr uint32_t idesc = umma_idesc(kTcM, kN);
-  const int nst = a.cin / kCK;  // stages of work
+  const int nst = a.cin / 16;  // chunks
   if (tid == 0) {
     const uint64_t ta = reinterpret_cast<uint64_t>(&tmA);
     const unsigned char *wsrc =
         reinterpret_cast<const unsigned char *>(wblk) + (size_t)grp * (a.cin / 16) * (18 * kN * 16);
     for (int c = 0; c < nst; c++) {
-      const int st = c % stages, k = c / stages;
-      if (c >= stages && !tc_wait(empty + st, (k - 1) & 1)) {
+      const int st = c % kS, k = c / kS;
+      if (c >= kS && !tc_wait(empty + st, (k - 1) & 1)) {
         s_fail = 1;
         break;
       }
       unsigned char *sA = sm + st * kStage;
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(
                        smem_u32(full + st)),
-                   "r"((uint32_t)(cv_a_bytes<kJ, kCK>() + cv_b_bytes<kN, kCK>()))
+                   "r"((uint32_t)(cv_a_bytes<kJ>() + cv_b_bytes<kN>()))
                    : "memory");
       asm volatile(
           "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
           " [%0], [%1, {%2, %3, %4, %5}], [%6];\n" ::"r"(smem_u32(sA)),
-          "l"(ta), "r"(c * kCK), "r"(w0 - 1), "r"(row0 - 1), "r"(img), "r"(smem_u32(full + st))
+          "l"(ta), "r"(c * 16), "r"(w0 - 1), "r"(row0 - 1), "r"(img), "r"(smem_u32(full + st))
           : "memory");
       asm volatile(
           "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
               smem_u32(sA + kA)),
-          "l"(wsrc + (size_t)c * cv_b_bytes<kN, kCK>()), "r"((uint32_t)cv_b_bytes<kN, kCK>()),
+          "l"(wsrc + (size_t)c * cv_b_bytes<kN>()), "r"((uint32_t)cv_b_bytes<kN>()),
           "r"(smem_u32(full + st))
           : "memory");
     }
   } else if (tid == 32) {
     for (int c = 0; c < nst; c++) {
-      const int st = c % stages, k = c / stages;
+      const int st = c % kS, k = c / kS;
       if (!tc_wait(full + st, k & 1)) {
         s_fail = 1;
         break;
@@ -492,23 +480,19 @@ __global__ void __launch_bounds__(128) k_conv3x3_tma(ConvArgs a, const __grid_co
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
       const uint32_t a_base = smem_u32(sm + st * kStage), b_base = a_base + kA;
 #pragma unroll
-      for (int k2 = 0; k2 < kCK / 16; k2++)
+      for (int j = 0; j < kJ; j++)
 #pragma unroll
-        for (int j = 0; j < kJ; j++)
-#pragma unroll
-          for (int tap = 0; tap < 9; tap++) {
-            const int ky = tap / 3, kx = tap % 3;
-            const uint64_t ad = umma_desc_sw<kCK>(
-                a_base + (ky * kP + kx + 8 * j) * (kCK * 2) + k2 * 32, kP * kCK * 2);
-            const uint64_t bd =
-                umma_desc(b_base + ((k2 * 9 + tap) * 2) * (kN * 16), kN * 16, 128);
-            const uint32_t acc = (c > 0 || k2 > 0 || tap > 0) ? 1u : 0u;
-            asm volatile(
-                "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-                    tmem + (uint32_t)(j * kN)),
-                "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
-          }
+        for (int tap = 0; tap < 9; tap++) {
+          const int ky = tap / 3, kx = tap % 3;
+          const uint64_t ad = umma_desc_sw32(a_base + (ky * kP + kx + 8 * j) * 32, kP * 32);
+          const uint64_t bd = umma_desc(b_base + (tap * 2) * (kN * 16), kN * 16, 128);
+          const uint32_t acc = (c > 0 || tap > 0) ? 1u : 0u;
+          asm volatile(
+              "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+              "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+                  tmem + (uint32_t)(j * kN)),
+              "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+        }
       asm volatile(
           "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
               smem_u32(empty + st)));
@@ -1443,18 +1427,17 @@ TmEncodeFn tm_encode_fn() {
   return fn;
 }
 
-// Tensor map of one convolution's input [n][h][w][cin]: box ck channels x `pitch` pixels x 18 rows,
-// swizzled over the ck channels, zeros outside the image.
-bool conv_tensor_map(const ConvArgs &a, int ck, int pitch, CUtensorMap *ta) {
+// Tensor map of one convolution's input [n][h][w][cin]: box 16 channels x `pitch` pixels x 18 rows,
+// swizzled over the channels, zeros outside the image.
+bool conv_tensor_map(const ConvArgs &a, int pitch, CUtensorMap *ta) {
   TmEncodeFn enc = tm_encode_fn();
   if (!enc) return false;
   const cuuint64_t dA[4] = {(cuuint64_t)a.cin, (cuuint64_t)a.w, (cuuint64_t)a.h, (cuuint64_t)a.n};
   const cuuint64_t sA[3] = {(cuuint64_t)a.cin * 2, (cuuint64_t)a.w * a.cin * 2,
                             (cuuint64_t)a.h * a.w * a.cin * 2};
-  const cuuint32_t bA[4] = {(cuuint32_t)ck, (cuuint32_t)pitch, kTileH + 2, 1}, e4[4] = {1, 1, 1, 1};
+  const cuuint32_t bA[4] = {16, (cuuint32_t)pitch, kTileH + 2, 1}, e4[4] = {1, 1, 1, 1};
   return enc(ta, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void *)a.in, dA, sA, bA, e4,
-             CU_TENSOR_MAP_INTERLEAVE_NONE,
-             ck == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B,
              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -1483,39 +1466,40 @@ bool wgrad_tensor_maps(const WgradArgs &a, int xc, CUtensorMap *tz, CUtensorMap 
   return map(tz, a.dz, a.cout, a.zcs, 32, kWgP) && map(tx, a.x, a.cin, a.cin, xc, kWtHalo);
 }
 
-template <int kN, int kJ, int kCK>
-int launch_conv(ds2d_unet *u, const ConvArgs &a, const bf16 *wblk, int stages) {
+template <int kN, int kJ, int kS>
+cudaError_t conv_attribute() {
+  return cudaFuncSetAttribute(k_conv3x3_tma<kN, kJ, kS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              cv_smem_bytes<kN, kJ, kS>());
+}
+template <int kN, int kJ, int kS>
+int launch_conv(ds2d_unet *u, const ConvArgs &a, const bf16 *wblk) {
   CUtensorMap ta;
-  if (!conv_tensor_map(a, kCK, cv_pitch<kJ>(), &ta))
+  if (!conv_tensor_map(a, cv_pitch<kJ>(), &ta))
     return unet_fail(u, DS2D_E_CUDA, "conv: cuTensorMapEncodeTiled failed");
-  stages = std::min(stages, a.cin / kCK);
-  while (stages > 1 && cv_smem_bytes<kN, kJ, kCK>(stages) > 226 * 1024) stages--;
   const dim3 grid((a.w + 8 * kJ - 1) / (8 * kJ), (a.h + kTileH - 1) / kTileH, a.n * (a.cout / kN));
-  const int smem = cv_smem_bytes<kN, kJ, kCK>(stages);
-  UCK(cudaFuncSetAttribute(k_conv3x3_tma<kN, kJ, kCK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  k_conv3x3_tma<kN, kJ, kCK><<<grid, 128, smem, u->stream>>>(a, ta, wblk, stages, u->d_err);
+  k_conv3x3_tma<kN, kJ, kS><<<grid, 128, cv_smem_bytes<kN, kJ, kS>(), u->stream>>>(a, ta, wblk, u->d_err);
   UCK(cudaGetLastError());
   return DS2D_OK;
 }
 
 int conv(ds2d_unet *u, const ds2d_unet::Layer &L, const bf16 *in, const bf16 *w, int cin, int cout,
-         const float *bias, bf16 *out, int ocs, int oco, float *out_f32, const bf16 *mask, int relu,
+         const float *bias, bf16 *out, int ocs, int oco, const bf16 *mask, int relu,
          int n, int h, int wd) {
-  ConvArgs a{in, w, bias, out, out_f32, mask, n, h, wd, cin, cout, ocs, oco, relu};
+  ConvArgs a{in, w, bias, out, mask, n, h, wd, cin, cout, ocs, oco, relu};
   if (u->use_tc && u->tc_tma && cout % 32 == 0 && cin % 16 == 0) {
     // tcgen05, operands by bulk-tensor loads
     const int kn = conv_kn(cout);
     const bf16 *wblk = w == L.wf ? L.wfb : (w == L.wb ? L.wbb : nullptr);
     if (!wblk) return unet_fail(u, DS2D_E_STATE, "conv: no blocked weights");
     // Tiles of 8 or 16 pixels x 16 rows and one or two stages: small CTAs, several per SM, whose
-    // loads, MMAs and epilogues interleave.  2008x608 forward / training gradients on 8 x 128x256, ms
-    // (0.94 / 1.33 as chosen): 128 channels 16 pixels 0.97 / 1.39, stages of 32 channels 1.01 /
-    // 1.31; 64 channels 32 pixels 1.01 / 1.37; 32 channels 32 pixels 0.98 / 1.36, two stages 0.97
-    // / 1.33; 96 channels 8 pixels 1.05 / 1.34.
-    if (kn == 128) return launch_conv<128, 1, 16>(u, a, wblk, 2);
-    if (kn == 96) return launch_conv<96, 2, 16>(u, a, wblk, 2);
-    if (kn == 64) return launch_conv<64, 1, 16>(u, a, wblk, 1);
-    return launch_conv<32, 2, 16>(u, a, wblk, 1);
+    // loads, MMAs and epilogues interleave.  2008x608 forward / training gradients on 8 x 128x256 in
+    // one sweep, ms (0.94 / 1.33 as chosen; a whole forward call is at 0.87 now): 128 channels 16
+    // pixels 0.97 / 1.39, chunks of 32 channels 1.01 / 1.31; 64 channels 32 pixels 1.01 / 1.37; 32
+    // channels 32 pixels 0.98 / 1.36, two stages 0.97 / 1.33; 96 channels 8 pixels 1.05 / 1.34.
+    if (kn == 128) return launch_conv<128, 1, 2>(u, a, wblk);
+    if (kn == 96) return launch_conv<96, 2, 2>(u, a, wblk);
+    if (kn == 64) return launch_conv<64, 1, 1>(u, a, wblk);
+    return launch_conv<32, 2, 1>(u, a, wblk);
   }
   if (u->use_tc && cout % 32 == 0) {
     const int kn = cout % 128 == 0 ? 128 : (cout % 64 == 0 ? 64 : 32);
@@ -1712,12 +1696,12 @@ int forward(ds2d_unet *u, const float *x, int n, int h, int w) {
   for (int l = 0; l < 4; l++) {
     const auto &La = u->layers[2 * l], &Lb = u->layers[2 * l + 1];
     if ((rc = conv(u, La, u->act[src].p, La.wf, cin, c[l], u->params + La.b_off, u->act[ea[l]].p,
-                   c[l], 0, nullptr, nullptr, 1, n, hh, ww)))
+                   c[l], 0, nullptr, 1, n, hh, ww)))
       return rc;
     // levels 1-3: the skip goes straight into its channels of the decoder's input
     const auto &E = u->act[eb[l]];
     if ((rc = conv(u, Lb, u->act[ea[l]].p, Lb.wf, c[l], c[l], u->params + Lb.b_off, E.p, E.c, 0,
-                   nullptr, nullptr, 1, n, hh, ww)))
+                   nullptr, 1, n, hh, ww)))
       return rc;
     if (l < 3) {
       k_pool<<<row_grid((long long)n * (hh / 2), (ww / 2) * (c[l] / 8)), 256, 0, u->stream>>>(
@@ -1740,10 +1724,10 @@ int forward(ds2d_unet *u, const float *x, int n, int h, int w) {
     const int li = 8 + 2 * (2 - l);
     const auto &La = u->layers[li], &Lb = u->layers[li + 1];
     if ((rc = conv(u, La, u->act[ca[l]].p, La.wf, cc, c[l], u->params + La.b_off, u->act[da[l]].p,
-                   c[l], 0, nullptr, nullptr, 1, n, hh, ww)))
+                   c[l], 0, nullptr, 1, n, hh, ww)))
       return rc;
     if ((rc = conv(u, Lb, u->act[da[l]].p, Lb.wf, c[l], c[l], u->params + Lb.b_off,
-                   u->act[db[l]].p, c[l], 0, nullptr, nullptr, 1, n, hh, ww)))
+                   u->act[db[l]].p, c[l], 0, nullptr, 1, n, hh, ww)))
       return rc;
     prev = db[l];
     cprev = c[l];
@@ -1792,12 +1776,12 @@ int backward(ds2d_unet *u, int n, int h, int w) {
     // d(d_la output) = conv_bwd(d(db)) masked by d_la's output
     if ((rc = wgrad(u, Lb, u->grad[db[l]].p, c[l], u->act[da[l]].p, n, hh, ww))) return rc;
     if ((rc = conv(u, Lb, u->grad[db[l]].p, Lb.wb, c[l], c[l], nullptr, u->grad[da[l]].p, c[l], 0,
-                   nullptr, u->act[da[l]].p, 0, n, hh, ww)))
+                   u->act[da[l]].p, 0, n, hh, ww)))
       return rc;
     if ((rc = wgrad(u, La, u->grad[da[l]].p, c[l], u->act[ca[l]].p, n, hh, ww))) return rc;
     // d(concat) masked by the concat input (up(prev) and skip are both ReLU outputs)
     if ((rc = conv(u, La, u->grad[da[l]].p, La.wb, c[l], cc, nullptr, u->grad[ca[l]].p, cc, 0,
-                   nullptr, u->act[ca[l]].p, 0, n, hh, ww)))
+                   u->act[ca[l]].p, 0, n, hh, ww)))
       return rc;
     // up part -> gradient of the coarser level's output
     const int prev = l == 2 ? U::E4B : db[l + 1];
@@ -1820,7 +1804,7 @@ int backward(ds2d_unet *u, int n, int h, int w) {
     const int cin = l == 0 ? 16 : c[l - 1];
     if ((rc = wgrad(u, Lb, u->grad[eb[l]].p, c[l], u->act[ea[l]].p, n, hh, ww))) return rc;
     if ((rc = conv(u, Lb, u->grad[eb[l]].p, Lb.wb, c[l], c[l], nullptr, u->grad[ea[l]].p, c[l], 0,
-                   nullptr, u->act[ea[l]].p, 0, n, hh, ww)))
+                   u->act[ea[l]].p, 0, n, hh, ww)))
       return rc;
     if (l == 0) {
       // first layer: cin padded 1 -> 16; weight gradient through the padded scratch, then
@@ -1834,7 +1818,7 @@ int backward(ds2d_unet *u, int n, int h, int w) {
     if ((rc = wgrad(u, La, u->grad[ea[l]].p, c[l], u->act[src].p, n, hh, ww))) return rc;
     // gradient of the pooled input (no mask: pooling output is not a ReLU output)
     if ((rc = conv(u, La, u->grad[ea[l]].p, La.wb, c[l], cin, nullptr, u->grad[src].p, cin, 0,
-                   nullptr, nullptr, 0, n, hh, ww)))
+                   nullptr, 0, n, hh, ww)))
       return rc;
     hh *= 2;
     ww *= 2;
@@ -1963,6 +1947,9 @@ int ds2d_unet_create(int base, int max_n, int max_h, int max_w, int device, ds2d
     if (ea == cudaSuccess)
       ea = cudaFuncSetAttribute(k_conv3x3_tc<64, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 tc_smem_bytes<64, 4>());
+    for (cudaError_t (*f)() : {conv_attribute<128, 1, 2>, conv_attribute<96, 2, 2>,
+                              conv_attribute<64, 1, 1>, conv_attribute<32, 2, 1>})
+      if (ea == cudaSuccess) ea = f();
     if (ea == cudaSuccess)
       ea = cudaFuncSetAttribute(k_conv3x3_tc<32, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 tc_smem_bytes<32, 4>());
