@@ -339,7 +339,7 @@ struct ds2d_ctx {
   double batch_cells = 0, batch_wcells = 0;  // padded / interior cells of the current batch
   // CUDA graphs of whole batches (time loops included), keyed by everything baked into them.
   int opt_graph = 1;
-  bool graph_failed = false;  // no graph could be made on this stream: direct launches
+  bool graph_failed = false;  // no further graph can be made on this stream: direct launches
   long long graph_held = 0;   // launches in the graphs of kinds from kGraphBounded on
   struct GraphEntry {
     std::array<long long, 5> key;
@@ -1317,7 +1317,7 @@ GraphKey graph_key(const ds2d_ctx *c, int kind, int n, int shot_base) {
 }
 template <class F>
 int run_graph(ds2d_ctx *c, const GraphKey &key, F &&body) {
-  if (!c->opt_graph || c->graph_failed || c->prof.on || c->stream == nullptr) return body();
+  if (!c->opt_graph || c->prof.on || c->stream == nullptr) return body();
   for (const auto &g : c->graphs)
     if (key == g.key) {
       CK(cudaGraphLaunch(g.exec, c->stream));
@@ -1325,7 +1325,7 @@ int run_graph(ds2d_ctx *c, const GraphKey &key, F &&body) {
       return DS2D_OK;
     }
   const bool bounded = key[0] >= kGraphBounded;
-  if (bounded && c->graph_held >= kGraphLaunches) return body();
+  if (c->graph_failed || (bounded && c->graph_held >= kGraphLaunches)) return body();
   const long long before = c->last_launches;
   ds2d_ctx::GraphEntry g{};
   g.key = key;
@@ -1347,7 +1347,7 @@ int run_graph(ds2d_ctx *c, const GraphKey &key, F &&body) {
     if (g.exec) cudaGraphExecDestroy(g.exec);
   }
   // A stream that cannot be captured (cudaStreamLegacy) or no memory for another graph: the same
-  // work in direct launches, from now on.
+  // work in direct launches, from now on (graphs made before are still replayed).
   cudaGetLastError();
   c->graph_failed = true;
   c->last_launches = before;
