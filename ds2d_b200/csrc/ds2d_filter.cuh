@@ -19,7 +19,7 @@
 // 2n - 1 points.  Along x the forward transform, the filter and the inverse transform are one
 // kernel (a column never leaves shared memory in between), so an image is read and written three
 // times in all.  The filter and every table are computed on the device.  Two 1201 x 401
-// host images on a B200: 82 -> 1.37 ms a call, 0.31 ms of it in kernels (k_fft_x 181 us: six radix-4
+// host images on a B200: 80 (up to 180) -> 1.35 ms a call, 0.31 ms of it in kernels (k_fft_x 181 us: six radix-4
 // passes of shared memory per transform set the pace), the rest copies.  Longer transforms take dense DFT products (k_dft_gemm) with
 // tables built on the host: exact for any size, about 0.1 s a call.
 #pragma once

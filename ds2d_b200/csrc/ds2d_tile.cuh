@@ -16,9 +16,10 @@
 // State ping-pongs between two buffers as in the marching kernels.
 //
 // Measured (B200, whole calls, against the marching kernels): forward of one 251x101 shot + 20 PML,
-// 2000 steps: 391 -> 9.6 ms; RTM of 2 64x32 shots, 200 steps: 22 -> 1.3 ms; ELSRTM of 4 251x101
-// shots, 500 steps: 529 -> 25 ms; CG-LSRTM of 8 96x48 shots: 245 -> 11 ms.  What bounds a full grid
-// is instruction issue (0.65 a cycle and scheduler), not bytes.
+// 2000 steps: 391 -> 9.1 ms; RTM of 2 64x32 shots, 200 steps: 22 -> 1.25 ms; ELSRTM of 4 251x101
+// shots, 500 steps: 536 -> 25 ms; CG-LSRTM of 8 96x48 shots: 245 -> 11 ms (7.8 with L^T on L's
+// background).  What bounds a full grid is latency: registers hold an SM to 20-25 warps, which use
+// 38-51 % of the issue slots, global loads first among the stalls.
 //
 // Launches of consecutive steps use programmatic dependent launch: a CTA fetches everything that
 // no step writes (moduli, damping, image weights, trace indexes, residuals) before
